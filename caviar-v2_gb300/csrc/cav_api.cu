@@ -279,7 +279,7 @@ int enqueue_chunk(cavgpu_ctx *c, const ChunkPlan &pl, bool capture, long long *l
       CK(capture ? cudaEventRecordWithFlags(c->ev1[k], c->st, cudaEventRecordExternal) : cudaEventRecord(c->ev1[k], c->st));
     nl += 1;
     if (fuse) {  // the next step gathers the coordinates this launch wrote
-      if (mixed) std::swap(view.rel, view.rel_alt);
+      if (mixed) std::swap(view.ic, view.ic_alt);
       else std::swap(view.pos, view.pos_alt);
     }
     if (th && !fold) RK(enqueue_thermo_after_force(c, ring_slot, &nl));
@@ -420,7 +420,12 @@ int make_repbox(double ce, const double lo[3], const double hi[3], RepBox *rb) {
     rb->w[a] = rb->L[a] / rb->nc[a];
     rb->inv_w[a] = 1.0 / rb->w[a];
     rb->wf[a] = (float)rb->w[a];
-    rb->wlo[a] = (float)(rb->w[a] - (double)rb->wf[a]);
+    // fixed-point coordinates (to_fixed): m windows of at least 4 cutoff_extra
+    const int m = (int)std::min(std::max(std::floor(rb->L[a] / (4.0 * ce)), 1.0), 131072.0);
+    const double unit = rb->L[a] / m / 4294967296.0;
+    rb->fx_s[a] = 4294967296.0 * m / rb->L[a];
+    rb->uh[a] = (float)unit;
+    rb->ul[a] = (float)(unit - (double)rb->uh[a]);
   }
   rb->ncell = rb->nc[0] * rb->nc[1] * rb->nc[2];
   return CAVGPU_OK;
@@ -461,7 +466,13 @@ int create_common(const cavgpu_params *p, int nrep, const double *lo3, const dou
   b.ce2_lo = (float)(b.ce2 * (1.0 - 2e-4));
   b.ce2_hi = (float)(b.ce2 * (1.0 + 2e-4));
   b.thr2 = 0.25 * (ce - p->nl_cutoff) * (ce - p->nl_cutoff);
-  b.thr2f = (float)(b.thr2 * (1.0 - 1e-6));
+  // mixed form: shrunk by two fixed-point units of the coarsest axis and by 1e-6; without
+  // a skin every step rebuilds
+  double unit = 0.0;
+  for (const RepBox &rb : c->reps)
+    for (int a = 0; a < 3; ++a) unit = std::max(unit, (double)rb.uh[a]);
+  const double thr = 0.5 * (ce - p->nl_cutoff) - 4.0 * unit;
+  b.thr2f = thr > 0.0 ? (float)(thr * thr * (1.0 - 1e-6)) : -1.0f;
   // pair table (force_field::Lj, src/force/lj.cpp:453-484)
   PairTab &t = c->tab_h;
   const int nt = p->ntypes;
@@ -701,9 +712,9 @@ int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, cons
     };
     for (dbl4 **pp : {&d.pos, &d.vel, &d.acc, &d.pos_ref, &d.t_pos, &d.t_vel, &d.t_acc}) take(pp, NS);
     take(&d.rel, NS);
-    take(&d.rel_ref, NS);
-    // the second buffer of the coordinates a pair kernel gathers (it drifts into it)
-    if (c->p.precision == CAVGPU_MIXED) take(&d.rel_alt, NS);
+    // the coordinates a pair kernel gathers and the second buffer of them (it drifts into it)
+    if (c->p.precision == CAVGPU_MIXED)
+      for (int4 **pp : {&d.ic, &d.ic_ref, &d.ic_alt}) take(pp, NS);
     else take(&d.pos_alt, NS);
     for (int **pp : {&d.type, &d.cell_of, &d.t_type, &d.atom_cell, &d.perm, &d.perm_tmp, &d.nnbr}) take(pp, NS);
     take(&d.id, NS);
@@ -843,9 +854,7 @@ int ensure_status(cavgpu_ctx *c) {
 int complete_overflowed_step(cavgpu_ctx *c, const ChunkPlan &pl, int k, int64_t g, int64_t nsteps, int64_t every,
                              double *out5, int need) {
   if (pl.fused_before(k) & 1) {
-    if (c->p.precision == CAVGPU_MIXED)
-      CK(cudaMemcpyAsync(c->d.rel, c->d.rel_alt, (size_t)c->b.nslot * sizeof(float4), cudaMemcpyDeviceToDevice, c->st));
-    else
+    if (c->p.precision == CAVGPU_FP64)  // (mixed: the build derives the coordinates from the positions)
       CK(cudaMemcpyAsync(c->d.pos, c->d.pos_alt, (size_t)c->b.nslot * sizeof(dbl4), cudaMemcpyDeviceToDevice, c->st));
   }
   RK(alloc_nbr(c, (int)(need * 1.25) + 32));

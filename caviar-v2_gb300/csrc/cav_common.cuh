@@ -93,8 +93,11 @@ struct PairTab {
 struct RepBox {
   double lo[3], hi[3], L[3];
   double w[3], inv_w[3];  // search cell width >= list cutoff
-  float wf[3];            // cell width rounded to FP32 ...
-  float wlo[3];           // ... and the rest, w - wf (a cell offset is d*wf + d*wlo in the mixed form)
+  float wf[3];            // cell width rounded to FP32 (the build's group frames)
+  // fixed-point coordinates (to_fixed): units per length, and the unit's length as an
+  // FP32 pair uh + ul
+  double fx_s[3];
+  float uh[3], ul[3];
   int nc[3];
   int cell_off, ncell;    // cells [cell_off, cell_off + ncell); cell cell_off + ncell holds the padding
   int slot_off, natoms, pad;
@@ -111,7 +114,7 @@ struct Box {
   double ce2;           // cutoff_extra^2, the list predicate r^2 < ce2 (src/neighborlist.cpp:258, :508)
   float ce2_lo, ce2_hi; // FP32 pre-screen band around ce2
   double thr2;          // 0.25 (cutoff_extra - cutoff)^2 (src/neighborlist.cpp:318)
-  float thr2f;          // thr2 * (1 - 1e-6) in FP32: the mixed form's test may only fire early
+  float thr2f;          // thr2 in FP32, shrunk: the mixed form's test may only fire early
   RepBox r0;            // replica 0 by value: the single-system path reads no replica table
 };
 
@@ -134,13 +137,14 @@ struct Dev {
   // acc holds a(t) from the pair kernel until the next pair kernel replaces it, so
   // the velocity-Verlet kick reads it as a_old (leap-frog's drift zeroes it)
   dbl4 *pos, *vel, *acc, *pos_ref;
-  float4 *rel;                // position relative to the build cell's origin; w = type bits
-  float4 *rel_ref;            // rel at the last build (mixed form: rel = rel_ref + (x - pos_ref))
+  float4 *rel;                // position at the last build relative to the build cell's origin; w = type bits
+  int4 *ic;                   // mixed form: fixed-point coordinates (to_fixed); w = type
+  int4 *ic_ref;               // ic at the last build (half-skin test)
   // the coordinates a pair kernel gathers from its neighbours, for the next step: a pair
   // kernel that also drifts its atoms writes them here (FP64 form: positions; mixed
-  // form: rel), while other atoms still read the current ones, and the two swap
+  // form: ic), while other atoms still read the current ones, and the two swap
   dbl4 *pos_alt;
-  float4 *rel_alt;
+  int4 *ic_alt;
   unsigned int *force_ticket; // pair kernel: blocks done (the last one ends the step and resets it)
   int *type;
   uint32_t *id;               // host (insertion) index
@@ -338,16 +342,53 @@ __device__ inline void half_skin_test(const Dev &d, const Box &b, int rep, int i
   if (dx * dx + dy * dy + dz * dz > b.thr2) request_rebuild(d, b, rep);
 }
 
-// Mixed form: the displacement since the build is taken once in FP64 (3
-// subtractions) and serves both the half-skin test (in FP32 against a threshold
-// shrunk by 1e-6, so it can only fire early) and the FP32 cell-relative
-// coordinates, rel = rel_at_build + (float)(x - x_at_build), written to rel_out.
-__device__ inline void mixed_track(const Dev &d, const Box &b, int rep, int i, const dbl4 &x, float4 *rel_out) {
-  const dbl4 r = d.pos_ref[i];
-  const float fx = (float)(x.x - r.x), fy = (float)(x.y - r.y), fz = (float)(x.z - r.z);
-  if (fx * fx + fy * fy + fz * fz > b.thr2f) request_rebuild(d, b, rep);
-  const float4 q = d.rel_ref[i];
-  rel_out[i] = make_float4(q.x + fx, q.y + fy, q.z + fz, q.w);
+// Fixed-point coordinates of the mixed form.  Along an axis the box is cut into m
+// windows of length W = L / m (m = 1 for a box below two windows of 4 list cutoffs)
+// and the coordinate is the position modulo W in units of W / 2^32, as a 32-bit
+// integer that wraps by itself: the difference of two atoms' integers is their
+// displacement to the nearest image, with no cell offset or image shift to decode,
+// for every pair the list holds (a listed image never drifts beyond cutoff_extra +
+// skin <= L - lj cutoff before the half-skin test rebuilds the list, so a difference
+// that wraps to the other image is beyond the cutoff, as that image is).  The unit
+// is below 8 cutoff_extra / 2^32 (5e-9 sigma at 2.8), 25 times finer than the
+// rounding of an FP32 coordinate inside a cell, and differences are exact before
+// their one conversion to FP32.  One FMA per axis: adding 1.5 * 2^52 leaves the
+// rounded integer in the low mantissa bits, the low word of which is taken.
+__device__ __forceinline__ double to_fixed(double x, double lo, double s) {
+  return fma(x - lo, s, 6755399441055744.0);  // 1.5 * 2^52
+}
+__device__ __forceinline__ int4 fixed_pos(const RepBox &rb, const dbl4 &x, int type, int3 &window) {
+  const double tx = to_fixed(x.x, rb.lo[0], rb.fx_s[0]), ty = to_fixed(x.y, rb.lo[1], rb.fx_s[1]),
+               tz = to_fixed(x.z, rb.lo[2], rb.fx_s[2]);
+  window = make_int3(__double2hiint(tx) & 1023, __double2hiint(ty) & 1023, __double2hiint(tz) & 1023);
+  return make_int4(__double2loint(tx), __double2loint(ty), __double2loint(tz), type);
+}
+// the same as a reference of later displacements: w holds ten bits of each window index
+__device__ __forceinline__ int4 fixed_ref(const int4 &q, const int3 &window) {
+  return make_int4(q.x, q.y, q.z, window.x | (window.y << 10) | (window.z << 20));
+}
+// b - a modulo 2^32, as a signed displacement
+__device__ __forceinline__ int fixed_diff(int b, int a) { return (int)((unsigned)b - (unsigned)a); }
+// whether the displacement from (r, rw) to (q, qw) is more than half a window
+__device__ __forceinline__ bool beyond_window(int q, int qw, int r, int rw) {
+  const int high = qw - rw - ((unsigned)q < (unsigned)r ? 1 : 0);  // of the two-word difference
+  return ((high - (fixed_diff(q, r) >> 31)) & 1023) != 0;
+}
+
+// Mixed form: the new fixed-point coordinates, written to `out`, and the half-skin
+// test on their difference to those of the last build (in FP32 against a threshold
+// shrunk by the units' rounding and 1e-6, so it can only fire early; the window
+// indices tell a displacement that wrapped, as in a system that flies apart).
+__device__ inline void mixed_track(const Dev &d, const Box &b, int rep, int i, const dbl4 &x, int4 *out) {
+  const RepBox &rb = repbox(b, rep);
+  int3 w;
+  const int4 q = fixed_pos(rb, x, type_of(x.w), w), r = d.ic_ref[i];
+  const float fx = (float)fixed_diff(q.x, r.x) * rb.uh[0], fy = (float)fixed_diff(q.y, r.y) * rb.uh[1],
+              fz = (float)fixed_diff(q.z, r.z) * rb.uh[2];
+  if (fx * fx + fy * fy + fz * fz > b.thr2f || beyond_window(q.x, w.x, r.x, r.w & 1023) ||
+      beyond_window(q.y, w.y, r.y, (r.w >> 10) & 1023) || beyond_window(q.z, w.z, r.z, (r.w >> 20) & 1023))
+    request_rebuild(d, b, rep);
+  out[i] = q;
 }
 
 __device__ inline void nan_check(const Dev &d, int i, const dbl4 &a) {
@@ -419,7 +460,7 @@ inline int rebuild_kernels(const Box &b) { return 8 + (scan_slices(b) > 1 ? 1 : 
 // kick: 0 = force only, 1 = VV closing kick, 2 = Langevin closing update.
 // thermo: virial/PE partials (and KE partials unless kick == 2).
 // fuse (Fuse): the next step's drift in the same launch, written to d.pos_alt (FP64)
-// or d.rel_alt (mixed); the caller swaps them with d.pos / d.rel afterwards.
+// or d.ic_alt (mixed); the caller swaps them with d.pos / d.ic afterwards.
 // cond: when set_cond, the last block sets the conditional node of the next step's
 // rebuild to the half-skin flag (unless halted).  The last block also counts the
 // step (F_STEPS_OK) and raises the halt on a NaN.

@@ -5,9 +5,9 @@
 // atom, a warp on A = 32/TPA atoms, and the list layout (nbr_index) makes every
 // iteration one coalesced 128-byte read of neighbour words.  Two precisions:
 //   FP64  : image = x_j + s*L, all pair arithmetic in double;
-//   MIXED : FP32 pair arithmetic on coordinates relative to each atom's build cell
-//           (float4 x,y,z,type; cell offsets decoded from the stencil index), FP64
-//           accumulation across lanes, FP64 acceleration/velocity/reductions.
+//   MIXED : FP32 pair arithmetic on exact differences of fixed-point coordinates
+//           (int4 x,y,z,type; to_fixed), FP64 accumulation across lanes, FP64
+//           acceleration/velocity/reductions.
 #include <type_traits>
 
 #include "cav_common.cuh"
@@ -47,18 +47,13 @@ struct SmemTabF {
   float pk[MAXT * MAXT];   // 0.5 gc rc2 - uc, rounded once from FP64: V = eps4 s6 (s6 - 1) - 0.5 gc r2 + pk
   double minv[MAXT], mass[MAXT];
 };
-// per warp: the 27 image shifts s*L (FP64) or the cell widths (mixed) of the
-// replica the warp's current atoms belong to (a warp never straddles two).  The
-// mixed offsets are FP32 pairs d*wf + d*wlo: with the rounded width alone, every
-// pair across a cell face would be displaced by the same d*(wf - w), a fixed
-// distortion of the potential that changes pattern at each rebuild and drifts
-// the NVE energy (measured -2.4e-4 per 1e6 steps).
+// per warp: the 27 image shifts s*L (FP64) or the fixed-point units (mixed) of the
+// replica the warp's current atoms belong to (a warp never straddles two)
 template <bool MIXED>
 struct WarpImages;
 template <>
 struct WarpImages<true> {
-  float4 w;   // (wf, 0): cell widths rounded to FP32; a neighbour's offset is d*wf + d*wlo,
-  float4 lo;  // (wlo, 0)  with d in {-1,0,1}^3 decoded from its stencil index
+  float4 hi, lo;  // length of a coordinate unit per axis, as an FP32 pair hi + lo
 };
 
 // Single-type systems keep the pair constants in registers (no table lookups).
@@ -157,104 +152,114 @@ __device__ __forceinline__ uint4 ld_list(const uint4 *p) {
   return v;
 }
 
+// One pair evaluation of the mixed form, two list entries at a time in packed FP32x2
+// arithmetic: sums of the even and of the odd entries of a lane's chunks.
+struct PairSums {
+  F2 ax, ay, az, vr, pp;  // vr: sum of +coef r^2
+};
+
+// Displacement r_j - r_i: the integer difference is exact, its conversion to FP32 and
+// the product with the unit (an FP32 pair, so that no scale error is left) round once
+// each; all of it is odd in the difference, so d_ji = -d_ij bit for bit and the FP32
+// pair forces obey Newton's third law exactly (each half of a packed operation rounds
+// as the scalar one).
+__device__ __forceinline__ F2 displacement2(int ja, int jb, int i, float hi, float lo) {
+  const F2 f = f2((float)fixed_diff(ja, i), (float)fixed_diff(jb, i));
+  return fma2(f, f2(lo, lo), mul2(f, f2(hi, hi)));
+}
+
+template <bool EV, bool ONE>
+__device__ __forceinline__ void mixed_pair2(const int4 &ja, const int4 &jb, bool va, bool vb, const int4 &ri, int nt,
+                                            const SmemTabF &tab, const OneType &c1, const float4 &uh,
+                                            const float4 &ul, float jtol, PairSums &S) {
+  const F2 dx = displacement2(ja.x, jb.x, ri.x, uh.x, ul.x), dy = displacement2(ja.y, jb.y, ri.y, uh.y, ul.y),
+           dz = displacement2(ja.z, jb.z, ri.z, uh.z, ul.z);
+  const F2 r2d = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+  float r2a, r2b;
+  unf2(r2d, r2a, r2b);
+  float rc2a, rc2b, sg2a, sg2b, e4a, e4b, gca, gcb, pka, pkb;
+  if (ONE) {
+    rc2a = rc2b = c1.rc2; sg2a = sg2b = c1.sig2; e4a = e4b = c1.eps4; gca = gcb = c1.gc; pka = pkb = c1.pk;
+  } else {
+    const int ta = ri.w * nt + ja.w, tb = ri.w * nt + jb.w;
+    const float4 pa = tab.c4[ta], pb = tab.c4[tb];
+    rc2a = pa.x; sg2a = pa.y; e4a = pa.z; gca = pa.w;
+    rc2b = pb.x; sg2b = pb.y; e4b = pb.z; gcb = pb.w;
+    pka = EV ? tab.pk[ta] : 0.0f;
+    pkb = EV ? tab.pk[tb] : 0.0f;
+  }
+  const bool ina = va && r2a <= rc2a, inb = vb && r2b <= rc2b;
+  if (!(ina || inb)) return;
+  const float r2ca = fmaxf(r2a, jtol), r2cb = fmaxf(r2b, jtol);  // Lj jump_fix floor (0 when off)
+  const F2 r2 = f2(r2ca, r2cb), r2i = f2(rcp_approx(r2ca), rcp_approx(r2cb));
+  const F2 eps4 = f2(e4a, e4b);
+  const F2 s2 = mul2(f2(sg2a, sg2b), r2i);
+  const F2 s6 = mul2(mul2(s2, s2), s2);
+  const F2 w = mul2(mul2(eps4, r2i), s6);
+  F2 coef = fma2(w, fma2(f2(-12.0f, -12.0f), s6, f2(6.0f, 6.0f)), f2(-gca, -gcb));
+  float ca, cb;
+  unf2(coef, ca, cb);
+  coef = f2(ina ? ca : 0.0f, inb ? cb : 0.0f);
+  S.ax = fma2(coef, dx, S.ax);
+  S.ay = fma2(coef, dy, S.ay);
+  S.az = fma2(coef, dz, S.az);
+  if (EV) {
+    S.vr = fma2(coef, r2, S.vr);
+    const F2 pe = fma2(mul2(eps4, s6), sub2(s6, f2(1.0f, 1.0f)), fma2(f2(-0.5f * gca, -0.5f * gcb), r2, f2(pka, pkb)));
+    float pa, pb;
+    unf2(pe, pa, pb);
+    S.pp = add2(S.pp, f2(ina ? pa : 0.0f, inb ? pb : 0.0f));
+  }
+}
+
 // Mixed-form pair loop of one lane: list chunks t, t+TPA, ... of atom i (four words
 // per 128-bit load; the next chunk's load and four neighbour coordinates in
-// flight); `gather(word)` returns the neighbour's float4 (global memory or a
-// shared-memory stage).  Two pairs go through each packed FP32x2 evaluation (even
-// and odd list entries, with their own accumulators, folded at the end); a pair
-// beyond its cutoff gets coef = 0.  ONE: single-type system, pair constants in
-// registers; otherwise from the shared-memory table.
-//
-// ((r_j - r_i) + d wf) + d wlo, each sum rounded once (d wf and d wlo are exact
-// products): rounding is symmetric under negation and i seen from j has offset -d,
-// so d_ji = -d_ij bit for bit and the FP32 pair forces obey Newton's third law
-// exactly (each half of a packed operation rounds as the scalar one).  d comes from
-// the stencil index k = (dx+1) + 3 (dy+1) + 9 (dz+1) by integer arithmetic (a table
-// in shared memory would load the L1 pipe that the neighbour gathers saturate).
+// flight); `gather(word)` returns the neighbour's int4 (global memory or a
+// shared-memory stage).  Whole chunks run without tests of the entry number; the
+// row's last, partial chunk follows, its missing entries stood in for by the first.
+// What bounds it: the gathers (16 bytes per lane from some 10 lines: the LSU data path is
+// busy 71% of the time) and their latency.  Against coordinates relative to each atom's
+// cell, whose offsets had to be decoded from the list words and added (and lists in
+// stencil order), the loop issues 99 M instead of 135 M instructions on the 1,048,576-atom
+// fluid and a launch takes 160 us instead of 186 (one lane per atom); half or a quarter
+// of the gathers through the texture path: 174 and 192 us; 40 or 48 warps per SM (48 and
+// 40 registers): 240 and 320 us, the loop spills.
+// ONE: single-type system, pair constants in registers; otherwise from the
+// shared-memory table.
 template <int TPA, bool EV, bool ONE, class Gather>
-__device__ __forceinline__ void mixed_pairs(const uint4 *row4, int nn, int t, const float4 ri, int ti, int nt,
-                                            const SmemTabF &tab, const OneType c1, const float4 wf,
-                                            const float4 wl, const float jtol, Gather gather, float &ax,
+__device__ __forceinline__ void mixed_pairs(const uint4 *row4, int nn, int t, const int4 ri, int nt,
+                                            const SmemTabF &tab, const OneType c1, const float4 uh,
+                                            const float4 ul, const float jtol, Gather gather, float &ax,
                                             float &ay, float &az, float &vr, float &pp) {
-  F2 ax2 = f2(0.f, 0.f), ay2 = ax2, az2 = ax2, vr2 = ax2, pp2 = ax2;  // vr2: sum of +coef r^2
+  PairSums S;
+  S.ax = S.ay = S.az = S.vr = S.pp = f2(0.f, 0.f);
+  const int nfull = nn >> 2;
   uint4 nxt = 4 * t < nn ? ld_list(row4) : make_uint4(0, 0, 0, 0);
-  for (int q = 0, k0 = 4 * t; k0 < nn; ++q, k0 += 4 * TPA) {
+  int g = t;
+  for (; g < nfull; g += TPA) {
     const uint4 w4 = nxt;
-    if (k0 + 4 * TPA < nn) nxt = ld_list(row4 + (size_t)(q + 1) * 32);  // the next list chunk in flight
-    const uint32_t e[4] = {w4.x, w4.y, w4.z, w4.w};
-    float4 rj[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)  // four independent gathers in flight
-      if (k0 + u < nn) rj[u] = gather(e[u]);
-      else rj[u] = make_float4(1e18f, 1e18f, 1e18f, __int_as_float(ti));  // beyond every cutoff
-#pragma unroll
-    for (int a = 0; a < 4; a += 2) {
-      if (k0 + a >= nn) break;
-      // d = k - 1 for k in {0, 1, 2} without an int-to-float conversion: the float
-      // with bits 0x4B400000 | k is 12582912 + k exactly, and 12582913 is subtracted
-      float dd[6];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int code = e[a + h] >> CODE_SHIFT;
-        const int kz = (code * 57) >> 9, r9 = code - 9 * kz, ky = (r9 * 11) >> 5, kx = r9 - 3 * ky;  // k/9, k/3
-        dd[h] = __int_as_float(0x4B400000 | kx);
-        dd[2 + h] = __int_as_float(0x4B400000 | ky);
-        dd[4 + h] = __int_as_float(0x4B400000 | kz);
-      }
-      const F2 magic = f2(12582913.0f, 12582913.0f);
-      const F2 ddx = sub2(f2(dd[0], dd[1]), magic), ddy = sub2(f2(dd[2], dd[3]), magic),
-               ddz = sub2(f2(dd[4], dd[5]), magic);
-      const F2 dx = fma2(ddx, f2(wl.x, wl.x), fma2(ddx, f2(wf.x, wf.x), sub2(f2(rj[a].x, rj[a + 1].x), f2(ri.x, ri.x))));
-      const F2 dy = fma2(ddy, f2(wl.y, wl.y), fma2(ddy, f2(wf.y, wf.y), sub2(f2(rj[a].y, rj[a + 1].y), f2(ri.y, ri.y))));
-      const F2 dz = fma2(ddz, f2(wl.z, wl.z), fma2(ddz, f2(wf.z, wf.z), sub2(f2(rj[a].z, rj[a + 1].z), f2(ri.z, ri.z))));
-      const F2 r2d = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
-      float r2a, r2b;
-      unf2(r2d, r2a, r2b);
-      float rc2a, rc2b, sg2a, sg2b, e4a, e4b, gca, gcb, pka, pkb;
-      if (ONE) {
-        rc2a = rc2b = c1.rc2; sg2a = sg2b = c1.sig2; e4a = e4b = c1.eps4; gca = gcb = c1.gc; pka = pkb = c1.pk;
-      } else {
-        const int ta = ti * nt + __float_as_int(rj[a].w), tb = ti * nt + __float_as_int(rj[a + 1].w);
-        const float4 pa = tab.c4[ta], pb = tab.c4[tb];
-        rc2a = pa.x; sg2a = pa.y; e4a = pa.z; gca = pa.w;
-        rc2b = pb.x; sg2b = pb.y; e4b = pb.z; gcb = pb.w;
-        pka = EV ? tab.pk[ta] : 0.0f;
-        pkb = EV ? tab.pk[tb] : 0.0f;
-      }
-      const bool ina = r2a <= rc2a, inb = r2b <= rc2b;
-      if (!(ina || inb)) continue;
-      const float r2ca = fmaxf(r2a, jtol), r2cb = fmaxf(r2b, jtol);  // Lj jump_fix floor (0 when off)
-      const F2 r2 = f2(r2ca, r2cb), r2i = f2(rcp_approx(r2ca), rcp_approx(r2cb));
-      const F2 eps4 = f2(e4a, e4b);
-      const F2 s2 = mul2(f2(sg2a, sg2b), r2i);
-      const F2 s6 = mul2(mul2(s2, s2), s2);
-      const F2 w = mul2(mul2(eps4, r2i), s6);
-      F2 coef = fma2(w, fma2(f2(-12.0f, -12.0f), s6, f2(6.0f, 6.0f)), f2(-gca, -gcb));
-      float ca, cb;
-      unf2(coef, ca, cb);
-      ca = ina ? ca : 0.0f;
-      cb = inb ? cb : 0.0f;
-      coef = f2(ca, cb);
-      ax2 = fma2(coef, dx, ax2);
-      ay2 = fma2(coef, dy, ay2);
-      az2 = fma2(coef, dz, az2);
-      if (EV) {
-        vr2 = fma2(coef, r2, vr2);
-        const F2 pe = fma2(mul2(eps4, s6), sub2(s6, f2(1.0f, 1.0f)),
-                           fma2(f2(-0.5f * gca, -0.5f * gcb), r2, f2(pka, pkb)));
-        float pa, pb;
-        unf2(pe, pa, pb);
-        pp2 = add2(pp2, f2(ina ? pa : 0.0f, inb ? pb : 0.0f));
-      }
+    row4 += 32;
+    if (4 * (g + TPA) < nn) nxt = ld_list(row4);  // the next list chunk in flight
+    const int4 j0 = gather(w4.x), j1 = gather(w4.y), j2 = gather(w4.z), j3 = gather(w4.w);
+    mixed_pair2<EV, ONE>(j0, j1, true, true, ri, nt, tab, c1, uh, ul, jtol, S);
+    mixed_pair2<EV, ONE>(j2, j3, true, true, ri, nt, tab, c1, uh, ul, jtol, S);
+  }
+  const int rest = nn & 3;
+  if (g == nfull && rest) {
+    const int4 j0 = gather(nxt.x), j1 = rest > 1 ? gather(nxt.y) : j0;
+    mixed_pair2<EV, ONE>(j0, j1, true, rest > 1, ri, nt, tab, c1, uh, ul, jtol, S);
+    if (rest > 2) {
+      const int4 j2 = gather(nxt.z);
+      mixed_pair2<EV, ONE>(j2, j2, true, false, ri, nt, tab, c1, uh, ul, jtol, S);
     }
   }
   float lo, hi;
-  unf2(ax2, lo, hi); ax += lo + hi;
-  unf2(ay2, lo, hi); ay += lo + hi;
-  unf2(az2, lo, hi); az += lo + hi;
+  unf2(S.ax, lo, hi); ax += lo + hi;
+  unf2(S.ay, lo, hi); ay += lo + hi;
+  unf2(S.az, lo, hi); az += lo + hi;
   if (EV) {
-    unf2(vr2, lo, hi); vr -= lo + hi;
-    unf2(pp2, lo, hi); pp += lo + hi;
+    unf2(S.vr, lo, hi); vr -= lo + hi;
+    unf2(S.pp, lo, hi); pp += lo + hi;
   }
 }
 
@@ -273,7 +278,7 @@ __device__ inline OneType one_type(const SmemTabF &tab) {
 // fuse: then the first half of the next step, with the arithmetic of the drift
 // kernels (k_drift_vv, k_drift_lf, k_lang_a): the NaN check of the new acceleration,
 // the drift, the half-skin test; the new coordinates go to the alternate buffer
-// (FP64: pos_alt, which the neighbours of this step no longer read; mixed: rel_alt,
+// (FP64: pos_alt, which the neighbours of this step no longer read; mixed: ic_alt,
 // the FP64 positions being this atom's alone).  Leap-frog keeps a_old = 0 for the
 // next kick, as its drift kernel does.
 template <int A, bool MIXED, int KICK, bool EV, class Tab>
@@ -365,7 +370,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
       d.vel[i] = v;
       if (MIXED) {
         d.pos[i] = x;
-        mixed_track(d, b, rep, i, x, d.rel_alt);
+        mixed_track(d, b, rep, i, x, d.ic_alt);
       } else {
         d.pos_alt[i] = x;
         half_skin_test(d, b, rep, i, x);
@@ -526,8 +531,8 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
       const RepBox &rb = repbox(b, rep);
       if constexpr (MIXED) {
         if (lane == 0) {
-          wimg[wid].w = make_float4(rb.wf[0], rb.wf[1], rb.wf[2], 0.f);
-          wimg[wid].lo = make_float4(rb.wlo[0], rb.wlo[1], rb.wlo[2], 0.f);
+          wimg[wid].hi = make_float4(rb.uh[0], rb.uh[1], rb.uh[2], 0.f);
+          wimg[wid].lo = make_float4(rb.ul[0], rb.ul[1], rb.ul[2], 0.f);
         }
       } else if (lane < 27) {
         const int sx = lane % 3 - 1, sy = (lane / 3) % 3 - 1, sz = lane / 9 - 1;
@@ -546,12 +551,12 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
       // load each; the warp's loads for one q cover 512 consecutive bytes (nbr_index)
       const uint4 *row4 = reinterpret_cast<const uint4 *>(d.nbr + (size_t)task * cap * A) + (t * A + a);
       if constexpr (MIXED) {
-        const float4 ri = d.rel[i];
-        ti = __float_as_int(ri.w);
+        const int4 ri = d.ic[i];
+        ti = ri.w;
         float ax = 0.f, ay = 0.f, az = 0.f, vr = 0.f, pp = 0.f;
-        const float4 *rel = d.rel;
-        mixed_pairs<TPA, EV, ONE>(row4, nn, t, ri, ti, nt, tab, one_type(tab), wimg[wid].w, wimg[wid].lo, sc.jump_tolf,
-                             [rel](uint32_t w) { return __ldg(&rel[w & IDX_MASK]); }, ax, ay, az, vr, pp);
+        const int4 *ic = d.ic;
+        mixed_pairs<TPA, EV, ONE>(row4, nn, t, ri, nt, tab, one_type(tab), wimg[wid].hi, wimg[wid].lo, sc.jump_tolf,
+                                  [ic](uint32_t w) { return __ldg(&ic[w & IDX_MASK]); }, ax, ay, az, vr, pp);
         fx = ax; fy = ay; fz = az; vir = vr; pe = pp;
       } else {
         const dbl4 xi = d.pos[i];
@@ -629,7 +634,7 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
 
 // Mixed-form pair kernel over row segments.  A block takes a segment -- up to
 // seg_umax - 2 consecutive cells of one x-row of one replica -- and stages into
-// shared memory the FP32 coordinates of the atoms of the 9 neighbouring rows'
+// shared memory the fixed-point coordinates of the atoms of the 9 neighbouring rows'
 // cells x0-1 .. x0+len (periodic), so that every neighbour gather of the
 // segment's atoms reads shared memory.  A list word (slot j, stencil index k)
 // finds its copy through a table: row r = k / 3 of the stencil, staged cell
@@ -643,9 +648,9 @@ __global__ void __launch_bounds__(256) k_force_seg(Dev d, Box b, StepConsts sc, 
   constexpr int A = 32 / TPA;
   constexpr int AS = 5 - (TPA == 1 ? 0 : TPA == 2 ? 1 : TPA == 4 ? 2 : TPA == 8 ? 3 : 4);  // log2(A)
   __shared__ SmemTabF tab;
-  __shared__ float4 s_wf, s_wl;
+  __shared__ float4 s_uh, s_ul;
   __shared__ int s_total;
-  extern __shared__ float4 stage[];
+  extern __shared__ int4 stage[];
   const int umax = d.seg_umax;
   int *const toff = reinterpret_cast<int *>(stage + d.stage_cap);  // [9 * umax] stage offset - first slot
   int *const tcnt = toff + 9 * umax;                                 // [9 * umax] atoms, then exclusive scan
@@ -673,8 +678,8 @@ __global__ void __launch_bounds__(256) k_force_seg(Dev d, Box b, StepConsts sc, 
     __syncthreads();  // the previous segment's gathers are done with the stage and tables
     if (rep != img_rep) {
       if (threadIdx.x == 0) {
-        s_wf = make_float4(rb.wf[0], rb.wf[1], rb.wf[2], 0.f);
-        s_wl = make_float4(rb.wlo[0], rb.wlo[1], rb.wlo[2], 0.f);
+        s_uh = make_float4(rb.uh[0], rb.uh[1], rb.uh[2], 0.f);
+        s_ul = make_float4(rb.ul[0], rb.ul[1], rb.ul[2], 0.f);
       }
       img_rep = rep;
     }
@@ -715,7 +720,7 @@ __global__ void __launch_bounds__(256) k_force_seg(Dev d, Box b, StepConsts sc, 
       for (int q = wid; q < nq; q += nwarp) {
         const int st = toff[q], base = tcnt[q];
         const int cn = (q + 1 < nq ? tcnt[q + 1] : s_total) - base;
-        for (int k = lane; k < cn; k += 32) stage[base + k] = __ldg(&d.rel[st + k]);
+        for (int k = lane; k < cn; k += 32) stage[base + k] = __ldg(&d.ic[st + k]);
       }
       __syncthreads();
       for (int q = threadIdx.x; q < nq; q += blockDim.x) toff[q] = tcnt[q] - toff[q];
@@ -734,22 +739,22 @@ __global__ void __launch_bounds__(256) k_force_seg(Dev d, Box b, StepConsts sc, 
         if (act) {
           const int nn = d.nnbr[i];
           const uint4 *row4 = reinterpret_cast<const uint4 *>(d.nbr + (size_t)task * cap * A) + (t * A + a);
-          const float4 ri = d.rel[i];
-          ti = __float_as_int(ri.w);
+          const int4 ri = d.ic[i];
+          ti = ri.w;
           float ax = 0.f, ay = 0.f, az = 0.f, vr = 0.f, pp = 0.f;
           if (staged) {
             const int hx = d.cell_of[i] - rowc - x0;  // home cell within the segment
             const int *tr = toff + hx;
-            mixed_pairs<TPA, EV, ONE>(row4, nn, t, ri, ti, nt, tab, one_type(tab), s_wf, s_wl, sc.jump_tolf,
+            mixed_pairs<TPA, EV, ONE>(row4, nn, t, ri, nt, tab, one_type(tab), s_uh, s_ul, sc.jump_tolf,
                                  [tr, U](uint32_t w) {  // `stage` is the block's shared array
                                    const int k = (int)(w >> CODE_SHIFT), r = (k * 11) >> 5;  // k / 3 for k < 27
                                    return stage[(int)(w & IDX_MASK) + tr[r * U + (k - 3 * r)]];
                                  },
                                  ax, ay, az, vr, pp);
           } else {
-            const float4 *rel = d.rel;
-            mixed_pairs<TPA, EV, ONE>(row4, nn, t, ri, ti, nt, tab, one_type(tab), s_wf, s_wl, sc.jump_tolf,
-                                 [rel](uint32_t w) { return __ldg(&rel[w & IDX_MASK]); }, ax, ay, az, vr, pp);
+            const int4 *ic = d.ic;
+            mixed_pairs<TPA, EV, ONE>(row4, nn, t, ri, nt, tab, one_type(tab), s_uh, s_ul, sc.jump_tolf,
+                                 [ic](uint32_t w) { return __ldg(&ic[w & IDX_MASK]); }, ax, ay, az, vr, pp);
           }
           fx = ax; fy = ay; fz = az; vir = vr; pe = pp;
         }

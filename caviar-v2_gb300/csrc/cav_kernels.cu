@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) k_drift_vv(Dev d, Box b, StepConsts sc) {
   nan_check(d, i, a);
   drift_vv<MIXED>(x, v, a, sc);
   d.pos[i] = x;  // acc stays: the pair kernel's kick reads it as a_old
-  if (MIXED) mixed_track(d, b, rep, i, x, d.rel);
+  if (MIXED) mixed_track(d, b, rep, i, x, d.ic);
   else half_skin_test(d, b, rep, i, x);
 }
 
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(256) k_drift_lf(Dev d, Box b, StepConsts sc) {
   d.pos[i] = x;
   d.vel[i] = v;
   d.acc[i] = make_dbl4(0.0, 0.0, 0.0, 0.0);  // a_old = 0 for the kick
-  if (MIXED) mixed_track(d, b, rep, i, x, d.rel);
+  if (MIXED) mixed_track(d, b, rep, i, x, d.ic);
   else half_skin_test(d, b, rep, i, x);
 }
 
@@ -112,7 +112,7 @@ __device__ __forceinline__ void lang_position(const Dev &d, const Box &b, const 
   }
   lang_move<MIXED>(x, v, sc);
   d.pos[i] = x;
-  if (MIXED) mixed_track(d, b, rep, i, x, d.rel);
+  if (MIXED) mixed_track(d, b, rep, i, x, d.ic);
   else half_skin_test(d, b, rep, i, x);
 }
 
@@ -383,8 +383,14 @@ __global__ void __launch_bounds__(256) k_gather(Dev d, Box b, int forced) {
   if (d.img) d.img[k] = d.t_img[o];
   if (d.mol) d.mol[k] = d.t_mol[o];
   d.cell_of[k] = d.perm_tmp[o];
-  update_rel(d, repbox(b, rep), k, x);
-  d.rel_ref[k] = d.rel[k];
+  const RepBox &rb = repbox(b, rep);
+  update_rel(d, rb, k, x);
+  if (d.ic) {
+    int3 w;
+    const int4 q = fixed_pos(rb, x, type_of(x.w), w);
+    d.ic[k] = q;
+    d.ic_ref[k] = fixed_ref(q, w);
+  }
 }
 
 // Verlet-list build over the 27-cell stencil with periodic image shifts.
@@ -409,14 +415,36 @@ __device__ __noinline__ bool exact_pair(const Dev &d, const RepBox &rb, double c
 // it, form a group (a window that crosses the end of a row, or a sparse row, takes
 // two or more groups in turn).  Slots are sorted by cell, so a group is 32 (or
 // fewer) atoms from 1-3 neighbouring cells.  Its candidates are the atoms of the
-// cells cx_first - 1 .. cx_last + 1 of the 3 x 3 neighbouring rows, taken row by row
-// (dz, then dy, then x, slot order inside a cell), and of those only the ones within
-// the list cutoff (plus the FP32 band) of the group's bounding box are staged: ~540
-// staged candidates per 32 atoms of the 1M-atom fluid, against 27 cells x 19 atoms
-// = 516 per 19-atom cell when a warp took one cell.  Every atom's row keeps the
-// stencil order k = (dx+1) + 3(dy+1) + 9(dz+1), slot order inside a cell, so the
-// lists do not depend on how slots fall into windows.
+// cells cx_first - 1 .. cx_last + 1 of the 3 x 3 neighbouring rows, taken row by row,
+// and of those only the ones within the list cutoff (plus the FP32 band) of the
+// group's bounding box are staged: ~540 staged candidates per 32 atoms of the 1M-atom
+// fluid, against 27 cells x 19 atoms = 516 per 19-atom cell when a warp took one cell.
 //
+// Order of an atom's row: the neighbouring rows of cells as ROW_ORDER has them, in a row
+// the cells by their x index modulo 3, slot order inside a cell; it depends on the
+// atom's cell alone, not on how slots fall into windows.  The order is chosen for the
+// pair kernel's gathers, where the 32 lanes of a warp are 32 atoms that each read the
+// k-th entry of their own row: they touch the fewest 128-byte lines when the lanes are
+// at the same cell at the same k.  In stencil order (z, then y, then x) they are not --
+// an atom at the bottom of its cell has half its neighbours in the lower layer, one at
+// the top next to none -- so the rows alternate between opposite sides of the stencil,
+// which keeps the running counts of the lanes close, and the x index modulo 3 makes
+// atoms of adjacent cells take their common cells at the same time.  Distinct lines per
+// gather in a melted fluid (counted on the host): 16.0 in stencil order, 10.6 in this one.
+__constant__ const int8_t ROW_ORDER[9] = {4, 0, 8, 2, 6, 1, 7, 3, 5};  // (dy+1) + 3 (dz+1), nearest row first
+// Which of the group's nu candidate cells of a row comes k-th: cells x0 + u by
+// (x0 + u) mod 3, ascending inside a class (x0 >= -1).
+__device__ __forceinline__ int class_cell(int x0, int nu, int k) {
+  int u = 0;
+  for (int c = 0; c < 3; ++c) {
+    u = (c + 3 - (x0 + 3) % 3) % 3;  // first cell of class c
+    const int n = (nu - u + 2) / 3;  // nu >= 3: every class has a cell
+    if (k < n) break;
+    k -= n;
+  }
+  return u + 3 * k;
+}
+
 // Staging: candidates u and u+1 (u even) interleaved as {x_u, x_u+1, y_u, y_u+1}
 // and {z_u, z_u+1} in the warp's slice of shared memory (coordinates relative to
 // the origin of the group's first cell), the words (j | code) in an array of their
@@ -616,7 +644,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 4) k_build_group(Dev d, Box 
       L.rzz = pack2(gz);
       L.hi = L.me ? b.ce2_hi : -1.0f;
       L.cnt = 0;
-      // candidate cells q = r * nu + u: row r = (dy+1) + 3 (dz+1), x cell cx0 - 1 + u
+      // candidate cells, nu in each of the 9 rows r = (dy+1) + 3 (dz+1): x cell cx0 - 1 + u
       const int nu = span + 3, ncand = 9 * nu;
       int nst = 0;
       selfpos[lane] = -1;
@@ -628,7 +656,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 4) k_build_group(Dev d, Box 
         float kox = 0.f, koy = 0.f, koz = 0.f;
         const int q = q0 + lane;
         if (q < ncand) {
-          const int r = q / nu, u = q - r * nu;
+          const int qr = q / nu, r = ROW_ORDER[qr], u = class_cell(cx0 - 1, nu, q - qr * nu);
           const int dy = r % 3 - 1, dz = r / 3 - 1;
           int nx = cx0 - 1 + u, ny = cy + dy, nz = cz + dz, sx = 0, sy = 0, sz = 0;
           if (nx < 0) { nx += rb.nc[0]; sx = -1; } else if (nx >= rb.nc[0]) { nx -= rb.nc[0]; sx = 1; }
