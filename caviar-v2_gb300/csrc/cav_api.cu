@@ -599,6 +599,18 @@ int build_segments(cavgpu_ctx *c) {
   return prepare_force_seg(seg_smem_bytes(c->d.stage_cap, umax));
 }
 
+// Force-kernel lanes per atom when the caller leaves the choice to the library
+// (threads_per_atom = 0), from the number of slots.  One lane per atom reads the fewest
+// lines per gather and folds nothing, so it wins as soon as the atoms alone fill the GPU;
+// below that more lanes per atom shorten the walk through a list.  In the FP64 form 1, 2
+// and 4 lanes give the same sums bit for bit (RowSplit): a batch's replicas equal their
+// single-system runs whatever the sizes.
+// Step times with 1, 2 and 4 lanes (LJ fluid, us): 4,000 atoms mixed 36, 32, 30 and FP64
+// 101, 66, 50; 32,000 atoms mixed 41, 40, 43 and FP64 172, 160, 166; 131,072 atoms mixed
+// 66, 70, 84 and FP64 537, 554, 565; 1,048,576 atoms mixed 299, 328, 449 and FP64 3935,
+// 4060, 4256.  8 lanes gain under 2% on the smallest systems.
+int default_tpa(int nslot) { return nslot >= 49152 ? 1 : nslot >= 24576 ? 2 : 4; }
+
 // Lay the replicas out (32-aligned slot ranges, consecutive cell ranges with one
 // padding cell each), allocate every per-slot array and upload the atoms.
 int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, const double *vel3,
@@ -674,6 +686,7 @@ int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, cons
   c->natoms = N;
   c->sc.n = NS;
   c->lc.n = NS;
+  if (!c->p.threads_per_atom) c->lc.tpa = c->d.tpa = default_tpa(NS);
   c->tc.n = N;
   c->tc.n_r_df = c->p.n_r_df;
   c->tc.k_b = c->p.k_b;

@@ -267,6 +267,89 @@ __device__ inline OneType one_type(const SmemTabF &tab) {
   return OneType{tab.rc2[0], tab.sig2[0], tab.eps4[0], tab.gc[0], tab.pk[0]};
 }
 
+// How an atom's row is split over lanes in the FP64 form.  Entry e of the row adds to
+// partial sum e mod 4, in row order; a lane holds all four sums (TPA 1), two of them (TPA
+// 2) or one (TPA >= 4: t mod 4, of the chunks t / 4, t / 4 + TPA / 4, ...).  Sums 0 and 1, 2
+// and 3 are added, then the two halves, then the lanes: 1, 2 and 4 lanes per atom give the
+// same sums bit for bit, so that the lane count may follow the size of a whole batch and
+// its replicas still equal their single-system runs.
+template <int TPA>
+struct RowSplit {
+  static constexpr int PER = TPA == 1 ? 4 : TPA == 2 ? 2 : 1;  // entries of a chunk a lane takes
+  static constexpr int STRIDE = TPA <= 4 ? 1 : TPA / 4;        // chunks a lane steps by
+  static __device__ __forceinline__ int first_chunk(int t) { return TPA <= 4 ? 0 : t >> 2; }
+  static __device__ __forceinline__ int first_entry(int t) { return TPA == 1 ? 0 : TPA == 2 ? 2 * t : t & 3; }
+};
+
+// FP64 pair loop of one lane (the entries RowSplit gives it).  ONE: single type, the pair
+// constants in registers, no table lookups; t1 = the atom's first table entry.  The
+// cutoff test r^2 <= rc^2 compares the bit patterns as integers (the same order for
+// doubles >= +0, and rc^2 < 0, an eps == 0 pair, admits none), off the FP64 pipe.
+template <int TPA, bool EV, bool ONE>
+__device__ __forceinline__ void fp64_pairs(const Dev &d, const uint4 *row4, int nn, int t, const dbl4 &xi, int t1,
+                                           const SmemTabD &tab, const double3 *img, double jump_tol, double (&F)[5]) {
+  using Split = RowSplit<TPA>;
+  constexpr int A = 32 / TPA, NV = EV ? 5 : 3, PER = Split::PER;
+  const bool jump = jump_tol > 0.0;
+  const long long rc2b1 = __double_as_longlong(tab.rc2[t1]);
+  const double sig21 = tab.sig2[t1], e61 = tab.e6[t1], e121 = tab.e12[t1], gc1 = tab.gc[t1];
+  const int e0 = Split::first_entry(t);
+  double P[PER][5];
+#pragma unroll
+  for (int u = 0; u < PER; ++u)
+#pragma unroll
+    for (int q = 0; q < 5; ++q) P[u][q] = 0.0;
+  const uint32_t *row = reinterpret_cast<const uint32_t *>(row4) + e0;
+  for (int g = Split::first_chunk(t); 4 * g + e0 < nn; g += Split::STRIDE) {
+    uint32_t e[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) e[u] = __ldg(row + (size_t)g * (4 * A) + u);
+    const int k0 = 4 * g + e0;
+    dbl4 xj[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u)
+      if (k0 + u < nn) xj[u] = ldg_dbl4(&d.pos[e[u] & IDX_MASK]);
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      if (k0 + u >= nn) break;
+      // image x_j + s L (the reference's ghost coordinate); s = 0 for most
+      // entries, where x_j + 0 is x_j exactly and the three adds are skipped
+      const int code = (int)(e[u] >> CODE_SHIFT);
+      double jx = xj[u].x, jy = xj[u].y, jz = xj[u].z;
+      if (code != CODE_ZERO) {
+        const double3 s = img[code];
+        jx += s.x; jy += s.y; jz += s.z;
+      }
+      const double dx = jx - xi.x, dy = jy - xi.y, dz = jz - xi.z;
+      const double r2d = dx * dx + dy * dy + dz * dz;
+      const int tt = ONE ? t1 : t1 + type_of(xj[u].w);
+      const long long rc2b = ONE ? rc2b1 : __double_as_longlong(tab.rc2[tt]);
+      if (__double_as_longlong(r2d) <= rc2b) {
+        // Lj jump_fix (src/force/lj.cpp:459-468): r^2 floored at jump_tol after the
+        // cutoff test (jump_tol = 0 when off); the direction stays dx, dy, dz
+        double r2 = r2d;
+        if (jump) r2 = r2d < jump_tol ? jump_tol : r2d;
+        const double r2i = rcp_nr(r2);
+        const double s2 = (ONE ? sig21 : tab.sig2[tt]) * r2i;
+        const double s6 = s2 * s2 * s2;
+        // eps4 s6 (6 - 12 s6) / r^2 - g(rc) as (s6 (e6 - e12 s6)) r2i - gc
+        const double coef = ONE ? fma(s6 * fma(-e121, s6, e61), r2i, -gc1)
+                                : fma(s6 * fma(-tab.e12[tt], s6, tab.e6[tt]), r2i, -tab.gc[tt]);
+        P[u][0] = fma(coef, dx, P[u][0]); P[u][1] = fma(coef, dy, P[u][1]); P[u][2] = fma(coef, dz, P[u][2]);
+        if (EV) {
+          P[u][3] -= coef * r2;
+          P[u][4] += tab.eps4[tt] * (s6 * s6 - s6) - tab.uc[tt] - 0.5 * tab.gc[tt] * (r2 - tab.rc2[tt]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NV; ++q)
+    F[q] = PER == 4   ? (P[0][q] + P[1 % PER][q]) + (P[2 % PER][q] + P[3 % PER][q])
+           : PER == 2 ? P[0][q] + P[1 % PER][q]
+                      : P[0][q];
+}
+
 // Folds the TPA lanes of each atom (lanes a, a+A, a+2A, ...; every lane of the warp
 // calls this) and applies the closing update of the step to atom i on lane t == 0.
 // KICK: 0 = store the acceleration only; 1 = velocity-Verlet closing kick
@@ -547,68 +630,23 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
     int ti = 0;
     if (act) {
       const int nn = d.nnbr[i];
-      // this lane's neighbour words: chunk g = t + TPA q (entries 4g..4g+3), one 128-bit
-      // load each; the warp's loads for one q cover 512 consecutive bytes (nbr_index)
-      const uint4 *row4 = reinterpret_cast<const uint4 *>(d.nbr + (size_t)task * cap * A) + (t * A + a);
+      // the atom's neighbour words: chunk g (entries 4g..4g+3) is row4[g * A] (nbr_index)
+      const uint4 *row4 = reinterpret_cast<const uint4 *>(d.nbr + (size_t)task * cap * A) + a;
       if constexpr (MIXED) {
         const int4 ri = d.ic[i];
         ti = ri.w;
         float ax = 0.f, ay = 0.f, az = 0.f, vr = 0.f, pp = 0.f;
         const int4 *ic = d.ic;
-        mixed_pairs<TPA, EV, ONE>(row4, nn, t, ri, nt, tab, one_type(tab), wimg[wid].hi, wimg[wid].lo, sc.jump_tolf,
+        mixed_pairs<TPA, EV, ONE>(row4 + t * A, nn, t, ri, nt, tab, one_type(tab), wimg[wid].hi, wimg[wid].lo, sc.jump_tolf,
                                   [ic](uint32_t w) { return __ldg(&ic[w & IDX_MASK]); }, ax, ay, az, vr, pp);
         fx = ax; fy = ay; fz = az; vir = vr; pe = pp;
       } else {
         const dbl4 xi = d.pos[i];
         ti = type_of(xi.w);
-        const bool jump = sc.jump_tol > 0.0;
-        // single type: the pair constants in registers, no table lookups; the cutoff
-        // test r^2 <= rc^2 compares the bit patterns as integers (the same order for
-        // doubles >= +0, and rc^2 < 0, an eps == 0 pair, admits none), off the FP64 pipe
-        const int t1 = ti * nt;
-        const long long rc2b1 = __double_as_longlong(tab.rc2[t1]);
-        const double sig21 = tab.sig2[t1], e61 = tab.e6[t1], e121 = tab.e12[t1], gc1 = tab.gc[t1];
-        for (int q = 0, k0 = 4 * t; k0 < nn; ++q, k0 += 4 * TPA) {
-          const uint4 w4 = __ldg(row4 + (size_t)q * 32);
-          const uint32_t e[4] = {w4.x, w4.y, w4.z, w4.w};
-          dbl4 xj[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (k0 + u < nn) xj[u] = ldg_dbl4(&d.pos[e[u] & IDX_MASK]);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (k0 + u >= nn) break;
-            // image x_j + s L (the reference's ghost coordinate); s = 0 for most
-            // entries, where x_j + 0 is x_j exactly and the three adds are skipped
-            const int code = (int)(e[u] >> CODE_SHIFT);
-            double jx = xj[u].x, jy = xj[u].y, jz = xj[u].z;
-            if (code != CODE_ZERO) {
-              const double3 s = wimg[wid].v[code];
-              jx += s.x; jy += s.y; jz += s.z;
-            }
-            const double dx = jx - xi.x, dy = jy - xi.y, dz = jz - xi.z;
-            const double r2d = dx * dx + dy * dy + dz * dz;
-            const int tt = ONE ? t1 : t1 + type_of(xj[u].w);
-            const long long rc2b = ONE ? rc2b1 : __double_as_longlong(tab.rc2[tt]);
-            if (__double_as_longlong(r2d) <= rc2b) {
-              // Lj jump_fix (src/force/lj.cpp:459-468): r^2 floored at jump_tol after the
-              // cutoff test (jump_tol = 0 when off); the direction stays dx, dy, dz
-              double r2 = r2d;
-              if (jump) r2 = r2d < sc.jump_tol ? sc.jump_tol : r2d;
-              const double r2i = rcp_nr(r2);
-              const double s2 = (ONE ? sig21 : tab.sig2[tt]) * r2i;
-              const double s6 = s2 * s2 * s2;
-              // eps4 s6 (6 - 12 s6) / r^2 - g(rc) as (s6 (e6 - e12 s6)) r2i - gc
-              const double coef = ONE ? fma(s6 * fma(-e121, s6, e61), r2i, -gc1)
-                                      : fma(s6 * fma(-tab.e12[tt], s6, tab.e6[tt]), r2i, -tab.gc[tt]);
-              fx = fma(coef, dx, fx); fy = fma(coef, dy, fy); fz = fma(coef, dz, fz);
-              if (EV) {
-                vir -= coef * r2;
-                pe += tab.eps4[tt] * (s6 * s6 - s6) - tab.uc[tt] - 0.5 * tab.gc[tt] * (r2 - tab.rc2[tt]);
-              }
-            }
-          }
-        }
+        double F[5];
+        fp64_pairs<TPA, EV, ONE>(d, row4, nn, t, xi, ti * nt, tab, wimg[wid].v, sc.jump_tol, F);
+        fx = F[0]; fy = F[1]; fz = F[2];
+        if (EV) vir = F[3], pe = F[4];
       }
     }
     double ke_t[4] = {0.0, 0.0, 0.0, 0.0}, ev_t[2] = {0.0, 0.0};
