@@ -95,6 +95,7 @@ struct cavgpu_ctx {
   long long prof_launches = 0;
   // allocations
   std::vector<void *> allocs;
+  void *x_mem = nullptr;  // FP64 pair exchange
   size_t nbr_bytes = 0;
 };
 
@@ -142,7 +143,7 @@ int enqueue_thermo_after_force(cavgpu_ctx *c, int ring_slot, long long *nl) {
   const bool lang = is_lang(c);
   if (c->b.nrep == 1) {
     const int nb_ke = lang ? drift_grid_blocks(c->lc) : force_grid_blocks(c->lc);
-    RK(launch_thermo_final(c->d, c->tc, nb_ke, force_grid_blocks(c->lc), lang ? force_grid_blocks(c->lc) : 0,
+    RK(launch_thermo_final(c->d, c->tc, nb_ke, ev_grid_blocks(c->lc), lang ? force_grid_blocks(c->lc) : 0,
                            ring_slot, c->st));
   } else {
     RK(launch_thermo_replicas(c->d, c->b, c->tc, lang ? 0 : 1, 1, c->st));
@@ -255,7 +256,7 @@ int enqueue_chunk(cavgpu_ctx *c, const ChunkPlan &pl, bool capture, long long *l
         nl += 1;
       }
       RK(launch_rebuild(view, c->b, c->lc, 0, c->st));
-      nl += rebuild_kernels(c->b);
+      nl += rebuild_kernels(c->b, c->lc);
     }
     const int fuse = pl.fuse[k] ? fuse_mode(c) : FUSE_NONE;
     int set_cond = 0;
@@ -271,14 +272,14 @@ int enqueue_chunk(cavgpu_ctx *c, const ChunkPlan &pl, bool capture, long long *l
       CK(capture ? cudaEventRecordWithFlags(c->ev0[k], c->st, cudaEventRecordExternal) : cudaEventRecord(c->ev0[k], c->st));
     // a recorded step of a single system: the pair kernel's last block folds the record
     const bool fold = th && c->b.nrep == 1 && c->nve.step == 0;
-    FoldArgs fa{c->tc, is_lang(c) ? drift_grid_blocks(c->lc) : force_grid_blocks(c->lc),
+    FoldArgs fa{c->tc, is_lang(c) ? drift_grid_blocks(c->lc) : force_grid_blocks(c->lc), ev_grid_blocks(c->lc),
                 is_lang(c) ? force_grid_blocks(c->lc) : 0, ring_slot};
     RK(launch_force(view, c->b, c->sc, c->lc, is_lang(c) ? 2 : 1, th, k, fuse, set_cond, hnext, c->st,
                     fold ? &fa : nullptr));
     if (c->prof && k < (int)c->ev1.size())
       CK(capture ? cudaEventRecordWithFlags(c->ev1[k], c->st, cudaEventRecordExternal) : cudaEventRecord(c->ev1[k], c->st));
-    nl += 1;
-    if (fuse) {  // the next step gathers the coordinates this launch wrote
+    nl += force_kernels(c->lc);
+    if (fuse && !c->lc.exchange) {  // the next step gathers the coordinates this launch wrote
       if (mixed) std::swap(view.ic, view.ic_alt);
       else std::swap(view.pos, view.pos_alt);
     }
@@ -353,6 +354,45 @@ int check_status(cavgpu_ctx *c) {
   return CAVGPU_OK;
 }
 
+// (Re)allocate the arrays of the FP64 pair exchange for the list's capacity: half of it
+// per atom each way, and no less than 64 of a capacity of 64 (an atom claims half its
+// entries and receives the other half; a row that outgrows this grows the list).  38 bytes
+// per entry, ~3.7 KB per atom of the benchmark fluid: a system for which that is more than a quarter of the device's
+// memory, or more than is free, evaluates its pairs from both sides over the full list
+// instead (k_force), at about twice the time and the same precision.
+int alloc_exchange(cavgpu_ctx *c) {
+  Dev &d = c->d;
+  if (c->x_mem) cudaFree(c->x_mem);
+  c->x_mem = nullptr;
+  d.hw = nullptr; d.hslot = nullptr; d.nh = d.nr = nullptr; d.recv = d.own = nullptr; d.ic = nullptr; d.ev_part = nullptr;
+  c->lc.exchange = 0;
+  if (d.tpa > 4) return CAVGPU_OK;  // four partial sums: at most four lanes per atom
+  const size_t n = ((size_t)c->b.nslot + 31) / 32 * 32, cap_h = (size_t)std::max(std::min(d.cap, 64), d.cap / 2);
+  const size_t recv = n * cap_h * sizeof(dbl4), words = n * cap_h * sizeof(uint32_t), slots = n * cap_h * sizeof(uint16_t);
+  const size_t evp = c->b.nrep > 1 ? n * d.tpa * sizeof(double2) : 0;
+  const size_t bytes = recv + 4 * n * sizeof(dbl4) + evp + words + slots + n * sizeof(int4) + 2 * n * sizeof(int);
+  size_t free_mem = 0, total_mem = 0;
+  CK(cudaMemGetInfo(&free_mem, &total_mem));
+  if (bytes > total_mem / 4) return CAVGPU_OK;
+  void *q = nullptr;
+  if (cudaMalloc(&q, bytes) != cudaSuccess) { cudaGetLastError(); return CAVGPU_OK; }
+  c->x_mem = q;
+  char *p = static_cast<char *>(q);
+  auto take = [&](size_t nb) { char *r = p; p += nb; return r; };
+  d.recv = reinterpret_cast<dbl4 *>(take(recv));
+  d.own = reinterpret_cast<dbl4 *>(take(4 * n * sizeof(dbl4)));
+  if (evp) d.ev_part = reinterpret_cast<double2 *>(take(evp));
+  d.ic = reinterpret_cast<int4 *>(take(n * sizeof(int4)));
+  d.hw = reinterpret_cast<uint32_t *>(take(words));
+  d.nh = reinterpret_cast<int *>(take(n * sizeof(int)));
+  d.nr = reinterpret_cast<int *>(take(n * sizeof(int)));
+  d.hslot = reinterpret_cast<uint16_t *>(take(slots));
+  d.cap_h = (int)cap_h;
+  c->lc.exchange = 1;
+  CK(cudaMemsetAsync(d.nh, 0, 2 * n * sizeof(int), c->st));  // padding slots keep 0
+  return CAVGPU_OK;
+}
+
 // (re)allocate the neighbour list for `cap` slots per atom
 int alloc_nbr(cavgpu_ctx *c, int cap) {
   cap = (cap + 63) / 64 * 64;  // nbr_index needs cap % (4 * tpa) == 0, tpa <= 16
@@ -370,6 +410,7 @@ int alloc_nbr(cavgpu_ctx *c, int cap) {
   c->d.nbr = static_cast<uint32_t *>(q);
   c->d.cap = cap;
   c->nbr_bytes = bytes;
+  if (c->p.precision == CAVGPU_FP64) RK(alloc_exchange(c));
   free_graphs(c);  // graphs hold the old Dev by value
   return CAVGPU_OK;
 }
@@ -390,7 +431,7 @@ int forced_build(cavgpu_ctx *c, bool count = true) {
     zero[F_PASSES] = f[F_PASSES];
     CK(cudaMemcpyAsync(c->d.flags, zero, sizeof(zero), cudaMemcpyHostToDevice, c->st));
     RK(launch_rebuild(c->d, c->b, c->lc, 1, c->st));
-    c->kernel_launches += rebuild_kernels(c->b);
+    c->kernel_launches += rebuild_kernels(c->b, c->lc);
     RK(read_flags(c, f));
     c->max_nb = f[F_MAXNB];
     if (!f[F_OVERFLOW]) {
@@ -489,6 +530,14 @@ int create_common(const cavgpu_params *p, int nrep, const double *lo3, const dou
       const double sc2 = rc2 > 0 ? sig * sig / rc2 : 0.0, sc6 = sc2 * sc2 * sc2;
       t.gc[k] = rc2 > 0 ? 4.0 * eps * sc6 * (6.0 - 12.0 * sc6) / rc2 : 0.0;
       t.uc[k] = 4.0 * eps * (sc6 * sc6 - sc6);
+      const long double s6 = (long double)sig * sig * sig * sig * sig * sig, e4 = 4.0L * eps;
+      t.l12[k] = (double)(e4 * s6 * s6);
+      t.l6[k] = (double)(e4 * s6);
+      t.w12[k] = (double)(-12.0L * e4 * s6 * s6);
+      t.w6[k] = (double)(6.0L * e4 * s6);
+      // the screen's margin: 1e-5 relative against FP32 rounding, four coordinate units
+      const double rs = (rc + 4.0 * unit) * (1.0 + 1e-5);
+      t.screen[k] = eps == 0.0 ? -1.0f : (float)(rs * rs);
     }
   for (int a = 0; a < nt; ++a) {
     t.mass[a] = p->mass[a];
@@ -709,6 +758,8 @@ int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, cons
         t.block = blk;
         t.use_seg = seg;
         nblk = std::max(nblk, (size_t)force_grid_blocks(t));
+        t.exchange = c->p.precision == CAVGPU_FP64;
+        nblk = std::max({nblk, (size_t)force_grid_blocks(t), (size_t)ev_grid_blocks(t)});
       }
   const size_t nblk_d = (size_t)std::max((NS + 255) / 256, 1);
   d.partials_blocks = (int)nblk;
@@ -836,9 +887,9 @@ int setup_common(cavgpu_ctx *c) {
   if (!c->uploaded) return CAVGPU_E_STATE;
   RK(forced_build(c));
   RK(launch_force(c->d, c->b, c->sc, c->lc, 0, 1, 0, FUSE_NONE, 0, 0, c->st));
-  c->kernel_launches += 1;
+  c->kernel_launches += force_kernels(c->lc);
   if (c->b.nrep == 1) {
-    RK(launch_thermo_final(c->d, c->tc, force_grid_blocks(c->lc), force_grid_blocks(c->lc), 0, -1, c->st));
+    RK(launch_thermo_final(c->d, c->tc, force_grid_blocks(c->lc), ev_grid_blocks(c->lc), 0, -1, c->st));
   } else {
     RK(launch_thermo_replicas(c->d, c->b, c->tc, 1, 1, c->st));
   }
@@ -867,7 +918,8 @@ int ensure_status(cavgpu_ctx *c) {
 int complete_overflowed_step(cavgpu_ctx *c, const ChunkPlan &pl, int k, int64_t g, int64_t nsteps, int64_t every,
                              double *out5, int need) {
   if (pl.fused_before(k) & 1) {
-    if (c->p.precision == CAVGPU_FP64)  // (mixed: the build derives the coordinates from the positions)
+    // (the mixed form's build derives its coordinates from the positions; the exchange drifts in place)
+    if (c->p.precision == CAVGPU_FP64 && !c->lc.exchange)
       CK(cudaMemcpyAsync(c->d.pos, c->d.pos_alt, (size_t)c->b.nslot * sizeof(dbl4), cudaMemcpyDeviceToDevice, c->st));
   }
   RK(alloc_nbr(c, (int)(need * 1.25) + 32));
@@ -876,7 +928,7 @@ int complete_overflowed_step(cavgpu_ctx *c, const ChunkPlan &pl, int k, int64_t 
   const int ring_slot = (th && every > 0) ? 0 : -1;
   long long nl = 0;
   RK(launch_force(c->d, c->b, c->sc, c->lc, is_lang(c) ? 2 : 1, th, 0, FUSE_NONE, 0, 0, c->st));
-  nl += 1;
+  nl += force_kernels(c->lc);
   if (th) RK(enqueue_thermo_after_force(c, ring_slot, &nl));
   if (c->nve.step > 0 && !is_lang(c)) {
     RK(launch_nve(c->d, c->b, c->tc, c->nve, 0, th, ring_slot, c->st));
@@ -991,7 +1043,7 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
   // rebuild kernels launched by the graphs' conditional nodes
   if (!eager) {
     RK(read_flags(c, f));
-    if (f[F_PASSES] > passes0) c->kernel_launches += (long long)rebuild_kernels(c->b) * (f[F_PASSES] - passes0);
+    if (f[F_PASSES] > passes0) c->kernel_launches += (long long)rebuild_kernels(c->b, c->lc) * (f[F_PASSES] - passes0);
   }
   return CAVGPU_OK;
 }
@@ -1055,6 +1107,7 @@ void cavgpu_destroy(cavgpu_ctx *c) {
   for (auto e : c->ev_status) if (e) cudaEventDestroy(e);
   if (c->h_status) cudaFreeHost(c->h_status);
   for (void *q : c->allocs) cudaFree(q);
+  if (c->x_mem) cudaFree(c->x_mem);
   if (c->st) cudaStreamDestroy(c->st);
   if (c->side) cudaStreamDestroy(c->side);
   delete c;
@@ -1270,9 +1323,9 @@ int cavgpu_forces(cavgpu_ctx *c, double *virial, double *pe) {
   if (!c->set_up) return CAVGPU_E_STATE;
   RK(forced_build(c));
   RK(launch_force(c->d, c->b, c->sc, c->lc, 0, 1, 0, FUSE_NONE, 0, 0, c->st));
-  c->kernel_launches += 1;
+  c->kernel_launches += force_kernels(c->lc);
   if (c->b.nrep == 1) {
-    RK(launch_thermo_final(c->d, c->tc, force_grid_blocks(c->lc), force_grid_blocks(c->lc), 0, -1, c->st));
+    RK(launch_thermo_final(c->d, c->tc, force_grid_blocks(c->lc), ev_grid_blocks(c->lc), 0, -1, c->st));
   } else {
     RK(launch_thermo_replicas(c->d, c->b, c->tc, 1, 1, c->st));
   }

@@ -85,6 +85,10 @@ enum Fuse : int { FUSE_NONE = 0, FUSE_VV = 1, FUSE_LF = 2, FUSE_LANG = 3 };
 // rc2 < 0 marks an eps == 0 pair (skipped, src/force/lj.cpp:471-472).
 struct PairTab {
   double rc2[MAXT * MAXT], sig2[MAXT * MAXT], eps4[MAXT * MAXT], gc[MAXT * MAXT], uc[MAXT * MAXT];
+  // powers folded in (cav_exchange.cu): l12 = eps4 sig^12, l6 = eps4 sig^6, w12 = -12 l12,
+  // w6 = 6 l6, each rounded once; screen: r^2 beyond which the FP32 screen drops a pair
+  double l12[MAXT * MAXT], l6[MAXT * MAXT], w12[MAXT * MAXT], w6[MAXT * MAXT];
+  float screen[MAXT * MAXT];
   double minv[MAXT], mass[MAXT];
   int nt;
 };
@@ -138,8 +142,8 @@ struct Dev {
   // the velocity-Verlet kick reads it as a_old (leap-frog's drift zeroes it)
   dbl4 *pos, *vel, *acc, *pos_ref;
   float4 *rel;                // position at the last build relative to the build cell's origin; w = type bits
-  int4 *ic;                   // mixed form: fixed-point coordinates (to_fixed); w = type
-  int4 *ic_ref;               // ic at the last build (half-skin test)
+  int4 *ic;                   // fixed-point coordinates (to_fixed), w = type: the mixed form's, the FP64 screen's
+  int4 *ic_ref;               // mixed form: ic at the last build (half-skin test)
   // the coordinates a pair kernel gathers from its neighbours, for the next step: a pair
   // kernel that also drifts its atoms writes them here (FP64 form: positions; mixed
   // form: ic), while other atoms still read the current ones, and the two swap
@@ -164,6 +168,14 @@ struct Dev {
   int *nnbr;
   int cap;                    // slots per atom (multiple of 64)
   int tpa;                    // force-kernel lanes per atom (fixes the list layout)
+  // FP64 pair exchange (cav_exchange.cu; all null when it is off)
+  uint32_t *hw;               // list words of the entries an atom claimed (layout of nbr with cap_h)
+  uint16_t *hslot;            // and the receiving slot of each at the other atom
+  int *nh, *nr;               // entries claimed, forces received
+  dbl4 *recv;                 // received forces, cap_h per atom (recv_index)
+  dbl4 *own;                  // the four partial sums over the claimed pairs
+  double2 *ev_part;           // batches: {virial, PE} of the claimed pairs per lane of an atom
+  int cap_h;
   // status, reductions
   int *flags;
   double *partials_ke;        // per-block {sum m v^2, sum m v} (4 per block)
@@ -272,6 +284,7 @@ __device__ inline void langevin_eta_f(uint64_t seed, long long step, uint32_t id
 // FP64 form: the reference's expression orders (src/md_simulator.cpp:654, 898-899,
 // 765, 822-827), no contraction, so that equal forces give equal trajectories.
 // Mixed form: FMAs (the FP64 pipe of these updates is their scarcest resource).
+// (a*0.5)*dt is taken as a*hdt: both halvings are exact, so the products round alike.
 
 // velocity Verlet: pos += vel*dt + ((acc*0.5)*dt)*dt
 template <bool MIXED>
@@ -281,9 +294,9 @@ __device__ __forceinline__ void drift_vv(dbl4 &x, const dbl4 &v, const dbl4 &a, 
     x.y = fma(a.y, sc.hdt2, fma(v.y, sc.dt, x.y));
     x.z = fma(a.z, sc.hdt2, fma(v.z, sc.dt, x.z));
   } else {
-    x.x = __dadd_rn(x.x, __dadd_rn(__dmul_rn(v.x, sc.dt), __dmul_rn(__dmul_rn(__dmul_rn(a.x, 0.5), sc.dt), sc.dt)));
-    x.y = __dadd_rn(x.y, __dadd_rn(__dmul_rn(v.y, sc.dt), __dmul_rn(__dmul_rn(__dmul_rn(a.y, 0.5), sc.dt), sc.dt)));
-    x.z = __dadd_rn(x.z, __dadd_rn(__dmul_rn(v.z, sc.dt), __dmul_rn(__dmul_rn(__dmul_rn(a.z, 0.5), sc.dt), sc.dt)));
+    x.x = __dadd_rn(x.x, __dadd_rn(__dmul_rn(v.x, sc.dt), __dmul_rn(__dmul_rn(a.x, sc.hdt), sc.dt)));
+    x.y = __dadd_rn(x.y, __dadd_rn(__dmul_rn(v.y, sc.dt), __dmul_rn(__dmul_rn(a.y, sc.hdt), sc.dt)));
+    x.z = __dadd_rn(x.z, __dadd_rn(__dmul_rn(v.z, sc.dt), __dmul_rn(__dmul_rn(a.z, sc.hdt), sc.dt)));
   }
 }
 
@@ -312,9 +325,9 @@ __device__ __forceinline__ void lang_half(dbl4 &v, const dbl4 &a, double e0, dou
     v.y = fma(a.y, sc.hdt, fma(e1, sc.lb, v.y));
     v.z = fma(a.z, sc.hdt, fma(e2, sc.lb, v.z));
   } else {
-    v.x = __dadd_rn(v.x, __dadd_rn(__dmul_rn(__dmul_rn(a.x, 0.5), sc.dt), __dmul_rn(e0, sc.lb)));
-    v.y = __dadd_rn(v.y, __dadd_rn(__dmul_rn(__dmul_rn(a.y, 0.5), sc.dt), __dmul_rn(e1, sc.lb)));
-    v.z = __dadd_rn(v.z, __dadd_rn(__dmul_rn(__dmul_rn(a.z, 0.5), sc.dt), __dmul_rn(e2, sc.lb)));
+    v.x = __dadd_rn(v.x, __dadd_rn(__dmul_rn(a.x, sc.hdt), __dmul_rn(e0, sc.lb)));
+    v.y = __dadd_rn(v.y, __dadd_rn(__dmul_rn(a.y, sc.hdt), __dmul_rn(e1, sc.lb)));
+    v.z = __dadd_rn(v.z, __dadd_rn(__dmul_rn(a.z, sc.hdt), __dmul_rn(e2, sc.lb)));
   }
 }
 
@@ -335,14 +348,7 @@ __device__ inline void request_rebuild(const Dev &d, const Box &b, int rep) {
   d.flags[F_REBUILD] = 1;
 }
 
-// Half-skin test of the reference (src/neighborlist.cpp:134-143), FP64 form.
-__device__ inline void half_skin_test(const Dev &d, const Box &b, int rep, int i, const dbl4 &x) {
-  const dbl4 r = d.pos_ref[i];
-  const double dx = x.x - r.x, dy = x.y - r.y, dz = x.z - r.z;
-  if (dx * dx + dy * dy + dz * dz > b.thr2) request_rebuild(d, b, rep);
-}
-
-// Fixed-point coordinates of the mixed form.  Along an axis the box is cut into m
+// Fixed-point coordinates.  Along an axis the box is cut into m
 // windows of length W = L / m (m = 1 for a box below two windows of 4 list cutoffs)
 // and the coordinate is the position modulo W in units of W / 2^32, as a 32-bit
 // integer that wraps by itself: the difference of two atoms' integers is their
@@ -375,6 +381,20 @@ __device__ __forceinline__ bool beyond_window(int q, int qw, int r, int rw) {
   return ((high - (fixed_diff(q, r) >> 31)) & 1023) != 0;
 }
 
+// Half-skin test of the reference (src/neighborlist.cpp:134-143), FP64 form, and the
+// fixed-point coordinates of its screen.
+__device__ inline void half_skin_test(const Dev &d, const Box &b, int rep, int i, const dbl4 &x) {
+  const dbl4 r = d.pos_ref[i];
+  const double dx = x.x - r.x, dy = x.y - r.y, dz = x.z - r.z;
+  // compared as bit patterns (the order of doubles >= +0; a NaN counts as beyond), off the FP64 pipe
+  if ((__double_as_longlong(dx * dx + dy * dy + dz * dz) & 0x7fffffffffffffffll) > __double_as_longlong(b.thr2))
+    request_rebuild(d, b, rep);
+  if (d.ic) {
+    int3 w;
+    d.ic[i] = fixed_pos(repbox(b, rep), x, type_of(x.w), w);
+  }
+}
+
 // Mixed form: the new fixed-point coordinates, written to `out`, and the half-skin
 // test on their difference to those of the last build (in FP32 against a threshold
 // shrunk by the units' rounding and 1e-6, so it can only fire early; the window
@@ -392,7 +412,9 @@ __device__ inline void mixed_track(const Dev &d, const Box &b, int rep, int i, c
 }
 
 __device__ inline void nan_check(const Dev &d, int i, const dbl4 &a) {
-  if (isnan(a.x) || isnan(a.y) || isnan(a.z)) {
+  // on the bit patterns: comparing doubles would take the FP64 pipe
+  auto nan = [](double v) { return (unsigned long long)(__double_as_longlong(v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ull; };
+  if (nan(a.x) || nan(a.y) || nan(a.z)) {
     d.flags[F_NAN] = 1;
     d.flags[F_NAN_ATOM] = (int)d.id[i];
   }
@@ -409,7 +431,8 @@ struct LaunchCfg {
   int n;           // slots
   int nseg;        // row segments (mixed form; 0 = none)
   int use_seg;     // mixed form: run the segment kernel (shared-memory stage)
-  int ntypes;      // 1: the mixed kernels keep the pair constants in registers
+  int ntypes;      // 1: the kernels keep the pair constants in registers
+  int exchange;    // FP64 form: pairs evaluated once, two kernels per force (cav_exchange.cu)
 };
 
 struct ThermoCfg {
@@ -441,6 +464,7 @@ __device__ inline void thermo_finish(double ke2, const double P3[3], double msum
 // whose half-skin test did not fire.
 int drift_grid_blocks(const LaunchCfg &lc);
 int force_grid_blocks(const LaunchCfg &lc);
+int ev_grid_blocks(const LaunchCfg &lc);  // blocks that leave virial and PE partials
 // sets the dynamic shared-memory limit of every segment-kernel variant (call outside capture)
 int prepare_force_seg(size_t smem_bytes);
 // thermo < 0 (Langevin): the velocity half only; launch_lang_pos then moves the atoms
@@ -456,7 +480,9 @@ int launch_halt_check(const Dev &d, cudaStream_t st);
 constexpr int SCAN_SLICES = 64;
 inline int scan_slices(const Box &b) { return b.nrep == 1 ? SCAN_SLICES : 1; }
 // kernels launch_rebuild enqueues
-inline int rebuild_kernels(const Box &b) { return 8 + (scan_slices(b) > 1 ? 1 : 0); }
+inline int rebuild_kernels(const Box &b, const LaunchCfg &lc) { return 8 + (scan_slices(b) > 1 ? 1 : 0) + (lc.exchange ? 2 : 0); }
+// kernels one force evaluation launches
+inline int force_kernels(const LaunchCfg &lc) { return lc.exchange ? 2 : 1; }
 // kick: 0 = force only, 1 = VV closing kick, 2 = Langevin closing update.
 // thermo: virial/PE partials (and KE partials unless kick == 2).
 // fuse (Fuse): the next step's drift in the same launch, written to d.pos_alt (FP64)
@@ -466,13 +492,20 @@ inline int rebuild_kernels(const Box &b) { return 8 + (scan_slices(b) > 1 ? 1 : 
 // step (F_STEPS_OK) and raises the halt on a NaN.
 // The thermo fold of a recorded step done by the pair kernel's last block (single
 // systems): the fixed-order sums of the KE partials (nb_ke blocks; Langevin: the
-// drift kernel's) and of the launch's own virial/PE partials (and, Langevin, of its
+// drift kernel's) and of the launch's own virial/PE partials (nb_ev; and, Langevin, of its
 // end-of-step KE partials, nb_ke_end), then the record -- what launch_thermo_final
 // does after the launch, without its launch.
 struct FoldArgs {
   ThermoCfg tc;
-  int nb_ke, nb_ke_end, ring_slot;
+  int nb_ke, nb_ev, nb_ke_end, ring_slot;
 };
+// the pair exchange: its part of a list build, its two kernels, their block size
+struct ForceArgs;
+int launch_exchange_build(const Dev &d, const Box &b, int forced, cudaStream_t st);
+int launch_force_exchange(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int kick, bool ev,
+                          const ForceArgs &fa, int grid, int grid_ev, cudaStream_t st);
+int exchange_pair_blocks(int ntask, int sms);
+int exchange_close_threads();
 int launch_force(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int kick, int thermo,
                  int k_in_chunk, int fuse, int set_cond, cudaGraphConditionalHandle cond, cudaStream_t st,
                  const FoldArgs *fold = nullptr);

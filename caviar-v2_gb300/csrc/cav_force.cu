@@ -8,6 +8,8 @@
 //   MIXED : FP32 pair arithmetic on exact differences of fixed-point coordinates
 //           (int4 x,y,z,type; to_fixed), FP64 accumulation across lanes, FP64
 //           acceleration/velocity/reductions.
+#include <algorithm>
+
 #include "cav_pair.cuh"
 
 namespace cav {
@@ -596,25 +598,33 @@ int force_grid_blocks(const LaunchCfg &lc) {
   }
   if (lc.precision == CAVGPU_MIXED && lc.use_seg && lc.nseg > 0)  // one segment per block at a time
     return lc.nseg < g_num_sms * 4 ? lc.nseg : g_num_sms * 4;
-  const int A = 32 / lc.tpa;
+  const int A = 32 / lc.tpa, block = lc.exchange ? exchange_close_threads() : lc.block;
   const long long ntask = (lc.n + A - 1) / A;
-  const long long warps_per_block = lc.block / 32;
+  const long long warps_per_block = block / 32;
   long long need = (ntask + warps_per_block - 1) / warps_per_block;
   // the mixed kernels (64 registers) hold 32 warps per SM: one wave of resident blocks,
   // each warp walking its tasks grid-strided (fewer, longer-lived blocks: fewer block
   // reductions and tails; 5% less pair-kernel time and 16% less for the thermo
   // variant on the 1M-atom fluid than four waves); the FP64 kernels: four waves
-  const long long cap = lc.precision == CAVGPU_MIXED ? (long long)g_num_sms * (1024 / lc.block)
-                                                     : (long long)g_num_sms * (2048 / lc.block) * 4;
+  const long long cap = lc.precision == CAVGPU_MIXED ? (long long)g_num_sms * (1024 / block)
+                                                     : (long long)g_num_sms * (2048 / block) * 4;
   if (need > cap) need = cap;
   return (int)(need < 1 ? 1 : need);
+}
+
+int ev_grid_blocks(const LaunchCfg &lc) {
+  if (!lc.exchange) return force_grid_blocks(lc);
+  force_grid_blocks(lc);  // (the SM count)
+  const int A = 32 / lc.tpa;
+  return exchange_pair_blocks((lc.n + A - 1) / A, g_num_sms);
 }
 
 int launch_force(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int kick, int thermo,
                  int k, int fuse, int set_cond, cudaGraphConditionalHandle cond, cudaStream_t st,
                  const FoldArgs *fold) {
   const int grid = force_grid_blocks(lc);
-  if (grid > d.partials_blocks) return CAVGPU_E_ARG;  // each block writes its own partial sums
+  const int grid_ev = ev_grid_blocks(lc);
+  if (std::max(grid, grid_ev) > d.partials_blocks) return CAVGPU_E_ARG;  // each block writes its own partial sums
   if (kick == 0 && (fuse || set_cond)) return CAVGPU_E_ARG;
   if (fold && (kick == 0 || !thermo)) return CAVGPU_E_ARG;  // the fold needs this launch's EV partials
   ForceArgs fa{k, fuse, set_cond, cond, fold ? 1 : 0, {}};
@@ -624,6 +634,9 @@ int launch_force(const Dev &d, const Box &b, const StepConsts &sc, const LaunchC
     if (!d.seg || d.nseg != lc.nseg) return CAVGPU_E_ARG;
     rc = seg_tpa(true, lc.tpa, kick, thermo != 0, lc.ntypes == 1, grid, lc.block,
                  seg_smem_bytes(d.stage_cap, d.seg_umax), d, b, sc, fa, st);
+  } else if (lc.exchange) {
+    if (!d.recv) return CAVGPU_E_ARG;
+    rc = launch_force_exchange(d, b, sc, lc, kick, thermo != 0, fa, grid, grid_ev, st);
   } else {
     const bool one = lc.ntypes == 1;
     rc = lc.precision == CAVGPU_MIXED

@@ -389,8 +389,9 @@ __global__ void __launch_bounds__(256) k_gather(Dev d, Box b, int forced) {
     int3 w;
     const int4 q = fixed_pos(rb, x, type_of(x.w), w);
     d.ic[k] = q;
-    d.ic_ref[k] = fixed_ref(q, w);
+    if (d.ic_ref) d.ic_ref[k] = fixed_ref(q, w);
   }
+  if (d.nr) d.nr[k] = 0;
 }
 
 // Verlet-list build over the 27-cell stencil with periodic image shifts.
@@ -1222,6 +1223,10 @@ int launch_rebuild(const Dev &d, const Box &b, const LaunchCfg &lc, int forced, 
   const int build_grid = std::min(ceil_div(ceil_div(b.nslot, 32), BUILD_WARPS), num_sms() * 8);
   if (lc.precision == CAVGPU_MIXED) k_build_group<1><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
   else k_build_group<0><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
+  if (lc.exchange) {
+    const int rc = launch_exchange_build(d, b, forced, st);
+    if (rc) return rc;
+  }
   k_finish_rebuild<<<1, 256, 0, st>>>(d, b, forced);
   return chk();
 }

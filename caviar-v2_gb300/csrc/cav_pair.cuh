@@ -162,9 +162,9 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
       v.y = fma(an.y, sc.hdt, fma(v.y, sc.la, e1 * sc.lb));
       v.z = fma(an.z, sc.hdt, fma(v.z, sc.la, e2 * sc.lb));
     } else {  // v = (v a + eta b) + (a*0.5) dt, the reference's order
-      v.x = __dadd_rn(__dadd_rn(__dmul_rn(v.x, sc.la), __dmul_rn(e0, sc.lb)), __dmul_rn(__dmul_rn(an.x, 0.5), sc.dt));
-      v.y = __dadd_rn(__dadd_rn(__dmul_rn(v.y, sc.la), __dmul_rn(e1, sc.lb)), __dmul_rn(__dmul_rn(an.y, 0.5), sc.dt));
-      v.z = __dadd_rn(__dadd_rn(__dmul_rn(v.z, sc.la), __dmul_rn(e2, sc.lb)), __dmul_rn(__dmul_rn(an.z, 0.5), sc.dt));
+      v.x = __dadd_rn(__dadd_rn(__dmul_rn(v.x, sc.la), __dmul_rn(e0, sc.lb)), __dmul_rn(an.x, sc.hdt));
+      v.y = __dadd_rn(__dadd_rn(__dmul_rn(v.y, sc.la), __dmul_rn(e1, sc.lb)), __dmul_rn(an.y, sc.hdt));
+      v.z = __dadd_rn(__dadd_rn(__dmul_rn(v.z, sc.la), __dmul_rn(e2, sc.lb)), __dmul_rn(an.z, sc.hdt));
     }
     if (EV) {  // Atom_data::kinetic_energy() read after the step (the temperature was taken mid-step)
       const double m = tab.mass[ti];
@@ -252,10 +252,10 @@ __device__ __forceinline__ void fold_strided(const double *p, int n, double *v) 
 // The thermo fold in the last block: every thread sums a strided subset of the
 // partials, the block folds the threads' sums in a fixed order, thread 0 finishes
 // the record.  The sums do not depend on which block finished last.
-static __device__ __noinline__ void fold_thermo(const Dev &d, const FoldArgs &fa, int nb_ev) {
+static __device__ __noinline__ void fold_thermo(const Dev &d, const FoldArgs &fa) {
   double v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   fold_strided<4>(d.partials_ke, fa.nb_ke, v);
-  fold_strided<2>(d.partials_ev, nb_ev, v + 4);
+  fold_strided<2>(d.partials_ev, fa.nb_ev, v + 4);
   fold_strided<4>(d.partials_ke_end, fa.nb_ke_end, v + 6);
   __shared__ double out[10];
   block_sum_store_f<10>(v, out);
@@ -309,7 +309,7 @@ __device__ __forceinline__ void end_of_step(const Dev &d, bool was_halted, const
   }
   __syncthreads();
   if constexpr (EV) {
-    if (s_fold) fold_thermo(d, fa.fa, gridDim.x);
+    if (s_fold) fold_thermo(d, fa.fa);
   }
 }
 
