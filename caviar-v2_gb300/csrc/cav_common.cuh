@@ -480,7 +480,7 @@ int launch_halt_check(const Dev &d, cudaStream_t st);
 constexpr int SCAN_SLICES = 64;
 inline int scan_slices(const Box &b) { return b.nrep == 1 ? SCAN_SLICES : 1; }
 // kernels launch_rebuild enqueues
-inline int rebuild_kernels(const Box &b, const LaunchCfg &lc) { return 8 + (scan_slices(b) > 1 ? 1 : 0) + (lc.exchange ? 2 : 0); }
+inline int rebuild_kernels(const Box &b, const LaunchCfg &lc) { return 6 + (scan_slices(b) > 1 ? 1 : 0) + (lc.exchange ? 2 : 0); }
 // kernels one force evaluation launches
 inline int force_kernels(const LaunchCfg &lc) { return lc.exchange ? 2 : 1; }
 // kick: 0 = force only, 1 = VV closing kick, 2 = Langevin closing update.
