@@ -31,6 +31,7 @@ constexpr int MAX_GRAPH_STEPS = 1000;  // steps captured per graph, and thermo r
 struct ChunkPlan {
   int S = 0, ev = 0;          // steps; record period (thermo at step k iff ev > 0 and (k + 1) % ev == 0)
   std::vector<uint8_t> fuse;  // [S]
+  int dropped = -1;           // the step kept from drifting the next to make their number even
   bool thermo(int k) const { return ev > 0 && (k + 1) % ev == 0; }
   int fused_before(int k) const {
     int n = 0;
@@ -81,7 +82,7 @@ struct cavgpu_ctx {
   long long graph_launches = 0, kernel_launches = 0;
   int max_nb = 0;
   std::deque<GraphEntry> graphs;                      // stable references (chunks in flight hold them)
-  std::map<std::pair<int, int>, ChunkPlan> eager_plans;  // chunks launched from the host
+  std::map<std::pair<int, int>, ChunkPlan> eager_plans;  // chunks that are not graphs
   // status words of the last chunks, read back without a full synchronisation
   int *h_status = nullptr;   // pinned, 2 x F_NWORDS
   cudaEvent_t ev_status[2] = {nullptr, nullptr};
@@ -198,8 +199,25 @@ ChunkPlan make_plan(const cavgpu_ctx *c, int S, int ev) {
     ++nf;
     last = k;
   }
-  if (nf & 1) pl.fuse[last] = 0;  // an even number: the buffers end where they began
+  if (nf & 1) {  // an even number: the buffers end where they began
+    pl.fuse[last] = 0;
+    pl.dropped = last;
+  }
   return pl;
+}
+
+// the plan of a chunk that is not a graph, kept for the context's life (chunks in flight
+// refer to it)
+const ChunkPlan *plan_of(cavgpu_ctx *c, int S, int ev) {
+  auto it = c->eager_plans.find({S, ev});
+  if (it == c->eager_plans.end()) it = c->eager_plans.emplace(std::make_pair(S, ev), make_plan(c, S, ev)).first;
+  return &it->second;
+}
+
+// the fold of a recorded step by the pair kernel's last block (or the step kernel)
+FoldArgs fold_args(const cavgpu_ctx *c, int ring_slot) {
+  return FoldArgs{c->tc, is_lang(c) ? drift_grid_blocks(c->lc) : force_grid_blocks(c->lc), ev_grid_blocks(c->lc),
+                  is_lang(c) ? force_grid_blocks(c->lc) : 0, ring_slot};
 }
 
 // The steps of a chunk, captured into the graph being recorded on c->st (capture)
@@ -272,8 +290,7 @@ int enqueue_chunk(cavgpu_ctx *c, const ChunkPlan &pl, bool capture, long long *l
       CK(capture ? cudaEventRecordWithFlags(c->ev0[k], c->st, cudaEventRecordExternal) : cudaEventRecord(c->ev0[k], c->st));
     // a recorded step of a single system: the pair kernel's last block folds the record
     const bool fold = th && c->b.nrep == 1 && c->nve.step == 0;
-    FoldArgs fa{c->tc, is_lang(c) ? drift_grid_blocks(c->lc) : force_grid_blocks(c->lc), ev_grid_blocks(c->lc),
-                is_lang(c) ? force_grid_blocks(c->lc) : 0, ring_slot};
+    const FoldArgs fa = fold_args(c, ring_slot);
     RK(launch_force(view, c->b, c->sc, c->lc, is_lang(c) ? 2 : 1, th, k, fuse, set_cond, hnext, c->st,
                     fold ? &fa : nullptr));
     if (c->prof && k < (int)c->ev1.size())
@@ -371,9 +388,11 @@ int alloc_exchange(cavgpu_ctx *c) {
   const size_t recv = n * cap_h * sizeof(dbl4), words = n * cap_h * sizeof(uint32_t), slots = n * cap_h * sizeof(uint16_t);
   const size_t evp = c->b.nrep > 1 ? n * d.tpa * sizeof(double2) : 0;
   const size_t bytes = recv + 4 * n * sizeof(dbl4) + evp + words + slots + n * sizeof(int4) + 2 * n * sizeof(int);
-  size_t free_mem = 0, total_mem = 0;
-  CK(cudaMemGetInfo(&free_mem, &total_mem));
-  if (bytes > total_mem / 4) return CAVGPU_OK;
+  if (bytes > ((size_t)1 << 30)) {  // (the query takes longer than allocating for a small system)
+    size_t free_mem = 0, total_mem = 0;
+    CK(cudaMemGetInfo(&free_mem, &total_mem));
+    if (bytes > total_mem / 4) return CAVGPU_OK;
+  }
   void *q = nullptr;
   if (cudaMalloc(&q, bytes) != cudaSuccess) { cudaGetLastError(); return CAVGPU_OK; }
   c->x_mem = q;
@@ -591,6 +610,10 @@ int create_common(const cavgpu_params *p, int nrep, const double *lo3, const dou
   }
   int rc = dalloc(c, &c->d.tab, 1);
   if (!rc) rc = dalloc(c, &c->d.flags, F_NWORDS);
+  c->d.req = c->d.flags + F_REBUILD;
+  c->d.nan = c->d.flags + F_NAN;
+  if (!rc) rc = dalloc(c, &c->d.barrier, 1);
+  if (!rc) rc = cuda_rc(cudaMemsetAsync(c->d.barrier, 0, sizeof(unsigned int), c->st));
   if (!rc) rc = dalloc(c, &c->d.thermo, 8);
   if (!rc) rc = dalloc(c, &c->d.step_base, 1);
   if (!rc) rc = dalloc(c, &c->d.thermo_ring, THERMO_REC * (size_t)MAX_GRAPH_STEPS);
@@ -787,9 +810,10 @@ int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, cons
     take(&d.cell_count, ncell_all);
     take(&d.cell_cursor, ncell_all);
     take(&d.cell_start, (size_t)ncell_all + 1);
-    take(&d.partials_ke, 4 * std::max(nblk, nblk_d));
-    take(&d.partials_ke_end, 4 * nblk);
-    take(&d.partials_ev, 2 * nblk);
+    d.partials_alt = (int)std::max(nblk, nblk_d);  // two sets: the step kernel alternates between them
+    take(&d.partials_ke, 8 * (size_t)d.partials_alt);
+    take(&d.partials_ke_end, 8 * (size_t)d.partials_alt);
+    take(&d.partials_ev, 4 * (size_t)d.partials_alt);
     take(&d.h3, 3 * (size_t)N);
     take(&d.hi3, 3 * (size_t)N);
     if (c->p.msd_process) {  // Atom_data::msd_process: boundary crossings per atom
@@ -956,6 +980,9 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
   int S = c->p.steps_per_graph > 0 ? std::min(c->p.steps_per_graph, MAX_GRAPH_STEPS) : 50;
   if (every > 0) S = (int)std::max<int64_t>(every, (S / every) * every);
   const bool eager = c->p.steps_per_graph < 0;
+  // small systems: a chunk's steps in one launch (cav_chunk.cu); not while kernel times are
+  // taken, nor with constraint::Nve between the steps
+  const bool small = !eager && !c->prof && c->nve.step == 0 && chunk_fits(c->b, c->lc);
   RK(ensure_status(c));
   int f[F_NWORDS];
   RK(read_flags(c, f));
@@ -974,7 +1001,10 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
     while (launched < nsteps && q.size() < depth) {
       const int64_t left = nsteps - launched;
       int sz = (int)std::min<int64_t>(left, S), ev;
-      if (every == 0) ev = (left == sz) ? sz : 0;
+      if (every == 0 && small && c->b.nrep > 1 && left > 1) {
+        sz = (int)std::min<int64_t>(left - 1, S);  // the replicas' thermo, folded by a kernel of its own,
+        ev = 0;                                    // ends the call with a one-step graph
+      } else if (every == 0) ev = (left == sz) ? sz : 0;
       else if (launched % every != 0) {  // resuming after a completed overflow step: up to the next record
         sz = (int)std::min<int64_t>(left, every - launched % every);
         ev = (launched + sz) % every == 0 ? sz : 0;
@@ -984,7 +1014,12 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
         ev = ((launched + 1) % every == 0) ? 1 : 0;
       }
       const ChunkPlan *plan;
-      if (!eager) {
+      if (small && (ev == 0 || c->b.nrep == 1)) {
+        plan = plan_of(c, sz, ev);
+        const FoldArgs fa = fold_args(c, 0);
+        RK(launch_chunk(c->d, c->b, c->sc, c->lc, sz, ev, fuse_mode(c), plan->dropped, fa, c->st));
+        c->kernel_launches += 1;
+      } else if (!eager) {
         int rc = CAVGPU_OK;
         GraphEntry *g = get_graph(c, sz, ev, &rc);
         if (!g) return rc;
@@ -993,9 +1028,7 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
         c->kernel_launches += g->launches;
         plan = &g->plan;
       } else {
-        auto it = c->eager_plans.find({sz, ev});
-        if (it == c->eager_plans.end()) it = c->eager_plans.emplace(std::make_pair(sz, ev), make_plan(c, sz, ev)).first;
-        plan = &it->second;
+        plan = plan_of(c, sz, ev);
         if (c->prof) RK(ensure_events(c, sz));
         long long nl = 0;
         RK(enqueue_chunk(c, *plan, false, &nl));
@@ -1017,6 +1050,7 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
     CK(cudaEventSynchronize(c->ev_status[p.slot]));
     const int *hf = c->h_status + p.slot * F_NWORDS;
     c->max_nb = std::max(c->max_nb, hf[F_MAXNB]);
+    if (hf[F_STALL]) return CAVGPU_E_CUDA;  // a grid barrier of the step kernel gave up
     if (c->prof) RK(collect_profile(c, p.sz));
     if (!hf[F_HALT]) {
       done = p.start + p.sz;
@@ -1041,7 +1075,7 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
   }
   RK(check_status(c));
   // rebuild kernels launched by the graphs' conditional nodes
-  if (!eager) {
+  if (!eager && !small) {
     RK(read_flags(c, f));
     if (f[F_PASSES] > passes0) c->kernel_launches += (long long)rebuild_kernels(c->b, c->lc) * (f[F_PASSES] - passes0);
   }

@@ -38,10 +38,26 @@ __host__ __device__ inline double type_bits(int t) {
 }
 __device__ inline int type_of(const double w) { return (int)__double_as_longlong(w); }
 
+// Loads of what other blocks wrote.  A kernel that only reads it takes the read-only path;
+// COH: the step kernel (cav_chunk.cu), in which the data changes between its barriers, loads
+// coherently and in program order.
+template <bool COH, class T>
+__device__ __forceinline__ T ld_ro(const T *p) {
+  if constexpr (COH) return *p;
+  else return __ldg(p);
+}
 // read-only (non-coherent) 256-bit load of a neighbour's position
 __device__ inline dbl4 ldg_dbl4(const dbl4 *p) {
   dbl4 r;
   asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  return r;
+}
+
+template <bool COH>
+__device__ __forceinline__ dbl4 ld_dbl4(const dbl4 *p) {
+  if constexpr (!COH) return ldg_dbl4(p);
+  dbl4 r;
+  asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p) : "memory");
   return r;
 }
 
@@ -71,7 +87,10 @@ enum Flag : int {
   F_STEPS_OK = 8,   // steps of the current chunk whose pair kernel ran (the step counter adds them)
   F_HALT_STEP = 9,  // steps of the halted chunk that completed before the halt
   F_UPLOAD_BAD = 10,  // an uploaded atom outside the box, of an unknown type or with a bad id
-  F_NWORDS = 12
+  // the step kernel of small systems (cav_chunk.cu): rebuild requests and NaNs by phase,
+  // the phase, a barrier that gave up
+  F_PHASE_REQ = 12, F_PHASE_NAN = 15, F_PHASE = 18, F_STALL = 19,
+  F_NWORDS = 20
 };
 
 // what the pair kernel does after the closing update of its step: nothing, or the
@@ -178,6 +197,9 @@ struct Dev {
   int cap_h;
   // status, reductions
   int *flags;
+  int *req, *nan;             // where a drift asks for a rebuild and reports a NaN (F_REBUILD, F_NAN of flags)
+  unsigned int *barrier;      // grid barrier of the step kernel
+  int partials_alt;           // blocks after which the partial arrays' second halves begin (step kernel)
   double *partials_ke;        // per-block {sum m v^2, sum m v} (4 per block)
   double *partials_ke_end;    // Langevin: the same sums over the velocities at the end of the step
   double *partials_ev;        // per-block {sum -coef r^2, sum V} over both pair orders (2 per block)
@@ -343,9 +365,14 @@ __device__ __forceinline__ void lang_move(dbl4 &x, const dbl4 &v, const StepCons
   }
 }
 
+// m v^2, in one order of roundings wherever it is compiled
+__device__ __forceinline__ double twice_ke(double m, const dbl4 &v) {
+  return __dmul_rn(m, fma(v.z, v.z, fma(v.y, v.y, __dmul_rn(v.x, v.x))));
+}
+
 __device__ inline void request_rebuild(const Dev &d, const Box &b, int rep) {
   b.rep_flag[rep] = 1;
-  d.flags[F_REBUILD] = 1;
+  *d.req = 1;
 }
 
 // Fixed-point coordinates.  Along an axis the box is cut into m
@@ -415,7 +442,7 @@ __device__ inline void nan_check(const Dev &d, int i, const dbl4 &a) {
   // on the bit patterns: comparing doubles would take the FP64 pipe
   auto nan = [](double v) { return (unsigned long long)(__double_as_longlong(v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ull; };
   if (nan(a.x) || nan(a.y) || nan(a.z)) {
-    d.flags[F_NAN] = 1;
+    *d.nan = 1;
     d.flags[F_NAN_ATOM] = (int)d.id[i];
   }
 }
@@ -459,6 +486,16 @@ __device__ inline void thermo_finish(double ke2, const double P3[3], double msum
   out[4] = 0.5 * pe2;
 }
 
+// The thermo fold of a recorded step done by the pair kernel's last block (single
+// systems): the fixed-order sums of the KE partials (nb_ke blocks; Langevin: the
+// drift kernel's) and of the launch's own virial/PE partials (nb_ev; and, Langevin, of its
+// end-of-step KE partials, nb_ke_end), then the record -- what launch_thermo_final
+// does after the launch, without its launch.
+struct FoldArgs {
+  ThermoCfg tc;
+  int nb_ke, nb_ev, nb_ke_end, ring_slot;
+};
+
 // Kernel launchers (cav_kernels.cu, cav_force.cu).  `forced` rebuilds every
 // replica regardless of the flags; otherwise the rebuild kernels skip replicas
 // whose half-skin test did not fire.
@@ -490,15 +527,6 @@ inline int force_kernels(const LaunchCfg &lc) { return lc.exchange ? 2 : 1; }
 // cond: when set_cond, the last block sets the conditional node of the next step's
 // rebuild to the half-skin flag (unless halted).  The last block also counts the
 // step (F_STEPS_OK) and raises the halt on a NaN.
-// The thermo fold of a recorded step done by the pair kernel's last block (single
-// systems): the fixed-order sums of the KE partials (nb_ke blocks; Langevin: the
-// drift kernel's) and of the launch's own virial/PE partials (nb_ev; and, Langevin, of its
-// end-of-step KE partials, nb_ke_end), then the record -- what launch_thermo_final
-// does after the launch, without its launch.
-struct FoldArgs {
-  ThermoCfg tc;
-  int nb_ke, nb_ev, nb_ke_end, ring_slot;
-};
 // the pair exchange: its part of a list build, its two kernels, their block size
 struct ForceArgs;
 int launch_exchange_build(const Dev &d, const Box &b, int forced, cudaStream_t st);
@@ -518,6 +546,12 @@ int launch_thermo_final(const Dev &d, const ThermoCfg &tc, int nb_ke, int nb_ev,
 // batches: per-replica KE (ke = 1, from the current velocities) and/or virial+PE folds
 int launch_thermo_replicas(const Dev &d, const Box &b, const ThermoCfg &tc, int ke, int ev, cudaStream_t st);
 int launch_advance_step(const Dev &d, cudaStream_t st);
+// Small systems: S steps in one cooperative launch (cav_chunk.cu).  fuse: Fuse of the steps
+// that drift the next one (rule of ChunkPlan; `drop` = the step kept from it, -1: none),
+// ev: record period; fa: the fold of a recorded step.
+bool chunk_fits(const Box &b, const LaunchCfg &lc);
+int launch_chunk(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int S, int ev, int fuse, int drop,
+                 const FoldArgs &fa, cudaStream_t st);
 // constraint::Nve: kinetic energy, lambda (and the thermo point of the step,
 // ring_slot >= 0 or the current one when thermo != 0), velocity scaling; every
 // kernel returns at once unless (step_base + k) % cfg.step == 0

@@ -4,6 +4,7 @@
 // (see cav_common.cuh); a single system is R = 1.
 #include <algorithm>
 
+#include "cav_drift.cuh"
 #include "cav_rebuild.cuh"
 
 namespace cav {
@@ -49,85 +50,24 @@ __device__ inline void block_sum_store(double (&v)[NV], double *out /* NV double
 // integrator stage 1 -- src/md_simulator.cpp:640-656 (velocity Verlet) and
 // :748-837 (Langevin first half); NaN check; half-skin test per replica
 // ---------------------------------------------------------------------------
-// Velocity-Verlet drift (src/md_simulator.cpp:640-656) with the NaN check of the
-// acceleration and the half-skin test; the pair kernel fuses the same update into
-// the step before when it can (FUSE_VV), so this kernel runs at the start of a chunk.
 template <bool MIXED>
 __global__ void __launch_bounds__(256) k_drift_vv(Dev d, Box b, StepConsts sc) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= sc.n || halted(d)) return;
-  const int rep = rep_of_slot(b, i);
-  if (rep < 0) return;  // padding slot
-  dbl4 x = d.pos[i];
-  const dbl4 v = d.vel[i], a = d.acc[i];
-  nan_check(d, i, a);
-  drift_vv<MIXED>(x, v, a, sc);
-  d.pos[i] = x;  // acc stays: the pair kernel's kick reads it as a_old
-  if (MIXED) mixed_track(d, b, rep, i, x, d.ic);
-  else half_skin_test(d, b, rep, i, x);
+  if (i < sc.n && !halted(d)) drift_slot_vv<MIXED>(d, b, sc, i);
 }
 
-// Leap-frog first half (src/md_simulator.cpp:890-905): v += (0.5 dt) a ; r += dt v.
-// The closing half, v += (0.5 dt) a(t + dt), is the velocity-Verlet kick of the pair
-// kernel with a_old = 0: v + (a + 0)(0.5 dt) rounds exactly as v + (0.5 dt) a.
 template <bool MIXED>
 __global__ void __launch_bounds__(256) k_drift_lf(Dev d, Box b, StepConsts sc) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= sc.n || halted(d)) return;
-  const int rep = rep_of_slot(b, i);
-  if (rep < 0) return;  // padding slot
-  dbl4 x = d.pos[i], v = d.vel[i];
-  const dbl4 a = d.acc[i];
-  nan_check(d, i, a);
-  drift_lf<MIXED>(x, v, a, sc);
-  d.pos[i] = x;
-  d.vel[i] = v;
-  d.acc[i] = make_dbl4(0.0, 0.0, 0.0, 0.0);  // a_old = 0 for the kick
-  if (MIXED) mixed_track(d, b, rep, i, x, d.ic);
-  else half_skin_test(d, b, rep, i, x);
+  if (i < sc.n && !halted(d)) drift_slot_lf<MIXED>(d, b, sc, i);
 }
 
-// Langevin position update r += v*c (src/md_simulator.cpp:822-827) with the
-// half-skin tracking; with THERMO the temperature sums of the velocities first.
-template <bool MIXED, bool THERMO>
-__device__ __forceinline__ void lang_position(const Dev &d, const Box &b, const StepConsts &sc, int rep, int i, dbl4 x,
-                                              const dbl4 &v, double (&part)[4]) {
-  if (THERMO) {
-    const double m = d.tab->mass[type_of(x.w)];
-    part[0] = m * (v.x * v.x + v.y * v.y + v.z * v.z);
-    part[1] = m * v.x; part[2] = m * v.y; part[3] = m * v.z;
-  }
-  lang_move<MIXED>(x, v, sc);
-  d.pos[i] = x;
-  if (MIXED) mixed_track(d, b, rep, i, x, d.ic);
-  else half_skin_test(d, b, rep, i, x);
-}
-
-// Langevin first half (src/md_simulator.cpp:748-837):
-//   v += (a*0.5)*dt + eta*b ; [temperature here] ; r += v*c
-// POS false: the velocity half only; constraint::Nve then acts on the mid-step
-// velocities (:784-791) and k_lang_pos takes the temperature and moves the atoms.
 template <bool MIXED, bool THERMO, bool POS>
 __global__ void __launch_bounds__(256) k_lang_a(Dev d, Box b, StepConsts sc, int k_in_chunk) {
   if (halted(d)) return;  // the same value for every block: no block reaches the reduction alone
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double part[4] = {0.0, 0.0, 0.0, 0.0};
-  const int rep = i < sc.n ? rep_of_slot(b, i) : -1;
-  if (rep >= 0) {
-    dbl4 x = d.pos[i], v = d.vel[i];
-    const dbl4 a = d.acc[i];
-    nan_check(d, i, a);
-    double e0 = 0.0, e1 = 0.0, e2 = 0.0;
-    if (!sc.noise_off) {
-      const long long step = *d.step_base + k_in_chunk;
-      // replica r draws the noise stream of seed + r with its local ids
-      if (MIXED) langevin_eta_f(sc.seed + rep, step, d.id[i], e0, e1, e2);
-      else langevin_eta(sc.seed + rep, step, d.id[i], e0, e1, e2);
-    }
-    lang_half<MIXED>(v, a, e0, e1, e2, sc);
-    d.vel[i] = v;
-    if (POS) lang_position<MIXED, THERMO>(d, b, sc, rep, i, x, v, part);
-  }
+  if (i < sc.n) lang_slot<MIXED, THERMO, POS>(d, b, sc, *d.step_base + k_in_chunk, i, part);
   if (POS && THERMO) block_sum_store<4>(part, &d.partials_ke[(size_t)blockIdx.x * 4]);
 }
 
@@ -256,8 +196,16 @@ __global__ void __launch_bounds__(256) k_sort_gather(Dev d, Box b, int forced) {
 template <int MODE>
 __global__ void __launch_bounds__(BUILD_WARPS * 32, 4) k_build_group(Dev d, Box b, int forced) {
   __shared__ BuildStage stage[BUILD_WARPS];
-  rebuild_build<MODE>(d, b, forced, stage[threadIdx.x >> 5], (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                      (gridDim.x * blockDim.x) >> 5);
+  rebuild_build<MODE, false>(d, b, forced, stage[threadIdx.x >> 5], (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                             (gridDim.x * blockDim.x) >> 5, nullptr);
+}
+
+// few windows: a block of four warps each (BuildShare)
+constexpr int SHARED_WINDOWS = 8;  // per SM
+template <int MODE>
+__global__ void __launch_bounds__(128) k_build_shared(Dev d, Box b, int forced) {
+  __shared__ BuildShare share;
+  rebuild_build<MODE, true>(d, b, forced, share.stage[threadIdx.x >> 5], blockIdx.x, gridDim.x, &share);
 }
 
 // after the build: count the rebuilt replicas, clear their flags and the global one;
@@ -381,7 +329,7 @@ __global__ void __launch_bounds__(256) k_thermo_rep(Dev d, Box b, ThermoCfg tc, 
     if (ke) {
       const dbl4 vv = d.vel[i];
       const double m = d.tab->mass[d.type[i]];
-      v[0] += m * (vv.x * vv.x + vv.y * vv.y + vv.z * vv.z);
+      v[0] += twice_ke(m, vv);
       v[1] += m * vv.x; v[2] += m * vv.y; v[3] += m * vv.z;
       v[4] += m;
     }
@@ -437,7 +385,7 @@ __global__ void __launch_bounds__(256) k_nve_ke(Dev d, int n, NveCfg c, int k) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const dbl4 v = d.vel[i];
     const double m = d.tab->mass[d.type[i]];
-    part[0] += m * (v.x * v.x + v.y * v.y + v.z * v.z);
+    part[0] += twice_ke(m, v);
     part[1] += m * v.x; part[2] += m * v.y; part[3] += m * v.z;
   }
   block_sum_store<4>(part, &d.nve_partials[(size_t)blockIdx.x * 4]);
@@ -738,8 +686,13 @@ int launch_rebuild(const Dev &d, const Box &b, const LaunchCfg &lc, int forced, 
   k_scan_rep<<<b.nrep * P, 1024, 0, st>>>(d, b, forced, P);
   k_scatter<<<g, 256, 0, st>>>(d, b, forced);
   k_sort_gather<<<ceil_div((long long)b.ncell_all * 32, 256), 256, 0, st>>>(d, b, forced);
-  const int build_grid = std::min(ceil_div(ceil_div(b.nslot, 32), BUILD_WARPS), num_sms() * 8);
-  if (lc.precision == CAVGPU_MIXED) k_build_group<1><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
+  const int windows = ceil_div(b.nslot, 32), build_grid = std::min(ceil_div(windows, BUILD_WARPS), num_sms() * 8);
+  // up to SHARED_WINDOWS windows per SM (38,912 atoms) a window's own chain of work is the
+  // time: 33 us with its four warps, 46 us with one, at 32,000 atoms
+  if (windows <= num_sms() * SHARED_WINDOWS) {
+    if (lc.precision == CAVGPU_MIXED) k_build_shared<1><<<windows, 128, 0, st>>>(d, b, forced);
+    else k_build_shared<0><<<windows, 128, 0, st>>>(d, b, forced);
+  } else if (lc.precision == CAVGPU_MIXED) k_build_group<1><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
   else k_build_group<0><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
   if (lc.exchange) {
     const int rc = launch_exchange_build(d, b, forced, st);

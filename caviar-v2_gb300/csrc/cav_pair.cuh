@@ -76,6 +76,17 @@ __device__ inline void load_tab(const Dev &d, Tab &tab) {
   for (int k = threadIdx.x; k < nt; k += blockDim.x) { tab.minv[k] = T.minv[k]; tab.mass[k] = T.mass[k]; }
 }
 
+// masses alone, for the closing update (finish_atom)
+struct MassTab {
+  double minv[MAXT], mass[MAXT];
+  __device__ __forceinline__ void load(const Dev &d) {
+    if (threadIdx.x < MAXT) {
+      minv[threadIdx.x] = d.tab->minv[threadIdx.x];
+      mass[threadIdx.x] = d.tab->mass[threadIdx.x];
+    }
+  }
+};
+
 // How an atom's row is split over lanes in the FP64 form.  Entry e of the row adds to
 // partial sum e mod 4, in row order; a lane holds all four sums (TPA 1), two of them (TPA
 // 2) or one (TPA >= 4: t mod 4, of the chunks t / 4, t / 4 + TPA / 4, ...).  Sums 0 and 1, 2
@@ -130,7 +141,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     if (EV) {
       v = d.vel[i];
       const double m = tab.mass[ti];
-      ke_p[0] += m * (v.x * v.x + v.y * v.y + v.z * v.z);
+      ke_p[0] += twice_ke(m, v);
       ke_p[1] += m * v.x; ke_p[2] += m * v.y; ke_p[3] += m * v.z;
     }
   } else if (KICK == 1) {
@@ -147,7 +158,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
     if (EV) {
       const double m = tab.mass[ti];
-      ke_p[0] += m * (v.x * v.x + v.y * v.y + v.z * v.z);
+      ke_p[0] += twice_ke(m, v);
       ke_p[1] += m * v.x; ke_p[2] += m * v.y; ke_p[3] += m * v.z;
     }
   } else {
@@ -168,7 +179,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
     if (EV) {  // Atom_data::kinetic_energy() read after the step (the temperature was taken mid-step)
       const double m = tab.mass[ti];
-      ke_p[0] += m * (v.x * v.x + v.y * v.y + v.z * v.z);
+      ke_p[0] += twice_ke(m, v);
       ke_p[1] += m * v.x; ke_p[2] += m * v.y; ke_p[3] += m * v.z;
     }
   }

@@ -164,7 +164,7 @@ __device__ __forceinline__ void rebuild_sort_gather(const Dev &d, const Box &b, 
 // coordinates: only candidates inside a narrow band around the cutoff take
 // the FP64 path.  mode 0 stores image codes (FP64 force), mode 1 cell-offset
 // codes (mixed force).
-__device__ __noinline__ bool exact_pair(const Dev &d, const RepBox &rb, double ce2, int i, int j, int img) {
+static __device__ __noinline__ bool exact_pair(const Dev &d, const RepBox &rb, double ce2, int i, int j, int img) {
   const dbl4 xi = d.pos[i], xj = d.pos[j];
   const double shx = (img % 3 - 1) * rb.L[0], shy = ((img / 3) % 3 - 1) * rb.L[1], shz = (img / 9 - 1) * rb.L[2];
   const double ddx = __dsub_rn(__dadd_rn(xj.x, shx), xi.x);
@@ -219,6 +219,7 @@ __device__ __forceinline__ int class_cell(int x0, int nu, int k) {
 // mask per lane (one warp vote per 32 candidates for the rare exact FP64 test), and
 // only then are the hits (~15% of the staged candidates) written, in candidate order.
 constexpr int BUILD_STAGE = 256;  // staged candidates per warp and pass (4 KiB + 256 B)
+constexpr int SEG_HITS = 40;      // hits per lane that a part of a shared window holds
 constexpr int GROUP_SPAN = 5;     // a group spans at most 6 cells: x index + 8 row < 256
 
 // q_u, q_u+1 = |c - r|^2 of two candidates with packed FP32x2 arithmetic (sm_100+):
@@ -261,7 +262,7 @@ struct BuildLane {
 template <int MODE>
 __device__ __forceinline__ void build_sweep(const Dev &d, const Box &b, const RepBox &rb, int nst,
                                             const float4 *sxy, const float2 *sz, const uint32_t *sw,
-                                            const uint8_t *su, BuildLane &L, int cshift, bool by_mol) {
+                                            const uint8_t *su, BuildLane &L, int cshift, bool by_mol, uint32_t *seg) {
   const int lane = threadIdx.x & 31;
   float *pxy = const_cast<float *>(reinterpret_cast<const float *>(sxy));
   float *pz = const_cast<float *>(reinterpret_cast<const float *>(sz));
@@ -323,7 +324,11 @@ __device__ __forceinline__ void build_sweep(const Dev &d, const Box &b, const Re
       uint32_t w = swc[u];
       if (by_mol && d.mol[w & IDX_MASK] == L.mol) continue;
       if (MODE != 0) w -= ci_code;  // stencil index of j's cell relative to the atom's
-      if (L.cnt < cap) L.row[((L.cnt >> 2) << cshift) + (L.cnt & 3)] = w;
+      if (seg) {  // a part of the group's candidates: hits by number and lane
+        if (L.cnt < SEG_HITS) seg[L.cnt * 32 + lane] = w;
+      } else if (L.cnt < cap) {
+        L.row[((L.cnt >> 2) << cshift) + (L.cnt & 3)] = w;
+      }
       ++L.cnt;
     }
   }
@@ -351,9 +356,25 @@ struct BuildStage {
   int self[32];
 };
 
-// warp gw of nw: the windows gw, gw + nw, ...
-template <int MODE>
-__device__ __forceinline__ void rebuild_build(const Dev &d, const Box &b, int forced, BuildStage &stage, int gw, int nw) {
+// The four warps of a block share a window (small systems: a window takes one warp some
+// 38 us from end to end, whatever the rest of the GPU does): each takes a part of the
+// candidates' rows, about balanced by the candidates that survive the culling; the first
+// writes its hits straight to the list rows, the others keep theirs in shared memory and
+// move them behind those of the parts before.  An atom with more hits in a part than fit
+// there sends the window to one warp.
+struct BuildShare {
+  BuildStage stage[4];
+  uint32_t hits[3][SEG_HITS * 32];
+  int cnt[4][32];
+};
+__constant__ const int8_t PART_ROWS[5] = {0, 2, 5, 7, 9};  // of ROW_ORDER
+
+// SHARED false: warp gw of nw takes the windows gw, gw + nw, ...; true: block gw of nw, the
+// warps of a block (four) the parts of its windows.
+template <int MODE, bool SHARED>
+__device__ __forceinline__ void rebuild_build(const Dev &d, const Box &b, int forced, BuildStage &stage, int gw, int nw,
+                                              BuildShare *share) {
+  const int part = SHARED ? threadIdx.x >> 5 : 0;
   const int lane = threadIdx.x & 31;
   float4 *sxy = stage.xy;
   float2 *sz = stage.z;
@@ -412,11 +433,15 @@ __device__ __forceinline__ void rebuild_build(const Dev &d, const Box &b, int fo
       L.hi = L.me ? b.ce2_hi : -1.0f;
       L.cnt = 0;
       // candidate cells, nu in each of the 9 rows r = (dy+1) + 3 (dz+1): x cell cx0 - 1 + u
-      const int nu = span + 3, ncand = 9 * nu;
+      const int nu = span + 3;
+      int q_first = SHARED ? PART_ROWS[part] * nu : 0, ncand = SHARED ? PART_ROWS[part + 1] * nu : 9 * nu;
+      uint32_t *seg = SHARED && part > 0 ? share->hits[part - 1] : nullptr;
+      bool parts = SHARED;
+     again:
       int nst = 0;
       selfpos[lane] = -1;
       __syncwarp();
-      for (int q0 = 0; q0 < ncand; q0 += 32) {
+      for (int q0 = q_first; q0 < ncand; q0 += 32) {
         // lane q - q0: the candidate cell's first slot, count, image code, origin offset
         int kb = 0, kn = 0, ks = 0, kimg = 0;
         uint32_t kcode = 0u;
@@ -481,7 +506,7 @@ __device__ __forceinline__ void rebuild_build(const Dev &d, const Box &b, int fo
             nst += __popc(km);
             if (nst > BUILD_STAGE - 32) {
               __syncwarp();
-              build_sweep<MODE>(d, b, rb, nst, sxy, sz, sw, su, L, cshift, by_mol);
+              build_sweep<MODE>(d, b, rb, nst, sxy, sz, sw, su, L, cshift, by_mol, seg);
               selfpos[lane] = -1;
               __syncwarp();
               nst = 0;
@@ -491,9 +516,36 @@ __device__ __forceinline__ void rebuild_build(const Dev &d, const Box &b, int fo
       }
       if (nst > 0) {
         __syncwarp();
-        build_sweep<MODE>(d, b, rb, nst, sxy, sz, sw, su, L, cshift, by_mol);
+        build_sweep<MODE>(d, b, rb, nst, sxy, sz, sw, su, L, cshift, by_mol, seg);
       }
-      if (L.me) {
+      if (parts) {
+        share->cnt[part][lane] = L.cnt;
+        __syncthreads();
+        int before = 0, total = 0;
+        bool fits = true;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          const int n = share->cnt[p][lane];
+          if (p < part) before += n;
+          total += n;
+          fits = fits && (p == 0 || n <= SEG_HITS);
+        }
+        if (__syncthreads_and(fits)) {
+          if (L.me && part > 0)
+            for (int k = 0; k < L.cnt; ++k)
+              if (before + k < d.cap) L.row[(((before + k) >> 2) << cshift) + ((before + k) & 3)] = seg[k * 32 + lane];
+          L.cnt = total;
+        } else {  // warp 0 takes all candidates, straight to the rows
+          parts = false;
+          seg = nullptr;
+          q_first = 0;
+          ncand = part == 0 ? 9 * nu : 0;
+          L.cnt = 0;
+          goto again;
+        }
+      }
+      if (SHARED) __syncthreads();  // the counts are overwritten next
+      if (L.me && part == 0) {
         d.nnbr[L.i] = min(L.cnt, d.cap);
         if (L.cnt > d.cap) atomicMax(&d.flags[F_OVERFLOW], L.cnt);
         wmax = max(wmax, L.cnt);
