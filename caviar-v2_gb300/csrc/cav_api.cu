@@ -799,11 +799,12 @@ int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, cons
     };
     for (dbl4 **pp : {&d.pos, &d.vel, &d.acc, &d.pos_ref, &d.t_pos, &d.t_vel, &d.t_acc}) take(pp, NS);
     take(&d.rel, NS);
+    take(&d.t_rel, NS);
     // the coordinates a pair kernel gathers and the second buffer of them (it drifts into it)
     if (c->p.precision == CAVGPU_MIXED)
       for (int4 **pp : {&d.ic, &d.ic_ref, &d.ic_alt}) take(pp, NS);
     else take(&d.pos_alt, NS);
-    for (int **pp : {&d.type, &d.cell_of, &d.t_type, &d.atom_cell, &d.perm, &d.perm_tmp, &d.nnbr}) take(pp, NS);
+    for (int **pp : {&d.type, &d.cell_of, &d.atom_cell, &d.perm, &d.perm_tmp, &d.nnbr}) take(pp, NS);
     take(&d.id, NS);
     take(&d.t_id, NS);
     take(&d.skey, NS);

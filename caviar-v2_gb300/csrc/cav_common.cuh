@@ -176,7 +176,7 @@ struct Dev {
   int *mol;                   // molecule index (ignore_intra_molecule); null when off
   // rebuild scratch
   dbl4 *t_pos, *t_vel, *t_acc;
-  int *t_type;
+  float4 *t_rel;
   uint32_t *t_id;
   int4 *t_img;
   int *t_mol;

@@ -686,8 +686,9 @@ int launch_rebuild(const Dev &d, const Box &b, const LaunchCfg &lc, int forced, 
   k_scan_rep<<<b.nrep * P, 1024, 0, st>>>(d, b, forced, P);
   k_scatter<<<g, 256, 0, st>>>(d, b, forced);
   k_sort_gather<<<ceil_div((long long)b.ncell_all * 32, 256), 256, 0, st>>>(d, b, forced);
-  const int windows = ceil_div(b.nslot, 32), build_grid = std::min(ceil_div(windows, BUILD_WARPS), num_sms() * 8);
-  // up to SHARED_WINDOWS windows per SM (38,912 atoms) a window's own chain of work is the
+  const int windows = ceil_div(b.nslot, 32), build_grid = std::min(ceil_div(windows, BUILD_WARPS), num_sms() * 32);
+  // one window per warp up to 1.2 M slots: with 8 blocks per SM a warp had 3 or 4 of them at
+  // 1,048,576 atoms and the build 30 us of tail; up to SHARED_WINDOWS windows per SM (38,912 atoms) a window's own chain of work is the
   // time: 33 us with its four warps, 46 us with one, at 32,000 atoms
   if (windows <= num_sms() * SHARED_WINDOWS) {
     if (lc.precision == CAVGPU_MIXED) k_build_shared<1><<<windows, 128, 0, st>>>(d, b, forced);

@@ -11,17 +11,6 @@ namespace cav {
 #define FULL_MASK 0xffffffffu
 #endif
 
-__device__ inline void update_rel(const Dev &d, const RepBox &rb, int i, const dbl4 &x) {
-  const int c = d.cell_of[i] - rb.cell_off;
-  const int cx = c % rb.nc[0], cy = (c / rb.nc[0]) % rb.nc[1], cz = c / (rb.nc[0] * rb.nc[1]);
-  float4 r;
-  r.x = (float)(x.x - (rb.lo[0] + cx * rb.w[0]));
-  r.y = (float)(x.y - (rb.lo[1] + cy * rb.w[1]));
-  r.z = (float)(x.z - (rb.lo[2] + cz * rb.w[2]));
-  r.w = __int_as_float(type_of(x.w));
-  d.rel[i] = r;
-}
-
 // ---------------------------------------------------------------------------
 // list rebuild of the flagged replicas: wrap + bin -> per-replica scan ->
 // scatter -> per-cell sort -> gather -> build
@@ -41,6 +30,57 @@ __device__ inline int3 wrap_shift(const RepBox &rb, const dbl4 &p) {
                    p.z < rb.lo[2] ? -1 : (p.z > rb.hi[2] ? 1 : 0));
 }
 
+// Search cell of an atom (clamped into the grid), its place in it: position relative to the
+// cell's origin and Morton index of the 4x4x4 sub-cell.
+struct CellPlace {
+  int c[3];
+  float rel[3];
+  uint32_t morton;
+};
+__device__ __forceinline__ uint32_t spread_bits(int s) { return (s & 1) | ((s & 2) << 2); }
+
+// The general case: any position.  Wraps p (single image, exactly as Domain::fix_position)
+// and counts the crossings (+1 through the upper face) as exchange_owned adds them to
+// msd_domain_cross.
+static __device__ __noinline__ void place_general(const Dev &d, const RepBox &rb, int i, dbl4 &p, CellPlace &q) {
+  const int3 w = wrap_shift(rb, p);
+  if (w.x | w.y | w.z) {
+    if (w.x) p.x += w.x > 0 ? -rb.L[0] : rb.L[0];
+    if (w.y) p.y += w.y > 0 ? -rb.L[1] : rb.L[1];
+    if (w.z) p.z += w.z > 0 ? -rb.L[2] : rb.L[2];
+    d.pos[i] = p;
+    if (d.img) {
+      int4 m = d.img[i];
+      m.x += w.x; m.y += w.y; m.z += w.z;
+      d.img[i] = m;
+    }
+  }
+  const double x[3] = {p.x, p.y, p.z};
+  q.morton = 0;
+  for (int a = 0; a < 3; ++a) {
+    const double u = (x[a] - rb.lo[a]) * rb.inv_w[a];
+    q.c[a] = min(max((int)floor(u), 0), rb.nc[a] - 1);
+    q.rel[a] = (float)(x[a] - (rb.lo[a] + q.c[a] * rb.w[a]));
+    q.morton |= spread_bits(min(max((int)((u - q.c[a]) * 4.0), 0), 3)) << a;
+  }
+}
+
+// An atom inside the box, along one axis: the cell coordinate in fixed point with 34
+// fractional bits (one subtraction and one FMA, which leaves the integer in the mantissa),
+// the rest by integers.  The FP64 pipe bound the binning kernel (79% busy, 61 us for 1,048,576
+// atoms: floors, conversions and compares, ~36 FP64 instructions per atom); 6 are left.  The
+// rounding, 2^-35 of a cell, is below the 1e-10 by which cells are wider than the list
+// cutoff at least.  False when the atom is not well inside, or the grid too long for this.
+__device__ __forceinline__ bool place_axis(double x, double lo, double inv_w, int nc, float wf, int &c, float &rel,
+                                           int &sub) {
+  const long long t = __double_as_longlong(fma(x - lo, inv_w * 17179869184.0, 6755399441055744.0));  // 2^34, 1.5 * 2^52
+  const long long n = t - 0x4338000000000000ll;
+  c = (int)(n >> 34);
+  sub = (int)(n >> 32) & 3;
+  rel = (float)(unsigned)((unsigned long long)n >> 2) * (wf * 2.3283064365386963e-10f);  // 2^-32
+  return (t >> 52) == 0x433 && n >= 1 && n < ((long long)nc << 34) - 1 && nc <= 65536;
+}
+
 // Thread of slot i (the whole warp calls this): wraps the atom, counts it in its cell and
 // copies its state, which rebuild_sort_gather takes back in the new order.
 __device__ __forceinline__ void rebuild_bin(const Dev &d, const Box &b, int forced, int i) {
@@ -51,41 +91,23 @@ __device__ __forceinline__ void rebuild_bin(const Dev &d, const Box &b, int forc
   if (act) {
     const RepBox &rb = repbox(b, rep);
     dbl4 p = d.pos[i];
-    // single-image wrap exactly as Domain::fix_position, counting the crossings
-    // (+1 through the upper face) as exchange_owned adds them to msd_domain_cross
-    const int3 w = wrap_shift(rb, p);
-    if (w.x | w.y | w.z) {  // the few atoms that left the box
-      if (w.x) p.x += w.x > 0 ? -rb.L[0] : rb.L[0];
-      if (w.y) p.y += w.y > 0 ? -rb.L[1] : rb.L[1];
-      if (w.z) p.z += w.z > 0 ? -rb.L[2] : rb.L[2];
-      d.pos[i] = p;
-      if (d.img) {
-        int4 m = d.img[i];
-        m.x += w.x; m.y += w.y; m.z += w.z;
-        d.img[i] = m;
-      }
-    }
-    const double ux = (p.x - rb.lo[0]) * rb.inv_w[0], uy = (p.y - rb.lo[1]) * rb.inv_w[1],
-                 uz = (p.z - rb.lo[2]) * rb.inv_w[2];
-    int cx = (int)floor(ux), cy = (int)floor(uy), cz = (int)floor(uz);
-    cx = min(max(cx, 0), rb.nc[0] - 1);
-    cy = min(max(cy, 0), rb.nc[1] - 1);
-    cz = min(max(cz, 0), rb.nc[2] - 1);
-    c = rb.cell_off + cx + rb.nc[0] * (cy + rb.nc[1] * cz);
+    CellPlace q;
+    int sx, sy, sz;
+    const bool inside = place_axis(p.x, rb.lo[0], rb.inv_w[0], rb.nc[0], rb.wf[0], q.c[0], q.rel[0], sx) &
+                        place_axis(p.y, rb.lo[1], rb.inv_w[1], rb.nc[1], rb.wf[1], q.c[1], q.rel[1], sy) &
+                        place_axis(p.z, rb.lo[2], rb.inv_w[2], rb.nc[2], rb.wf[2], q.c[2], q.rel[2], sz);
+    q.morton = spread_bits(sx) | (spread_bits(sy) << 1) | (spread_bits(sz) << 2);
+    if (!inside) place_general(d, rb, i, p, q);
+    c = rb.cell_off + q.c[0] + rb.nc[0] * (q.c[1] + rb.nc[1] * q.c[2]);
     d.atom_cell[i] = c;
-    // order inside the cell: the Morton index of the atom's 4x4x4 sub-cell, then its id,
-    // so that consecutive slots (a warp's lanes) sit close together and their neighbour
-    // lists run through the same candidates
-    const int sx = min(max((int)((ux - cx) * 4.0), 0), 3), sy = min(max((int)((uy - cy) * 4.0), 0), 3),
-              sz = min(max((int)((uz - cz) * 4.0), 0), 3);
-    const uint32_t morton = (sx & 1) | ((sy & 1) << 1) | ((sz & 1) << 2) | ((sx & 2) << 2) | ((sy & 2) << 3) |
-                            ((sz & 2) << 4);
+    // order inside the cell: the sub-cell, then the id, so that consecutive slots (a warp's
+    // lanes) sit close together and their neighbour lists run through the same candidates
     const uint32_t id = d.id[i];
-    d.skey[i] = ((uint64_t)morton << 32) | id;
+    d.skey[i] = ((uint64_t)q.morton << 32) | id;
     d.t_pos[i] = p;
     d.t_vel[i] = d.vel[i];
     d.t_acc[i] = d.acc[i];  // a(t): the next kick reads it as a_old
-    d.t_type[i] = d.type[i];
+    d.t_rel[i] = make_float4(q.rel[0], q.rel[1], q.rel[2], __int_as_float(type_of(p.w)));
     d.t_id[i] = id;
     if (d.img) d.t_img[i] = d.img[i];
     if (d.mol) d.t_mol[i] = d.mol[i];
@@ -116,15 +138,17 @@ __device__ __forceinline__ void rebuild_gather(const Dev &d, const RepBox &rb, i
   d.pos_ref[k] = x;
   d.vel[k] = d.t_vel[o];
   d.acc[k] = d.t_acc[o];
-  d.type[k] = d.t_type[o];
+  const float4 rel = d.t_rel[o];
+  d.rel[k] = rel;
+  const int type = __float_as_int(rel.w);
+  d.type[k] = type;
   d.id[k] = d.t_id[o];
   if (d.img) d.img[k] = d.t_img[o];
   if (d.mol) d.mol[k] = d.t_mol[o];
   d.cell_of[k] = d.atom_cell[o];
-  update_rel(d, rb, k, x);
   if (d.ic) {
     int3 w;
-    const int4 q = fixed_pos(rb, x, type_of(x.w), w);
+    const int4 q = fixed_pos(rb, x, type, w);
     d.ic[k] = q;
     if (d.ic_ref) d.ic_ref[k] = fixed_ref(q, w);
   }
