@@ -47,6 +47,12 @@ struct GraphEntry {
   ChunkPlan plan;
 };
 
+// what the host reads back of a context: adjacent on the device, one copy
+struct Status {
+  double thermo[8];
+  int flags[F_NWORDS];
+};
+
 // autotuner results, per process: a system of the same kind and size on the same
 // device reuses the launch shape measured for the first one
 struct TuneKey {
@@ -83,8 +89,11 @@ struct cavgpu_ctx {
   int max_nb = 0;
   std::deque<GraphEntry> graphs;                      // stable references (chunks in flight hold them)
   std::map<std::pair<int, int>, ChunkPlan> eager_plans;  // chunks that are not graphs
-  // status words of the last chunks, read back without a full synchronisation
-  int *h_status = nullptr;   // pinned, 2 x F_NWORDS
+  // the status block (thermo and flags, adjacent on the device) in pinned memory: two copies
+  // for the chunks in flight, read back without a full synchronisation, one for other reads
+  Status *h_status = nullptr;
+  bool nan_seen = false;     // F_NAN and F_PASSES of the last status read
+  int passes = 0;
   cudaEvent_t ev_status[2] = {nullptr, nullptr};
   // reference binning (Neighborlist::init, src/neighborlist.cpp:334-342), single system
   double cutoff_extra = 0.0, cutoff_inv = 0.0, lo_local[3] = {0, 0, 0};
@@ -356,18 +365,39 @@ GraphEntry *get_graph(cavgpu_ctx *c, int S, int every, int *rc) {
   return &c->graphs.back();
 }
 
-int read_flags(cavgpu_ctx *c, int *f) {
-  CK(cudaMemcpyAsync(f, c->d.flags, F_NWORDS * sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
+int ensure_status(cavgpu_ctx *c) {
+  if (c->h_status) return CAVGPU_OK;
+  Status *h = nullptr;
+  CK(cudaMallocHost(&h, 3 * sizeof(Status)));
+  c->h_status = h;
+  for (auto &e : c->ev_status) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   return CAVGPU_OK;
 }
 
-int check_status(cavgpu_ctx *c) {
-  int f[F_NWORDS];
-  RK(read_flags(c, f));
-  c->max_nb = std::max(c->max_nb, f[F_MAXNB]);
-  if (f[F_NAN]) return CAVGPU_E_NAN;
-  if (f[F_OVERFLOW]) return CAVGPU_E_NLIST_OVERFLOW;
+// the status block as it is once the stream has done its work (one copy, one wait)
+int read_status(cavgpu_ctx *c, const Status **out) {
+  RK(ensure_status(c));
+  Status *h = c->h_status + 2;
+  CK(cudaMemcpyAsync(h, c->d.thermo, sizeof(Status), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  c->nan_seen = h->flags[F_NAN] != 0;
+  c->passes = h->flags[F_PASSES];
+  *out = h;
+  return CAVGPU_OK;
+}
+
+int read_flags(cavgpu_ctx *c, int *f) {
+  const Status *h = nullptr;
+  RK(read_status(c, &h));
+  std::memcpy(f, h->flags, sizeof(h->flags));
+  return CAVGPU_OK;
+}
+
+// zeroes every status word but the rebuild counts and the step kernel's phase
+int clear_status(cavgpu_ctx *c) {
+  static_assert(F_REBUILDS == 5 && F_PASSES == 6 && F_HALT == 7 && F_PHASE_REQ == 12, "word order");
+  CK(cudaMemsetAsync(c->d.flags, 0, F_REBUILDS * sizeof(int), c->st));
+  CK(cudaMemsetAsync(c->d.flags + F_HALT, 0, (F_PHASE - F_HALT) * sizeof(int), c->st));
   return CAVGPU_OK;
 }
 
@@ -439,16 +469,10 @@ int alloc_nbr(cavgpu_ctx *c, int cap) {
 // as they were (a build that completes a step whose own rebuild overflowed, or
 // that restarts from a snapshot, is not a rebuild of the trajectory).
 int forced_build(cavgpu_ctx *c, bool count = true) {
-  int f0[F_NWORDS];
-  RK(read_flags(c, f0));
+  int f0[F_NWORDS], f[F_NWORDS];
+  if (!count) RK(read_flags(c, f0));
   for (int attempt = 0; attempt < 4; ++attempt) {
-    int zero[F_NWORDS] = {0};
-    int f[F_NWORDS];
-    if (attempt == 0) std::memcpy(f, f0, sizeof(f));  // nothing ran since f0 was read
-    else RK(read_flags(c, f));
-    zero[F_REBUILDS] = f[F_REBUILDS];
-    zero[F_PASSES] = f[F_PASSES];
-    CK(cudaMemcpyAsync(c->d.flags, zero, sizeof(zero), cudaMemcpyHostToDevice, c->st));
+    RK(clear_status(c));
     RK(launch_rebuild(c->d, c->b, c->lc, 1, c->st));
     c->kernel_launches += rebuild_kernels(c->b, c->lc);
     RK(read_flags(c, f));
@@ -457,11 +481,34 @@ int forced_build(cavgpu_ctx *c, bool count = true) {
       if (!count) {
         f[F_REBUILDS] = f0[F_REBUILDS];
         f[F_PASSES] = f0[F_PASSES];
+        c->passes = f0[F_PASSES];
         CK(cudaMemcpyAsync(c->d.flags, f, sizeof(f), cudaMemcpyHostToDevice, c->st));
         CK(cudaStreamSynchronize(c->st));
       }
       return CAVGPU_OK;
     }
+    RK(alloc_nbr(c, (int)(f[F_OVERFLOW] * 1.25) + 32));
+  }
+  return CAVGPU_E_NLIST_OVERFLOW;
+}
+
+// Forced list build, forces, virial, potential energy and temperature at the current
+// positions, enqueued together and waited for once: a build that outgrows its rows halts
+// what follows it, and all of it is done again with longer rows.
+int build_and_force(cavgpu_ctx *c, const Status **out) {
+  for (int attempt = 0; attempt < 4; ++attempt) {
+    RK(clear_status(c));
+    RK(launch_rebuild(c->d, c->b, c->lc, 1, c->st));
+    RK(launch_force(c->d, c->b, c->sc, c->lc, 0, 1, 0, FUSE_NONE, 0, 0, c->st));
+    if (c->b.nrep == 1)
+      RK(launch_thermo_final(c->d, c->tc, force_grid_blocks(c->lc), ev_grid_blocks(c->lc), 0, -1, c->st));
+    else
+      RK(launch_thermo_replicas(c->d, c->b, c->tc, 1, 1, c->st));
+    c->kernel_launches += rebuild_kernels(c->b, c->lc) + force_kernels(c->lc) + 1;
+    RK(read_status(c, out));
+    const int *f = (*out)->flags;
+    c->max_nb = f[F_MAXNB];
+    if (!f[F_OVERFLOW]) return f[F_NAN] ? CAVGPU_E_NAN : CAVGPU_OK;
     RK(alloc_nbr(c, (int)(f[F_OVERFLOW] * 1.25) + 32));
   }
   return CAVGPU_E_NLIST_OVERFLOW;
@@ -609,12 +656,14 @@ int create_common(const cavgpu_params *p, int nrep, const double *lo3, const dou
     return CAVGPU_E_CUDA;
   }
   int rc = dalloc(c, &c->d.tab, 1);
-  if (!rc) rc = dalloc(c, &c->d.flags, F_NWORDS);
+  Status *status = nullptr;
+  if (!rc) rc = dalloc(c, &status, 1);
+  c->d.thermo = status ? status->thermo : nullptr;
+  c->d.flags = status ? status->flags : nullptr;
   c->d.req = c->d.flags + F_REBUILD;
   c->d.nan = c->d.flags + F_NAN;
   if (!rc) rc = dalloc(c, &c->d.barrier, 1);
   if (!rc) rc = cuda_rc(cudaMemsetAsync(c->d.barrier, 0, sizeof(unsigned int), c->st));
-  if (!rc) rc = dalloc(c, &c->d.thermo, 8);
   if (!rc) rc = dalloc(c, &c->d.step_base, 1);
   if (!rc) rc = dalloc(c, &c->d.thermo_ring, THERMO_REC * (size_t)MAX_GRAPH_STEPS);
   if (!rc) rc = dalloc(c, &c->d.fold, 10 * (size_t)THERMO_FOLD_BLOCKS);
@@ -624,8 +673,7 @@ int create_common(const cavgpu_params *p, int nrep, const double *lo3, const dou
   if (!rc) rc = dalloc(c, &c->d.force_ticket, 1);
   if (!rc) rc = cuda_rc(cudaMemsetAsync(c->d.force_ticket, 0, sizeof(unsigned int), c->st));
   if (!rc) rc = cuda_rc(cudaMemcpyAsync(c->d.tab, &c->tab_h, sizeof(PairTab), cudaMemcpyHostToDevice, c->st));
-  if (!rc) rc = cuda_rc(cudaMemsetAsync(c->d.flags, 0, F_NWORDS * sizeof(int), c->st));
-  if (!rc) rc = cuda_rc(cudaMemsetAsync(c->d.thermo, 0, 8 * sizeof(double), c->st));
+  if (!rc) rc = cuda_rc(cudaMemsetAsync(status, 0, sizeof(Status), c->st));
   const long long step0 = p->initial_step;  // Md_simulator::initial_step
   if (!rc) rc = cuda_rc(cudaMemcpyAsync(c->d.step_base, &step0, sizeof(long long), cudaMemcpyHostToDevice, c->st));
   if (!rc) rc = cuda_rc(cudaStreamSynchronize(c->st));
@@ -910,26 +958,9 @@ int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, cons
 
 int setup_common(cavgpu_ctx *c) {
   if (!c->uploaded) return CAVGPU_E_STATE;
-  RK(forced_build(c));
-  RK(launch_force(c->d, c->b, c->sc, c->lc, 0, 1, 0, FUSE_NONE, 0, 0, c->st));
-  c->kernel_launches += force_kernels(c->lc);
-  if (c->b.nrep == 1) {
-    RK(launch_thermo_final(c->d, c->tc, force_grid_blocks(c->lc), ev_grid_blocks(c->lc), 0, -1, c->st));
-  } else {
-    RK(launch_thermo_replicas(c->d, c->b, c->tc, 1, 1, c->st));
-  }
-  c->kernel_launches += 1;
-  RK(check_status(c));
+  const Status *h = nullptr;
+  RK(build_and_force(c, &h));
   c->set_up = true;
-  return CAVGPU_OK;
-}
-
-int ensure_status(cavgpu_ctx *c) {
-  if (c->h_status) return CAVGPU_OK;
-  int *h = nullptr;
-  CK(cudaMallocHost(&h, 2 * F_NWORDS * sizeof(int)));
-  c->h_status = h;
-  for (auto &e : c->ev_status) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   return CAVGPU_OK;
 }
 
@@ -986,9 +1017,8 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
   const bool small = !eager && !c->prof && c->nve.step == 0 && chunk_fits(c->b, c->lc);
   RK(ensure_status(c));
   int f[F_NWORDS];
-  RK(read_flags(c, f));
-  if (f[F_NAN]) return CAVGPU_E_NAN;  // a context that met a NaN does not step again
-  const int passes0 = f[F_PASSES];
+  if (c->nan_seen) return CAVGPU_E_NAN;  // a context that met a NaN does not step again
+  const int passes0 = c->passes;
   struct InFlight {
     int64_t start;
     int sz, slot;
@@ -1039,8 +1069,7 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
       if (every > 0 && nrec > 0)
         CK(cudaMemcpyAsync(out5 + THERMO_REC * ((launched + ev) / every - 1), c->d.thermo_ring,
                            THERMO_REC * sizeof(double) * nrec, cudaMemcpyDeviceToHost, c->st));
-      CK(cudaMemcpyAsync(c->h_status + slot * F_NWORDS, c->d.flags, F_NWORDS * sizeof(int), cudaMemcpyDeviceToHost,
-                         c->st));
+      CK(cudaMemcpyAsync(c->h_status + slot, c->d.thermo, sizeof(Status), cudaMemcpyDeviceToHost, c->st));
       CK(cudaEventRecord(c->ev_status[slot], c->st));
       q.push_back({launched, sz, slot, plan});
       slot ^= 1;
@@ -1049,8 +1078,10 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
     const InFlight p = q.front();
     q.pop_front();
     CK(cudaEventSynchronize(c->ev_status[p.slot]));
-    const int *hf = c->h_status + p.slot * F_NWORDS;
+    const int *hf = c->h_status[p.slot].flags;
     c->max_nb = std::max(c->max_nb, hf[F_MAXNB]);
+    c->nan_seen = hf[F_NAN] != 0;
+    c->passes = hf[F_PASSES];
     if (hf[F_STALL]) return CAVGPU_E_CUDA;  // a grid barrier of the step kernel gave up
     if (c->prof) RK(collect_profile(c, p.sz));
     if (!hf[F_HALT]) {
@@ -1074,12 +1105,10 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
     c->steps_done += 1;
     launched = done;
   }
-  RK(check_status(c));
+  // the last chunk's status (or that of a completed overflow step) has come with its event;
   // rebuild kernels launched by the graphs' conditional nodes
-  if (!eager && !small) {
-    RK(read_flags(c, f));
-    if (f[F_PASSES] > passes0) c->kernel_launches += (long long)rebuild_kernels(c->b, c->lc) * (f[F_PASSES] - passes0);
-  }
+  if (!eager && !small && c->passes > passes0)
+    c->kernel_launches += (long long)rebuild_kernels(c->b, c->lc) * (c->passes - passes0);
   return CAVGPU_OK;
 }
 
@@ -1250,6 +1279,7 @@ int cavgpu_autotune(cavgpu_ctx *c, int32_t trial_steps, int32_t flags, int64_t *
     c->lc.block = block;
     c->lc.use_seg = seg;
     c->d.tpa = tpa;
+    c->nan_seen = false;  // (a trial's; the build below reads the snapshot's)
     RK(alloc_nbr(c, c->d.cap));
     for (int k = 0; k < 3; ++k)
       CK(cudaMemcpyAsync(src4[k], snap + k * NS, NS * sizeof(dbl4), cudaMemcpyDeviceToDevice, c->st));
@@ -1269,6 +1299,7 @@ int cavgpu_autotune(cavgpu_ctx *c, int32_t trial_steps, int32_t flags, int64_t *
     // the forced build is not a rebuild of the trajectory: keep the counts of the snapshot
     f[F_REBUILDS] = snap_flags[F_REBUILDS];
     f[F_PASSES] = snap_flags[F_PASSES];
+    c->passes = f[F_PASSES];
     CK(cudaMemcpyAsync(c->d.flags, f, sizeof(f), cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
     return CAVGPU_OK;
@@ -1356,22 +1387,11 @@ int cavgpu_autotune(cavgpu_ctx *c, int32_t trial_steps, int32_t flags, int64_t *
 int cavgpu_forces(cavgpu_ctx *c, double *virial, double *pe) {
   if (!c) return CAVGPU_E_ARG;
   if (!c->set_up) return CAVGPU_E_STATE;
-  RK(forced_build(c));
-  RK(launch_force(c->d, c->b, c->sc, c->lc, 0, 1, 0, FUSE_NONE, 0, 0, c->st));
-  c->kernel_launches += force_kernels(c->lc);
+  const Status *h = nullptr;
+  RK(build_and_force(c, &h));
   if (c->b.nrep == 1) {
-    RK(launch_thermo_final(c->d, c->tc, force_grid_blocks(c->lc), ev_grid_blocks(c->lc), 0, -1, c->st));
-  } else {
-    RK(launch_thermo_replicas(c->d, c->b, c->tc, 1, 1, c->st));
-  }
-  c->kernel_launches += 1;
-  RK(check_status(c));
-  if (c->b.nrep == 1) {
-    double th[8];
-    CK(cudaMemcpyAsync(th, c->d.thermo, sizeof(th), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    if (virial) *virial = th[3];
-    if (pe) *pe = th[4];
+    if (virial) *virial = h->thermo[3];
+    if (pe) *pe = h->thermo[4];
   } else {  // sums over the replicas
     std::vector<double> th(8 * (size_t)c->b.nrep);
     CK(cudaMemcpyAsync(th.data(), c->d.thermo_rep, th.size() * sizeof(double), cudaMemcpyDeviceToHost, c->st));
@@ -1388,12 +1408,10 @@ int cavgpu_thermo(cavgpu_ctx *c, double *out6) {
   if (!c || !out6) return CAVGPU_E_ARG;
   if (!c->set_up) return CAVGPU_E_STATE;
   if (c->b.nrep > 1) return CAVGPU_E_ARG;  // cavgpu_thermo_batch
-  double th[8];
-  int f[F_NWORDS];
-  CK(cudaMemcpyAsync(th, c->d.thermo, sizeof(th), cudaMemcpyDeviceToHost, c->st));
-  RK(read_flags(c, f));
-  for (int k = 0; k < 5; ++k) out6[k] = th[k];
-  out6[5] = (double)f[F_REBUILDS];
+  const Status *h = nullptr;
+  RK(read_status(c, &h));
+  for (int k = 0; k < 5; ++k) out6[k] = h->thermo[k];
+  out6[5] = (double)h->flags[F_REBUILDS];
   return CAVGPU_OK;
 }
 
@@ -1413,13 +1431,17 @@ int cavgpu_thermo_batch(cavgpu_ctx *c, double *out6) {
 int cavgpu_download(cavgpu_ctx *c, double *pos3, double *vel3, double *acc3) {
   if (!c) return CAVGPU_E_ARG;
   if (!c->uploaded) return CAVGPU_E_STATE;
-  double *outs[3] = {pos3, vel3, acc3};
-  for (int w = 0; w < 3; ++w) {
-    if (!outs[w]) continue;
-    RK(launch_to_host_order(c->d, c->b, w, c->st));
-    CK(cudaMemcpyAsync(outs[w], c->d.h3, 3 * sizeof(double) * c->natoms, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-  }
+  // one kernel, the copies and one wait; the rebuild's scratch holds the host-order arrays
+  // (24 of its 32 bytes per slot)
+  double *const outs[3] = {pos3, vel3, acc3};
+  double *const stage[3] = {reinterpret_cast<double *>(c->d.t_pos), reinterpret_cast<double *>(c->d.t_vel),
+                            reinterpret_cast<double *>(c->d.t_acc)};
+  RK(launch_state_to_host(c->d, c->b, pos3 ? stage[0] : nullptr, vel3 ? stage[1] : nullptr, acc3 ? stage[2] : nullptr,
+                          c->st));
+  for (int w = 0; w < 3; ++w)
+    if (outs[w])
+      CK(cudaMemcpyAsync(outs[w], stage[w], 3 * sizeof(double) * c->natoms, cudaMemcpyDeviceToHost, c->st));
+  CK(cudaStreamSynchronize(c->st));
   return CAVGPU_OK;
 }
 
@@ -1461,7 +1483,7 @@ int cavgpu_export_bins(cavgpu_ctx *c, int32_t *owned3, int32_t *nbins3) {
   if (!c->uploaded) return CAVGPU_E_STATE;
   if (nbins3) for (int a = 0; a < 3; ++a) nbins3[a] = c->ref_nb[a];
   if (!owned3) return CAVGPU_OK;
-  RK(launch_to_host_order(c->d, c->b, 0, c->st));
+  RK(launch_to_host_order(c->d, c->b, c->st));
   RK(launch_ref_bins(c->d, c->natoms, c->cutoff_inv, c->ref_nb, c->lo_local, c->st));
   CK(cudaMemcpyAsync(owned3, c->d.hi3, 3 * sizeof(int32_t) * c->natoms, cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
@@ -1488,7 +1510,7 @@ int64_t cavgpu_export_ghosts(cavgpu_ctx *c, double ghost_cutoff, int32_t *src, i
   M((void **)&gp, (size_t)gcap * 3 * sizeof(double));
   M((void **)&gb, (size_t)gcap * 3 * sizeof(int32_t));
   int total = 0;
-  if (!rc) rc = launch_to_host_order(c->d, c->b, 0, c->st);
+  if (!rc) rc = launch_to_host_order(c->d, c->b, c->st);
   if (!rc) rc = launch_ghosts(c->d, c->b, N, ghost_cutoff, counts, starts, gs, gsh, gp, gb, gcap, c->cutoff_inv,
                               c->ref_nb, c->lo_local, c->st);
   if (!rc) rc = cuda_rc(cudaMemcpyAsync(&total, starts + N, sizeof(int), cudaMemcpyDeviceToHost, c->st));

@@ -563,7 +563,10 @@ struct NveCfg {
 constexpr int NVE_BLOCKS = 1024;
 int launch_nve(const Dev &d, const Box &b, const ThermoCfg &tc, const NveCfg &cfg, int k, int thermo, int ring_slot,
                cudaStream_t st);
-int launch_to_host_order(const Dev &d, const Box &b, int what, cudaStream_t st);
+// positions wrapped as Domain::fix_position would, in host order into d.h3
+int launch_to_host_order(const Dev &d, const Box &b, cudaStream_t st);
+// positions (wrapped), velocities, accelerations in host order; null: left out
+int launch_state_to_host(const Dev &d, const Box &b, double *pos3, double *vel3, double *acc3, cudaStream_t st);
 // boundary crossings per atom in host order into d.hi3, counting the wrap of the
 // current position that the next list build applies
 int launch_images_to_host(const Dev &d, const Box &b, cudaStream_t st);

@@ -435,21 +435,30 @@ __global__ void __launch_bounds__(256) k_nve_scale(Dev d, int n, NveCfg c, int k
 // ---------------------------------------------------------------------------
 // parity exports
 // ---------------------------------------------------------------------------
-// what: 0 = positions (wrapped as Domain::fix_position), 1 = velocities, 2 = accelerations
-__global__ void __launch_bounds__(256) k_to_host_order(Dev d, Box b, int what) {
+// The state in host order: positions wrapped as Domain::fix_position, velocities,
+// accelerations, each where asked for (one pass over the ids and one launch for all).
+__global__ void __launch_bounds__(256) k_state_to_host(Dev d, Box b, double *pos3, double *vel3, double *acc3) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= b.nslot) return;
   const int rep = rep_of_slot(b, k);
   if (rep < 0) return;
-  dbl4 v = what == 0 ? d.pos[k] : (what == 1 ? d.vel[k] : d.acc[k]);
   const RepBox &rb = repbox(b, rep);
-  if (what == 0) {
+  const size_t h = ((size_t)rb.id_off + d.id[k]) * 3;
+  if (pos3) {
+    dbl4 v = d.pos[k];
     if (v.x < rb.lo[0]) v.x += rb.L[0]; else if (v.x > rb.hi[0]) v.x -= rb.L[0];
     if (v.y < rb.lo[1]) v.y += rb.L[1]; else if (v.y > rb.hi[1]) v.y -= rb.L[1];
     if (v.z < rb.lo[2]) v.z += rb.L[2]; else if (v.z > rb.hi[2]) v.z -= rb.L[2];
+    pos3[h] = v.x; pos3[h + 1] = v.y; pos3[h + 2] = v.z;
   }
-  const size_t h = ((size_t)rb.id_off + d.id[k]) * 3;
-  d.h3[h] = v.x; d.h3[h + 1] = v.y; d.h3[h + 2] = v.z;
+  if (vel3) {
+    const dbl4 v = d.vel[k];
+    vel3[h] = v.x; vel3[h + 1] = v.y; vel3[h + 2] = v.z;
+  }
+  if (acc3) {
+    const dbl4 v = d.acc[k];
+    acc3[h] = v.x; acc3[h + 1] = v.y; acc3[h + 2] = v.z;
+  }
 }
 
 // boundary crossings in host order: the stored counts plus the wrap the current
@@ -739,9 +748,13 @@ int launch_nve(const Dev &d, const Box &b, const ThermoCfg &tc, const NveCfg &cf
   return chk();
 }
 
-int launch_to_host_order(const Dev &d, const Box &b, int what, cudaStream_t st) {
-  k_to_host_order<<<ceil_div(b.nslot, 256), 256, 0, st>>>(d, b, what);
+int launch_state_to_host(const Dev &d, const Box &b, double *pos3, double *vel3, double *acc3, cudaStream_t st) {
+  k_state_to_host<<<ceil_div(b.nslot, 256), 256, 0, st>>>(d, b, pos3, vel3, acc3);
   return chk();
+}
+
+int launch_to_host_order(const Dev &d, const Box &b, cudaStream_t st) {
+  return launch_state_to_host(d, b, d.h3, nullptr, nullptr, st);
 }
 
 int launch_images_to_host(const Dev &d, const Box &b, cudaStream_t st) {
