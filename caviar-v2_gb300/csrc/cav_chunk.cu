@@ -226,7 +226,7 @@ __device__ __forceinline__ void mixed_task(const Dev &d, const Box &b, const Ste
   fold_lanes<A, EV>(fx, fy, fz, vir, pe);
   if (act && t == 0) {
     finish_atom<true, KICK, EV>(d, b, sc, tab, i, ti, rep, step, fuse, fx, fy, fz, ke);
-    if (EV) add_ev(d, i, vir, pe, ev);
+    if (EV) set_ev(d, i, vir, pe, ev);
   }
 }
 

@@ -79,7 +79,11 @@ __global__ void __launch_bounds__(CLOSE_THREADS) k_close64(Dev d, Box b, StepCon
     double F[3];
     close_sum<TPA, false>(d, rep >= 0, i, t, F);
     if (rep >= 0 && t == 0) {
-      finish_atom<false, KICK, EV>(d, b, sc, tab, i, d.type[i], rep, step, fa.fuse, F[0], F[1], F[2], ke_p);
+      double ke[4];
+      finish_atom<false, KICK, EV>(d, b, sc, tab, i, d.type[i], rep, step, fa.fuse, F[0], F[1], F[2], ke);
+      if (EV)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ke_p[q] += ke[q];
       if (EV && d.ev_part) close_ev<TPA>(d, i);
     }
   }

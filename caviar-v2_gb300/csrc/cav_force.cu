@@ -117,11 +117,13 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
   const int warps_total = (gridDim.x * blockDim.x) >> 5;
   const int ntask = was_halted ? 0 : (n + A - 1) / A;
   // EV: each thread's KE / virial / PE sums live in shared memory between tasks;
-  // six doubles held in registers across the pair loop spill at 64 registers
-  __shared__ double s_sum[EV ? 6 * 256 : 1];
+  // six doubles held in registers across the pair loop spill at 64 registers (dynamic, no
+  // larger than the block: what shared memory takes, the gathers miss in L1)
+  extern __shared__ double s_sum[];
+  const int nthr = blockDim.x;
   if (EV)
 #pragma unroll
-    for (int q = 0; q < 6; ++q) s_sum[q * 256 + threadIdx.x] = 0.0;
+    for (int q = 0; q < 6; ++q) s_sum[q * nthr + threadIdx.x] = 0.0;
   long long step = 0;
   if (KICK == 2) step = *d.step_base + fa.k_in_chunk;
   int img_rep = -1;
@@ -168,25 +170,25 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
         if (EV) vir = F[3], pe = F[4];
       }
     }
-    double ke_t[4] = {0.0, 0.0, 0.0, 0.0}, ev_t[2] = {0.0, 0.0};
     fold_lanes<A, EV>(fx, fy, fz, vir, pe);
     if (act && t == 0) {
-      finish_atom<MIXED, KICK, EV>(d, b, sc, tab, i, ti, rep, step, fa.fuse, fx, fy, fz, ke_t);
-      if (EV) add_ev(d, i, vir, pe, ev_t);
-    }
-    if (EV) {
+      double ke[4], ev[2];
+      finish_atom<MIXED, KICK, EV>(d, b, sc, tab, i, ti, rep, step, fa.fuse, fx, fy, fz, ke);
+      if (EV) {
+        set_ev(d, i, vir, pe, ev);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) s_sum[q * 256 + threadIdx.x] += ke_t[q];
+        for (int q = 0; q < 4; ++q) s_sum[q * nthr + threadIdx.x] += ke[q];
 #pragma unroll
-      for (int q = 0; q < 2; ++q) s_sum[(4 + q) * 256 + threadIdx.x] += ev_t[q];
+        for (int q = 0; q < 2; ++q) s_sum[(4 + q) * nthr + threadIdx.x] += ev[q];
+      }
     }
   }
   double ke_p[4] = {0.0, 0.0, 0.0, 0.0}, ev_p[2] = {0.0, 0.0};
   if (EV) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) ke_p[q] = s_sum[q * 256 + threadIdx.x];
+    for (int q = 0; q < 4; ++q) ke_p[q] = s_sum[q * nthr + threadIdx.x];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) ev_p[q] = s_sum[(4 + q) * 256 + threadIdx.x];
+    for (int q = 0; q < 2; ++q) ev_p[q] = s_sum[(4 + q) * nthr + threadIdx.x];
   }
   if (!was_halted) store_partials<KICK, EV>(d, ke_p, ev_p);
   if (KICK != 0) end_of_step<EV>(d, was_halted, fa);
@@ -320,8 +322,15 @@ __global__ void __launch_bounds__(256) k_force_seg(Dev d, Box b, StepConsts sc, 
         }
         fold_lanes<A, EV>(fx, fy, fz, vir, pe);
         if (act && t == 0) {
-          finish_atom<true, KICK, EV>(d, b, sc, tab, i, ti, rep, step, fa.fuse, fx, fy, fz, ke_p);
-          if (EV) add_ev(d, i, vir, pe, ev_p);
+          double ke[4], ev[2];
+          finish_atom<true, KICK, EV>(d, b, sc, tab, i, ti, rep, step, fa.fuse, fx, fy, fz, ke);
+          if (EV) {
+            set_ev(d, i, vir, pe, ev);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) ke_p[q] += ke[q];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) ev_p[q] += ev[q];
+          }
         }
       }
     }
@@ -333,12 +342,13 @@ __global__ void __launch_bounds__(256) k_force_seg(Dev d, Box b, StepConsts sc, 
 template <int TPA, bool MIXED, int KICK>
 static void launch_ev(bool ev, bool one, int grid, int block, const Dev &d, const Box &b, const StepConsts &sc,
                       const ForceArgs &fa, cudaStream_t st) {
+  const size_t ev_smem = (size_t)6 * block * sizeof(double);
   if (one) {  // single-type systems: pair constants in registers
-    if (ev) k_force<TPA, MIXED, KICK, true, true><<<grid, block, 0, st>>>(d, b, sc, fa);
+    if (ev) k_force<TPA, MIXED, KICK, true, true><<<grid, block, ev_smem, st>>>(d, b, sc, fa);
     else k_force<TPA, MIXED, KICK, false, true><<<grid, block, 0, st>>>(d, b, sc, fa);
     return;
   }
-  if (ev) k_force<TPA, MIXED, KICK, true, false><<<grid, block, 0, st>>>(d, b, sc, fa);
+  if (ev) k_force<TPA, MIXED, KICK, true, false><<<grid, block, ev_smem, st>>>(d, b, sc, fa);
   else k_force<TPA, MIXED, KICK, false, false><<<grid, block, 0, st>>>(d, b, sc, fa);
 }
 

@@ -37,12 +37,10 @@ __device__ inline void block_sum_store(double (&v)[NV], double *out /* NV double
 #pragma unroll
     for (int k = 0; k < NV; ++k) sh[wid][k] = v[k];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < NV; ++k) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s += sh[w][k];
-      out[k] = s;
-    }
+  if (threadIdx.x < NV) {  // a thread per value
+    double s = 0.0;
+    for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
+    out[threadIdx.x] = s;
   }
 }
 

@@ -23,12 +23,11 @@ __device__ inline void block_sum_store_f(double (&v)[NV], double *out) {
 #pragma unroll
     for (int k = 0; k < NV; ++k) sh[wid][k] = v[k];
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (int k = 0; k < NV; ++k) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s += sh[w][k];
-      out[k] = s;
-    }
+  if (threadIdx.x < NV) {  // a thread per value: an FP64 add takes a warp 64 cycles, whoever needs it
+    double s = 0.0;
+    for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
+    out[threadIdx.x] = s;
+  }
 }
 
 struct SmemTabD {
@@ -121,7 +120,7 @@ __device__ __forceinline__ void fold_lanes(double &fx, double &fy, double &fz, d
 // KICK: 0 = store the acceleration only; 1 = velocity-Verlet closing kick
 // v += (a + a_old) * (0.5 dt) (src/md_simulator.cpp:672-679); 2 = Langevin closing
 // update v = (v a_L + eta b) + (a*0.5) dt (src/md_simulator.cpp:853-862).
-// EV: accumulate the KE (KICK == 2: that of the velocities at the end of the step, kept
+// EV: the atom's KE terms into `ke` (KICK == 2: that of the velocities at the end of the step, kept
 // apart from the mid-step temperature's).
 // fuse: then the first half of the next step, with the arithmetic of the drift
 // kernels (k_drift_vv, k_drift_lf, k_lang_a): the NaN check of the new acceleration,
@@ -132,7 +131,7 @@ __device__ __forceinline__ void fold_lanes(double &fx, double &fy, double &fz, d
 template <bool MIXED, int KICK, bool EV, class Tab>
 __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const StepConsts &sc, const Tab &tab, int i,
                                             int ti, int rep, long long step, int fuse, double fx, double fy,
-                                            double fz, double (&ke_p)[4]) {
+                                            double fz, double (&ke)[4]) {
   const double mi = tab.minv[ti];
   dbl4 an = make_dbl4(fx * mi, fy * mi, fz * mi, 0.0);
   dbl4 v;
@@ -141,8 +140,8 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     if (EV) {
       v = d.vel[i];
       const double m = tab.mass[ti];
-      ke_p[0] += twice_ke(m, v);
-      ke_p[1] += m * v.x; ke_p[2] += m * v.y; ke_p[3] += m * v.z;
+      ke[0] = twice_ke(m, v);
+      ke[1] = m * v.x; ke[2] = m * v.y; ke[3] = m * v.z;
     }
   } else if (KICK == 1) {
     v = d.vel[i];
@@ -158,8 +157,8 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
     if (EV) {
       const double m = tab.mass[ti];
-      ke_p[0] += twice_ke(m, v);
-      ke_p[1] += m * v.x; ke_p[2] += m * v.y; ke_p[3] += m * v.z;
+      ke[0] = twice_ke(m, v);
+      ke[1] = m * v.x; ke[2] = m * v.y; ke[3] = m * v.z;
     }
   } else {
     v = d.vel[i];
@@ -179,8 +178,8 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
     if (EV) {  // Atom_data::kinetic_energy() read after the step (the temperature was taken mid-step)
       const double m = tab.mass[ti];
-      ke_p[0] += twice_ke(m, v);
-      ke_p[1] += m * v.x; ke_p[2] += m * v.y; ke_p[3] += m * v.z;
+      ke[0] = twice_ke(m, v);
+      ke[1] = m * v.x; ke[2] = m * v.y; ke[3] = m * v.z;
     }
   }
   if (KICK != 0) {
@@ -219,9 +218,9 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
 }
 
 // virial and potential energy of atom i (both orders of its pairs are counted)
-__device__ __forceinline__ void add_ev(const Dev &d, int i, double vir, double pe, double (&ev_p)[2]) {
-  ev_p[0] += vir;
-  ev_p[1] += pe;
+__device__ __forceinline__ void set_ev(const Dev &d, int i, double vir, double pe, double (&ev)[2]) {
+  ev[0] = vir;
+  ev[1] = pe;
   if (d.ev_atom) d.ev_atom[i] = make_double2(vir, pe);
 }
 
