@@ -725,11 +725,12 @@ int build_segments(cavgpu_ctx *c) {
 // below that more lanes per atom shorten the walk through a list.  In the FP64 form 1, 2
 // and 4 lanes give the same sums bit for bit (RowSplit): a batch's replicas equal their
 // single-system runs whatever the sizes.
-// Step times with 1, 2 and 4 lanes (LJ fluid, us): 4,000 atoms mixed 36, 32, 30 and FP64
-// 101, 66, 50; 32,000 atoms mixed 41, 40, 43 and FP64 172, 160, 166; 131,072 atoms mixed
-// 66, 70, 84 and FP64 537, 554, 565; 1,048,576 atoms mixed 299, 328, 449 and FP64 3935,
-// 4060, 4256.  8 lanes gain under 2% on the smallest systems.
-int default_tpa(int nslot) { return nslot >= 49152 ? 1 : nslot >= 24576 ? 2 : 4; }
+// Four lanes up to 8 atoms for each of the 16 warps that an SM keeps in the step kernel
+// (19,456 slots on 152 SMs): step of 16,384 atoms mixed with 4 and 2 lanes 27.7 and 26.9 us,
+// of 19,652 34.0 and 31.8, of 23,328 34.3 and 32.6, in FP64 of 19,652 85.4 and 83.8.  Two up
+// to 49,152 slots: 42,592 atoms mixed with 2 and 1 lanes 36.6 and 41.9, 55,296 44.7 and 44.9,
+// 62,500 47.8 and 45.0; in FP64 55,296 187 and 164.  8 lanes gain under 2% on the smallest.
+int default_tpa(int nslot) { return nslot >= 49152 ? 1 : nslot > 19456 ? 2 : 4; }
 
 // Lay the replicas out (32-aligned slot ranges, consecutive cell ranges with one
 // padding cell each), allocate every per-slot array and upload the atoms.

@@ -37,6 +37,12 @@ constexpr int CHUNK_WARPS = CHUNK_THREADS / 32;
 // warps in flight)
 constexpr int BY_ATOM = 6144;
 constexpr int FP64_ATOMS = 12288;
+// With more than a few replicas one rebuilds in nearly every step, and the kernels' rebuild,
+// with more blocks than stay resident, takes less time: step of 4 replicas (4,900 slots) mixed
+// 36.6 us here and 39.1 with kernels, FP64 67.2 and 69.4; of 8 (10,400) mixed 48.9 and 51.4,
+// FP64 99.5 and 92.1; of 16 (5,200) mixed 73.9 and 66.6, FP64 120 and 101; of 36 (11,800)
+// mixed 77.0 and 71.2.
+constexpr int MAX_REPLICAS = 6;
 // polls of a barrier before a block gives up (seconds): the launch is cooperative, so a block
 // that never comes means a fault elsewhere; the host then reads F_STALL
 constexpr unsigned BARRIER_POLLS = 1u << 21;
@@ -440,6 +446,7 @@ int pick(const ChunkArgs &A, int kick, bool one, int want, cudaStream_t st) {
 // Sizes for which the kernels' blocks hold one task per warp (the partial sums are then
 // those of the virtual blocks), at the lane counts small systems use.
 bool chunk_fits(const Box &b, const LaunchCfg &lc) {
+  if (b.nrep > MAX_REPLICAS) return false;
   if (lc.use_seg || lc.block != CHUNK_THREADS || (lc.tpa != 2 && lc.tpa != 4)) return false;
   if (lc.precision == CAVGPU_FP64 && (!lc.exchange || lc.tpa != 4 || lc.n > FP64_ATOMS)) return false;
   const int ntask = (lc.n + 32 / lc.tpa - 1) / (32 / lc.tpa);

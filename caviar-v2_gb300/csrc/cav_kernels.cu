@@ -200,10 +200,14 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 4) k_build_group(Dev d, Box 
 
 // few windows: a block of four warps each (BuildShare)
 constexpr int SHARED_WINDOWS = 8;  // per SM
+// blocks per window of a batch: its replicas' rows of cells are short and a window meets one
+// to three of them, each a group with a chain of its own (step of 56 replicas: 92 us with 1, 89
+// with 2, 92 with 3; of 24 in FP64 182, 177, 177)
+constexpr int BATCH_SPLIT = 2;
 template <int MODE>
-__global__ void __launch_bounds__(128) k_build_shared(Dev d, Box b, int forced) {
+__global__ void __launch_bounds__(128) k_build_shared(Dev d, Box b, int forced, int split) {
   __shared__ BuildShare share;
-  rebuild_build<MODE, true>(d, b, forced, share.stage[threadIdx.x >> 5], blockIdx.x, gridDim.x, &share);
+  rebuild_build<MODE, true>(d, b, forced, share.stage[threadIdx.x >> 5], blockIdx.x, gridDim.x, &share, split);
 }
 
 // after the build: count the rebuilt replicas, clear their flags and the global one;
@@ -694,12 +698,18 @@ int launch_rebuild(const Dev &d, const Box &b, const LaunchCfg &lc, int forced, 
   k_scatter<<<g, 256, 0, st>>>(d, b, forced);
   k_sort_gather<<<ceil_div((long long)b.ncell_all * 32, 256), 256, 0, st>>>(d, b, forced);
   const int windows = ceil_div(b.nslot, 32), build_grid = std::min(ceil_div(windows, BUILD_WARPS), num_sms() * 32);
+  const bool batch = b.nrep > 1;
+  const int split = batch ? BATCH_SPLIT : 1;
   // one window per warp up to 1.2 M slots: with 8 blocks per SM a warp had 3 or 4 of them at
-  // 1,048,576 atoms and the build 30 us of tail; up to SHARED_WINDOWS windows per SM (38,912 atoms) a window's own chain of work is the
-  // time: 33 us with its four warps, 46 us with one, at 32,000 atoms
-  if (windows <= num_sms() * SHARED_WINDOWS) {
-    if (lc.precision == CAVGPU_MIXED) k_build_shared<1><<<windows, 128, 0, st>>>(d, b, forced);
-    else k_build_shared<0><<<windows, 128, 0, st>>>(d, b, forced);
+  // 1,048,576 atoms and the build 30 us of tail; up to SHARED_WINDOWS windows per SM (38,912
+  // atoms) a window's own chain of work is the time: 33 us with its four warps, 46 us with one,
+  // at 32,000 atoms.  Of a batch some replicas rebuild in a step, about a sixth when each does
+  // so every sixth, so the line lies further up: a step of 56 replicas (1,900 windows) takes 89
+  // us with four warps per window and 138 with one, of 128 (4,900) 137 and 178, but of 256
+  // large ones (34,900) 511 and 426.
+  if (windows <= num_sms() * SHARED_WINDOWS * (batch && !forced ? 8 : 1)) {
+    if (lc.precision == CAVGPU_MIXED) k_build_shared<1><<<windows * split, 128, 0, st>>>(d, b, forced, split);
+    else k_build_shared<0><<<windows * split, 128, 0, st>>>(d, b, forced, split);
   } else if (lc.precision == CAVGPU_MIXED) k_build_group<1><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
   else k_build_group<0><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
   if (lc.exchange) {

@@ -243,7 +243,10 @@ __device__ __forceinline__ int class_cell(int x0, int nu, int k) {
 // mask per lane (one warp vote per 32 candidates for the rare exact FP64 test), and
 // only then are the hits (~15% of the staged candidates) written, in candidate order.
 constexpr int BUILD_STAGE = 256;  // staged candidates per warp and pass (4 KiB + 256 B)
-constexpr int SEG_HITS = 40;      // hits per lane that a part of a shared window holds
+// hits per lane that a part of a shared window holds: up to ~0.42 of an atom's, ~46 of 110 at
+// density 1.2 (40: one warp did most dense windows again, a step of 24 replicas 101 us against
+// 82; 64: a block fewer per SM)
+constexpr int SEG_HITS = 56;
 constexpr int GROUP_SPAN = 5;     // a group spans at most 6 cells: x index + 8 row < 256
 
 // q_u, q_u+1 = |c - r|^2 of two candidates with packed FP32x2 arithmetic (sm_100+):
@@ -394,10 +397,11 @@ struct BuildShare {
 __constant__ const int8_t PART_ROWS[5] = {0, 2, 5, 7, 9};  // of ROW_ORDER
 
 // SHARED false: warp gw of nw takes the windows gw, gw + nw, ...; true: block gw of nw, the
-// warps of a block (four) the parts of its windows.
+// warps of a block (four) the parts of its windows.  split > 1: the groups of a window are
+// dealt to that many warps or blocks.
 template <int MODE, bool SHARED>
 __device__ __forceinline__ void rebuild_build(const Dev &d, const Box &b, int forced, BuildStage &stage, int gw, int nw,
-                                              BuildShare *share) {
+                                              BuildShare *share, int split = 1) {
   const int part = SHARED ? threadIdx.x >> 5 : 0;
   const int lane = threadIdx.x & 31;
   float4 *sxy = stage.xy;
@@ -410,7 +414,9 @@ __device__ __forceinline__ void rebuild_build(const Dev &d, const Box &b, int fo
   const unsigned lt_mask = (1u << lane) - 1u;
   const int nwin = (b.nslot + 31) >> 5;
   int wmax = 0;
-  for (int win = gw; win < nwin; win += nw) {
+  for (int task = gw; task < nwin * split; task += nw) {
+    const int win = task / split, mine = task - win * split;
+    int group = 0;
     BuildLane L;
     L.i = (win << 5) + lane;
     const int rep = L.i < b.nslot ? rep_of_slot(b, L.i) : -1;
@@ -441,6 +447,7 @@ __device__ __forceinline__ void rebuild_build(const Dev &d, const Box &b, int fo
       const int grep = __shfl_sync(FULL_MASK, rep, leader);
       const unsigned mem = __ballot_sync(FULL_MASK, ((pending >> lane) & 1u) && rowkey == rk && L.cx - cx0 <= GROUP_SPAN);
       pending &= ~mem;
+      if (group++ % split != mine) continue;
       L.me = (mem >> lane) & 1u;
       const RepBox &rb = repbox(b, grep);
       const int span = __reduce_max_sync(FULL_MASK, L.me ? L.cx - cx0 : 0);
