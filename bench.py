@@ -591,22 +591,23 @@ def main():
                                            tpa=rm["tpa"], block=rm["block"], steps_per_graph=spg, force_kernel=kern)
 
     # roofline of the dominant kernel (mixed force kernel): algorithmic bytes per launch
-    #   per atom: 4 * nbar list words + rel_i 16 + nnbr 4 + vel r/w 64 + acc r 32 (a_old) + acc w 32,
-    #   and on the launches that also drift the next step: pos r/w 64 + pos_ref 32 + rel_ref 16
-    #   + the next rel 16 = 128 more
+    #   per atom: 4 * nbar list words + coordinates 16 + nnbr 4 + vel r/w 64 + acc r 32 (a_old) + acc w 32,
+    #   and on the launches that also drift the next step: pos r/w 64 + the coordinates at the
+    #   last build 16 + the next ones 16 = 96 more
     peaks = measured_peaks()
     hbm = peaks.get("hbm_gbs")
     peak_note = "measured" if hbm else "fallback"
     hbm = hbm or 6800.0
     fused = fused_fraction(args.steps, rm["autotune"])
-    bytes_per_atom = 4.0 * rm["nbar"] + 148.0 + 128.0 * fused
+    bytes_per_atom = 4.0 * rm["nbar"] + 148.0 + 96.0 * fused
     launch_ms = rm["force_ms"] / max(rm["force_launches"], 1)
     achieved = bytes_per_atom * n / (launch_ms * 1e-3) / 1e9
     traffic = read_profile_traffic("lj_force_mixed_1M.md")
-    # FP64 form: FP64-pipe roofline, FLOPs per atom = 8 n_list + 17 n_cut (n_cut = n_list (rc/ce)^3)
+    # FP64 form: FP64-pipe roofline; every pair inside the cutoff once (n_cut = n_list (rc/ce)^3
+    # per atom, both orders): 8 FLOPs for the distance, 11 for the coefficient, 12 to add it to both
     fp64_peak, fp32_peak = cavgpu.measure_peaks()
     ncut = r64["nbar"] * (2.5 / 2.8) ** 3
-    flops_atom = 8 * r64["nbar"] + 17 * ncut
+    flops_atom = 31 * 0.5 * ncut
     l64 = r64["force_ms"] / max(r64["force_launches"], 1)
     fp64_achieved = flops_atom * n / (l64 * 1e-3) / 1e12
 
@@ -636,7 +637,7 @@ def main():
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": traffic, "kernel": "k_force<mixed>", "peak_source": peak_note,
                      "bytes_per_atom": bytes_per_atom, "launch_ms": launch_ms, "fused_launch_share": fused},
-        "fp64": {"value": value64, "ms_per_step": ms_fp64 / k64, "kernel": "k_force<fp64>",
+        "fp64": {"value": value64, "ms_per_step": ms_fp64 / k64, "kernel": "k_pairs64 + k_close64",
                  "roofline": {"bound": "fp64", "achieved": fp64_achieved, "peak": fp64_peak, "unit": "TFLOP/s",
                               "frac": fp64_achieved / fp64_peak, "flops_per_atom": flops_atom, "launch_ms": l64,
                               "peak_source": "measured by cavgpu_measure_peaks (DFMA chains)"},

@@ -76,7 +76,7 @@ typedef struct cavgpu_params {
   int32_t precision;              /* CAVGPU_FP64 or CAVGPU_MIXED */
   int32_t noise_off;              /* Langevin with eta = 0 (exactness checks) */
   int32_t nbr_capacity;           /* neighbour slots per atom; 0 = sized at set-up */
-  int32_t threads_per_atom;       /* force kernel lanes per atom (1,2,4,8,16); 0 = default */
+  int32_t threads_per_atom;       /* force kernel lanes per atom (1,2,4,8,16); 0 = by system size */
   int32_t block_size;             /* force kernel block size (32..256, multiple of 32); 0 = default */
   int32_t steps_per_graph;        /* steps captured per CUDA graph; 0 = default (50); < 0 = no
                                      graphs, every kernel launched from the host (for profilers,
