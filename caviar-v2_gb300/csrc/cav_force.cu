@@ -97,7 +97,8 @@ __device__ __forceinline__ void fp64_pairs(const Dev &d, const uint4 *row4, int 
                       : P[0][q];
 }
 
-// Grid-strided pair kernel (the FP64 form; the mixed form when it has no segments):
+// Grid-strided pair kernel over the full list (the mixed form when it has no segments; the FP64
+// form with 8 or 16 lanes or without room for the pair exchange):
 // warp-sized tasks of A consecutive slots, neighbour coordinates gathered from
 // global memory.
 template <int TPA, bool MIXED, int KICK, bool EV, bool ONE>
