@@ -984,9 +984,12 @@ int complete_overflowed_step(cavgpu_ctx *c, const ChunkPlan &pl, int k, int64_t 
   const bool th = (every > 0 && (g + 1) % every == 0) || (every == 0 && g == nsteps - 1);
   const int ring_slot = (th && every > 0) ? 0 : -1;
   long long nl = 0;
-  RK(launch_force(c->d, c->b, c->sc, c->lc, is_lang(c) ? 2 : 1, th, 0, FUSE_NONE, 0, 0, c->st));
+  // folded as the steps of a chunk fold it (a fold kernel's other order changes last bits)
+  const bool fold = th && c->b.nrep == 1 && c->nve.step == 0;
+  const FoldArgs fa = fold_args(c, ring_slot);
+  RK(launch_force(c->d, c->b, c->sc, c->lc, is_lang(c) ? 2 : 1, th, 0, FUSE_NONE, 0, 0, c->st, fold ? &fa : nullptr));
   nl += force_kernels(c->lc);
-  if (th) RK(enqueue_thermo_after_force(c, ring_slot, &nl));
+  if (th && !fold) RK(enqueue_thermo_after_force(c, ring_slot, &nl));
   if (c->nve.step > 0 && !is_lang(c)) {
     RK(launch_nve(c->d, c->b, c->tc, c->nve, 0, th, ring_slot, c->st));
     nl += 3;
