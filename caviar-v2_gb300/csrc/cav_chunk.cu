@@ -336,6 +336,11 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 4) k_chunk(const __grid_constan
     if (need) {
       if (!rebuild<MIXED>(A, d.ic, sh)) return;
       if (flags[F_OVERFLOW]) {
+        // the host completes the step and folds its record from the first set of sums: a
+        // Langevin step's temperature sums, of its drift above, go there (block 0 has folded
+        // the record before, if that was in it)
+        if (KICK == 2 && alt && blockIdx.x == 0)
+          for (int i = threadIdx.x; i < 4 * ((sc.n + 255) / 256); i += CHUNK_THREADS) d.partials_ke[i] = v.partials_ke[i];
         halt = true;
         break;
       }
