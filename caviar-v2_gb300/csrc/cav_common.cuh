@@ -159,6 +159,7 @@ struct StepConsts {
 struct Dev {
   // acc holds a(t) from the pair kernel until the next pair kernel replaces it, so
   // the velocity-Verlet kick reads it as a_old (leap-frog's drift zeroes it)
+  // (vel.w: 0, or 1 for an atom of the mixed form whose position is not a number)
   dbl4 *pos, *vel, *acc, *pos_ref;
   float4 *rel;                // position at the last build relative to the build cell's origin; w = type bits
   int4 *ic;                   // fixed-point coordinates (to_fixed), w = type: the mixed form's, the FP64 screen's
@@ -390,15 +391,24 @@ __device__ inline void request_rebuild(const Dev &d, const Box &b, int rep) {
 __device__ __forceinline__ double to_fixed(double x, double lo, double s) {
   return fma(x - lo, s, 6755399441055744.0);  // 1.5 * 2^52
 }
-__device__ __forceinline__ int4 fixed_pos(const RepBox &rb, const dbl4 &x, int type, int3 &window) {
+// `high`: the sums' upper words.  1.5 * 2^52 is 0x43380000 there, and a window counts one.
+__device__ __forceinline__ int4 fixed_pos(const RepBox &rb, const dbl4 &x, int type, int3 &high) {
   const double tx = to_fixed(x.x, rb.lo[0], rb.fx_s[0]), ty = to_fixed(x.y, rb.lo[1], rb.fx_s[1]),
                tz = to_fixed(x.z, rb.lo[2], rb.fx_s[2]);
-  window = make_int3(__double2hiint(tx) & 1023, __double2hiint(ty) & 1023, __double2hiint(tz) & 1023);
+  high = make_int3(__double2hiint(tx), __double2hiint(ty), __double2hiint(tz));
   return make_int4(__double2loint(tx), __double2loint(ty), __double2loint(tz), type);
 }
+// Whether ten bits tell the window of a coordinate: windows -256 .. 767.  Not so for one that
+// is further off, is infinite or is not a number (and in the far part of a box of more windows).
+__device__ __forceinline__ bool window_known(const int3 &high) {
+  auto known = [](int h) { return (unsigned)(h - 0x43380000 + 256) < 1024u; };
+  return known(high.x) && known(high.y) && known(high.z);
+}
 // the same as a reference of later displacements: w holds ten bits of each window index
-__device__ __forceinline__ int4 fixed_ref(const int4 &q, const int3 &window) {
-  return make_int4(q.x, q.y, q.z, window.x | (window.y << 10) | (window.z << 20));
+// and above them whether they do not tell the windows
+__device__ __forceinline__ int4 fixed_ref(const int4 &q, const int3 &high) {
+  return make_int4(q.x, q.y, q.z, (high.x & 1023) | ((high.y & 1023) << 10) | ((high.z & 1023) << 20) |
+                                      (window_known(high) ? 0 : 1 << 30));
 }
 // b - a modulo 2^32, as a signed displacement
 __device__ __forceinline__ int fixed_diff(int b, int a) { return (int)((unsigned)b - (unsigned)a); }
@@ -425,17 +435,29 @@ __device__ inline void half_skin_test(const Dev &d, const Box &b, int rep, int i
 // Mixed form: the new fixed-point coordinates, written to `out`, and the half-skin
 // test on their difference to those of the last build (in FP32 against a threshold
 // shrunk by the units' rounding and 1e-6, so it can only fire early; the window
-// indices tell a displacement that wrapped, as in a system that flies apart).
+// indices tell a displacement that wrapped, as in a system that flies apart).  Where the
+// windows are not known the positions themselves are compared; one that is not a number
+// marks its atom (vel.w), whose next acceleration is then NaN (finish_atom).
+__device__ __forceinline__ void track_far(const Dev &d, const Box &b, int rep, int i, const dbl4 &x) {
+  const dbl4 r = d.pos_ref[i];
+  const double dx = x.x - r.x, dy = x.y - r.y, dz = x.z - r.z, d2 = dx * dx + dy * dy + dz * dz;
+  if (!(d2 <= (double)b.thr2f)) request_rebuild(d, b, rep);
+  if (isnan(x.x) || isnan(x.y) || isnan(x.z)) d.vel[i].w = 1.0;
+}
 __device__ inline void mixed_track(const Dev &d, const Box &b, int rep, int i, const dbl4 &x, int4 *out) {
   const RepBox &rb = repbox(b, rep);
   int3 w;
   const int4 q = fixed_pos(rb, x, type_of(x.w), w), r = d.ic_ref[i];
+  out[i] = q;
+  if ((r.w >> 30) != 0 || !window_known(w)) {
+    track_far(d, b, rep, i, x);
+    return;
+  }
   const float fx = (float)fixed_diff(q.x, r.x) * rb.uh[0], fy = (float)fixed_diff(q.y, r.y) * rb.uh[1],
               fz = (float)fixed_diff(q.z, r.z) * rb.uh[2];
   if (fx * fx + fy * fy + fz * fz > b.thr2f || beyond_window(q.x, w.x, r.x, r.w & 1023) ||
       beyond_window(q.y, w.y, r.y, (r.w >> 10) & 1023) || beyond_window(q.z, w.z, r.z, (r.w >> 20) & 1023))
     request_rebuild(d, b, rep);
-  out[i] = q;
 }
 
 __device__ inline void nan_check(const Dev &d, int i, const dbl4 &a) {

@@ -135,6 +135,10 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
   const double mi = tab.minv[ti];
   dbl4 an = make_dbl4(fx * mi, fy * mi, fz * mi, 0.0);
   dbl4 v;
+  // (mixed form: the integers of a position that is not a number give a finite force)
+  auto poison = [&]() {
+    if (MIXED && __double2hiint(v.w) != 0) an.x = an.y = an.z = __longlong_as_double(0x7ff8000000000000ll);
+  };
   if (KICK == 0) {
     d.acc[i] = an;
     if (EV) {
@@ -145,6 +149,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
   } else if (KICK == 1) {
     v = d.vel[i];
+    poison();
     const dbl4 ao = d.acc[i];  // a(t), still in place until the store below
     if (MIXED) {
       v.x = fma(an.x + ao.x, sc.hdt, v.x);
@@ -162,6 +167,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
   } else {
     v = d.vel[i];
+    poison();
     double e0 = 0.0, e1 = 0.0, e2 = 0.0;
     if (!sc.noise_off) {  // replica r draws the noise stream of seed + r with its local ids
       if (MIXED) langevin_eta_f(sc.seed + rep, step, d.id[i], e0, e1, e2);
