@@ -514,8 +514,9 @@ int build_and_force(cavgpu_ctx *c, const Status **out) {
   return CAVGPU_E_NLIST_OVERFLOW;
 }
 
-// box and search grid of one replica; L >= 2 cutoff_extra (one image per pair)
-int make_repbox(double ce, const double lo[3], const double hi[3], RepBox *rb) {
+// box and search grid of one replica; L >= 2 cutoff_extra (one image per pair); rc: the
+// largest force cutoff
+int make_repbox(double ce, double skin, double rc, const double lo[3], const double hi[3], RepBox *rb) {
   for (int a = 0; a < 3; ++a) {
     rb->lo[a] = lo[a];
     rb->hi[a] = hi[a];
@@ -529,8 +530,12 @@ int make_repbox(double ce, const double lo[3], const double hi[3], RepBox *rb) {
     rb->wf[a] = (float)rb->w[a];
     // fixed-point coordinates (to_fixed): m windows of at least 4 cutoff_extra
     const int m = (int)std::min(std::max(std::floor(rb->L[a] / (4.0 * ce)), 1.0), 131072.0);
-    const double unit = rb->L[a] / m / 4294967296.0;
-    rb->fx_s[a] = 4294967296.0 * m / rb->L[a];
+    // a listed pair drifts to cutoff_extra + skin apart at most; where its other image could
+    // then be inside a force cutoff the window is two boxes (RepBox::flip)
+    const bool two = m == 1 && rc > (rb->L[a] - ce - skin) * (1.0 + 1e-9);
+    rb->flip[a] = two ? 0x80000000u : 0u;
+    const double unit = (two ? 2.0 : 1.0) * rb->L[a] / m / 4294967296.0;
+    rb->fx_s[a] = 1.0 / unit;
     rb->uh[a] = (float)unit;
     rb->ul[a] = (float)(unit - (double)rb->uh[a]);
   }
@@ -557,8 +562,13 @@ int create_common(const cavgpu_params *p, int nrep, const double *lo3, const dou
   const double ce = p->nl_cutoff * p->nl_coef;  // Neighborlist::init (src/neighborlist.cpp:317)
   c->cutoff_extra = ce;
   c->reps.resize(nrep);
-  for (int r = 0; r < nrep; ++r)
-    if (make_repbox(ce, lo3 + 3 * r, hi3 + 3 * r, &c->reps[r])) { delete c; return CAVGPU_E_ARG; }
+  double rc_max = 0.0;  // (the FP64 form only screens by these coordinates: the nearest image is right)
+  for (int k = 0; k < p->ntypes * p->ntypes; ++k)
+    if (p->precision == CAVGPU_MIXED && p->eps[k] != 0.0) rc_max = std::max(rc_max, p->cutoff_list_on ? p->cutoff_list[k] : p->lj_cutoff);
+  for (int r = 0; r < nrep; ++r) {
+    if (make_repbox(ce, ce - p->nl_cutoff, rc_max, lo3 + 3 * r, hi3 + 3 * r, &c->reps[r])) { delete c; return CAVGPU_E_ARG; }
+    for (int a = 0; a < 3; ++a) c->lc.images |= c->reps[r].flip[a] != 0;
+  }
   // reference binning of a single system: Domain::calculate_local_domain with grid
   // index 0 of 1 (src/domain.cpp:320-326), no_bins = ceil(size * 1/cutoff_extra)
   c->cutoff_inv = 1.0 / ce;
@@ -1337,7 +1347,7 @@ int cavgpu_autotune(cavgpu_ctx *c, int32_t trial_steps, int32_t flags, int64_t *
     // kernels: the mixed form tries the segment and the grid-strided kernel unless the
     // caller fixed one
     int kernels[2] = {c->lc.use_seg, -1};
-    if (c->p.precision == CAVGPU_MIXED && c->p.force_kernel == CAVGPU_FORCE_AUTO) kernels[0] = 1, kernels[1] = 0;
+    if (stencil_codes(c->lc) && c->p.force_kernel == CAVGPU_FORCE_AUTO) kernels[0] = 1, kernels[1] = 0;
     for (int seg : kernels) {
       if (seg < 0) break;
       for (int tpa : tpas)
@@ -1474,7 +1484,7 @@ int64_t cavgpu_export_pairs(cavgpu_ctx *c, int32_t *out5, int64_t cap) {
   if (cudaMalloc(&rows, (size_t)take * 5 * sizeof(int32_t)) != cudaSuccess) { cudaGetLastError(); return CAVGPU_E_NOMEM; }
   if (cudaMalloc(&cnt, sizeof(unsigned long long)) != cudaSuccess) { cudaFree(rows); cudaGetLastError(); return CAVGPU_E_NOMEM; }
   int rc = cuda_rc(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), c->st));
-  if (!rc) rc = launch_export_pairs(c->d, c->b, c->p.precision == CAVGPU_MIXED ? 1 : 0, rows, cnt, take, c->st);
+  if (!rc) rc = launch_export_pairs(c->d, c->b, stencil_codes(c->lc) ? 1 : 0, rows, cnt, take, c->st);
   if (!rc) rc = cuda_rc(cudaMemcpyAsync(out5, rows, (size_t)take * 5 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->st));
   if (!rc) rc = cuda_rc(cudaStreamSynchronize(c->st));
   cudaFree(rows);

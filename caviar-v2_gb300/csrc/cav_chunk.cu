@@ -452,6 +452,7 @@ int pick(const ChunkArgs &A, int kick, bool one, int want, cudaStream_t st) {
 // those of the virtual blocks), at the lane counts small systems use.
 bool chunk_fits(const Box &b, const LaunchCfg &lc) {
   if (b.nrep > MAX_REPLICAS) return false;
+  if (lc.images) return false;  // (k_force alone applies image codes to fixed-point coordinates)
   if (lc.use_seg || lc.block != CHUNK_THREADS || (lc.tpa != 2 && lc.tpa != 4)) return false;
   if (lc.precision == CAVGPU_FP64 && (!lc.exchange || lc.tpa != 4 || lc.n > FP64_ATOMS)) return false;
   const int ntask = (lc.n + 32 / lc.tpa - 1) / (32 / lc.tpa);

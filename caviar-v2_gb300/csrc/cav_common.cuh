@@ -121,6 +121,7 @@ struct RepBox {
   // FP32 pair uh + ul
   double fx_s[3];
   float uh[3], ul[3];
+  uint32_t flip[3];       // 2^31 where the coordinate's window is two boxes (lc.images), else 0
   int nc[3];
   int cell_off, ncell;    // cells [cell_off, cell_off + ncell); cell cell_off + ncell holds the padding
   int slot_off, natoms, pad;
@@ -383,7 +384,11 @@ __device__ inline void request_rebuild(const Dev &d, const Box &b, int rep) {
 // displacement to the nearest image, with no cell offset or image shift to decode,
 // for every pair the list holds (a listed image never drifts beyond cutoff_extra +
 // skin <= L - lj cutoff before the half-skin test rebuilds the list, so a difference
-// that wraps to the other image is beyond the cutoff, as that image is).  The unit
+// that wraps to the other image is beyond the cutoff, as that image is).  Not so with a
+// force cutoff above L - cutoff_extra - skin (a force cutoff beyond the neighbour cutoff in a
+// box hardly wider than two list cutoffs): there the window is two boxes long, the list
+// holds image codes, and an image shift, half a window either way, flips the top bit of a
+// neighbour's coordinate (RepBox::flip, lc.images).  The unit
 // is below 8 cutoff_extra / 2^32 (5e-9 sigma at 2.8), 25 times finer than the
 // rounding of an FP32 coordinate inside a cell, and differences are exact before
 // their one conversion to FP32.  One FMA per axis: adding 1.5 * 2^52 leaves the
@@ -482,7 +487,12 @@ struct LaunchCfg {
   int use_seg;     // mixed form: run the segment kernel (shared-memory stage)
   int ntypes;      // 1: the kernels keep the pair constants in registers
   int exchange;    // FP64 form: pairs evaluated once, two kernels per force (cav_exchange.cu)
+  int images;      // mixed form: the list holds image codes, applied by the pair kernel (RepBox::flip)
 };
+// the list words of the mixed form hold stencil indices, else image codes
+inline bool stencil_codes(const LaunchCfg &lc) { return lc.precision == CAVGPU_MIXED && !lc.images; }
+// the segment kernel runs (its table lookups need stencil indices)
+inline bool segments_on(const LaunchCfg &lc) { return stencil_codes(lc) && lc.use_seg && lc.nseg > 0; }
 
 struct ThermoCfg {
   int n_r_df;

@@ -21,12 +21,22 @@ struct WarpImages;
 template <>
 struct WarpImages<true> {
   float4 hi, lo;  // length of a coordinate unit per axis, as an FP32 pair hi + lo
+  uint3 flip;     // IMG: what an image shift does to a coordinate
 };
 
 template <>
 struct WarpImages<false> {
   double3 v[27];
 };
+
+// the coordinates of the image that a list word names (lists of image codes)
+__device__ __forceinline__ int4 image_of(int4 q, uint32_t word, const uint3 &flip) {
+  const int code = (int)(word >> CODE_SHIFT), sz = code / 9, sy = code / 3 - 3 * sz, sx = code % 3;
+  if (sx != 1) q.x ^= (int)flip.x;
+  if (sy != 1) q.y ^= (int)flip.y;
+  if (sz != 1) q.z ^= (int)flip.z;
+  return q;
+}
 
 // FP64 pair loop of one lane (the entries RowSplit gives it).  ONE: single type, the pair
 // constants in registers, no table lookups; t1 = the atom's first table entry.  The
@@ -100,8 +110,8 @@ __device__ __forceinline__ void fp64_pairs(const Dev &d, const uint4 *row4, int 
 // Grid-strided pair kernel over the full list (the mixed form when it has no segments; the FP64
 // form with 8 or 16 lanes or without room for the pair exchange):
 // warp-sized tasks of A consecutive slots, neighbour coordinates gathered from
-// global memory.
-template <int TPA, bool MIXED, int KICK, bool EV, bool ONE>
+// global memory.  IMG: the mixed form with image codes in the list.
+template <int TPA, bool MIXED, int KICK, bool EV, bool ONE, bool IMG>
 __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, StepConsts sc, ForceArgs fa) {
   constexpr int A = 32 / TPA;
   __shared__ typename std::conditional<MIXED, SmemTabF, SmemTabD>::type tab;
@@ -138,6 +148,7 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
         if (lane == 0) {
           wimg[wid].hi = make_float4(rb.uh[0], rb.uh[1], rb.uh[2], 0.f);
           wimg[wid].lo = make_float4(rb.ul[0], rb.ul[1], rb.ul[2], 0.f);
+          if (IMG) wimg[wid].flip = make_uint3(rb.flip[0], rb.flip[1], rb.flip[2]);
         }
       } else if (lane < 27) {
         const int sx = lane % 3 - 1, sy = (lane / 3) % 3 - 1, sz = lane / 9 - 1;
@@ -159,8 +170,13 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
         ti = ri.w;
         float ax = 0.f, ay = 0.f, az = 0.f, vr = 0.f, pp = 0.f;
         const int4 *ic = d.ic;
+        const uint3 flip = IMG ? wimg[wid].flip : make_uint3(0u, 0u, 0u);
         mixed_pairs<TPA, EV, ONE, false>(row4 + t * A, nn, t, ri, nt, tab, one_type(tab), wimg[wid].hi, wimg[wid].lo, sc.jump_tolf,
-                                  [ic](uint32_t w) { return __ldg(&ic[w & IDX_MASK]); }, ax, ay, az, vr, pp);
+                                  [ic, flip](uint32_t w) {
+                                    const int4 q = __ldg(&ic[w & IDX_MASK]);
+                                    return IMG ? image_of(q, w, flip) : q;
+                                  },
+                                  ax, ay, az, vr, pp);
         fx = ax; fy = ay; fz = az; vir = vr; pe = pp;
       } else {
         const dbl4 xi = d.pos[i];
@@ -341,35 +357,40 @@ __global__ void __launch_bounds__(256) k_force_seg(Dev d, Box b, StepConsts sc, 
 }
 
 template <int TPA, bool MIXED, int KICK>
-static void launch_ev(bool ev, bool one, int grid, int block, const Dev &d, const Box &b, const StepConsts &sc,
-                      const ForceArgs &fa, cudaStream_t st) {
+static void launch_ev(bool ev, bool one, bool img, int grid, int block, const Dev &d, const Box &b,
+                      const StepConsts &sc, const ForceArgs &fa, cudaStream_t st) {
   const size_t ev_smem = (size_t)6 * block * sizeof(double);
-  if (one) {  // single-type systems: pair constants in registers
-    if (ev) k_force<TPA, MIXED, KICK, true, true><<<grid, block, ev_smem, st>>>(d, b, sc, fa);
-    else k_force<TPA, MIXED, KICK, false, true><<<grid, block, 0, st>>>(d, b, sc, fa);
+  if (img) {  // (rare: whatever the types)
+    if (ev) k_force<TPA, MIXED, KICK, true, false, MIXED><<<grid, block, ev_smem, st>>>(d, b, sc, fa);
+    else k_force<TPA, MIXED, KICK, false, false, MIXED><<<grid, block, 0, st>>>(d, b, sc, fa);
     return;
   }
-  if (ev) k_force<TPA, MIXED, KICK, true, false><<<grid, block, ev_smem, st>>>(d, b, sc, fa);
-  else k_force<TPA, MIXED, KICK, false, false><<<grid, block, 0, st>>>(d, b, sc, fa);
+  if (one) {  // single-type systems: pair constants in registers
+    if (ev) k_force<TPA, MIXED, KICK, true, true, false><<<grid, block, ev_smem, st>>>(d, b, sc, fa);
+    else k_force<TPA, MIXED, KICK, false, true, false><<<grid, block, 0, st>>>(d, b, sc, fa);
+    return;
+  }
+  if (ev) k_force<TPA, MIXED, KICK, true, false, false><<<grid, block, ev_smem, st>>>(d, b, sc, fa);
+  else k_force<TPA, MIXED, KICK, false, false, false><<<grid, block, 0, st>>>(d, b, sc, fa);
 }
 
 template <int TPA, bool MIXED>
-static void launch_kick(int kick, bool ev, bool one, int grid, int block, const Dev &d, const Box &b,
+static void launch_kick(int kick, bool ev, bool one, bool img, int grid, int block, const Dev &d, const Box &b,
                         const StepConsts &sc, const ForceArgs &fa, cudaStream_t st) {
-  if (kick == 0) launch_ev<TPA, MIXED, 0>(ev, one, grid, block, d, b, sc, fa, st);
-  else if (kick == 1) launch_ev<TPA, MIXED, 1>(ev, one, grid, block, d, b, sc, fa, st);
-  else launch_ev<TPA, MIXED, 2>(ev, one, grid, block, d, b, sc, fa, st);
+  if (kick == 0) launch_ev<TPA, MIXED, 0>(ev, one, img, grid, block, d, b, sc, fa, st);
+  else if (kick == 1) launch_ev<TPA, MIXED, 1>(ev, one, img, grid, block, d, b, sc, fa, st);
+  else launch_ev<TPA, MIXED, 2>(ev, one, img, grid, block, d, b, sc, fa, st);
 }
 
 template <bool MIXED>
-static int launch_tpa(int tpa, int kick, bool ev, bool one, int grid, int block, const Dev &d, const Box &b,
+static int launch_tpa(int tpa, int kick, bool ev, bool one, bool img, int grid, int block, const Dev &d, const Box &b,
                       const StepConsts &sc, const ForceArgs &fa, cudaStream_t st) {
   switch (tpa) {
-    case 1: launch_kick<1, MIXED>(kick, ev, one, grid, block, d, b, sc, fa, st); break;
-    case 2: launch_kick<2, MIXED>(kick, ev, one, grid, block, d, b, sc, fa, st); break;
-    case 4: launch_kick<4, MIXED>(kick, ev, one, grid, block, d, b, sc, fa, st); break;
-    case 8: launch_kick<8, MIXED>(kick, ev, one, grid, block, d, b, sc, fa, st); break;
-    case 16: launch_kick<16, MIXED>(kick, ev, one, grid, block, d, b, sc, fa, st); break;
+    case 1: launch_kick<1, MIXED>(kick, ev, one, img, grid, block, d, b, sc, fa, st); break;
+    case 2: launch_kick<2, MIXED>(kick, ev, one, img, grid, block, d, b, sc, fa, st); break;
+    case 4: launch_kick<4, MIXED>(kick, ev, one, img, grid, block, d, b, sc, fa, st); break;
+    case 8: launch_kick<8, MIXED>(kick, ev, one, img, grid, block, d, b, sc, fa, st); break;
+    case 16: launch_kick<16, MIXED>(kick, ev, one, img, grid, block, d, b, sc, fa, st); break;
     default: return CAVGPU_E_ARG;
   }
   return CAVGPU_OK;
@@ -435,7 +456,7 @@ int force_grid_blocks(const LaunchCfg &lc) {
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
     if (g_num_sms <= 0) g_num_sms = 148;
   }
-  if (lc.precision == CAVGPU_MIXED && lc.use_seg && lc.nseg > 0)  // one segment per block at a time
+  if (segments_on(lc))  // one segment per block at a time
     return lc.nseg < g_num_sms * 4 ? lc.nseg : g_num_sms * 4;
   const int A = 32 / lc.tpa, block = lc.exchange ? exchange_close_threads() : lc.block;
   const long long ntask = (lc.n + A - 1) / A;
@@ -469,7 +490,7 @@ int launch_force(const Dev &d, const Box &b, const StepConsts &sc, const LaunchC
   ForceArgs fa{k, fuse, set_cond, cond, fold ? 1 : 0, {}};
   if (fold) fa.fa = *fold;
   int rc;
-  if (lc.precision == CAVGPU_MIXED && lc.use_seg && lc.nseg > 0) {
+  if (segments_on(lc)) {
     if (!d.seg || d.nseg != lc.nseg) return CAVGPU_E_ARG;
     rc = seg_tpa(true, lc.tpa, kick, thermo != 0, lc.ntypes == 1, grid, lc.block,
                  seg_smem_bytes(d.stage_cap, d.seg_umax), d, b, sc, fa, st);
@@ -479,8 +500,8 @@ int launch_force(const Dev &d, const Box &b, const StepConsts &sc, const LaunchC
   } else {
     const bool one = lc.ntypes == 1;
     rc = lc.precision == CAVGPU_MIXED
-             ? launch_tpa<true>(lc.tpa, kick, thermo != 0, one, grid, lc.block, d, b, sc, fa, st)
-             : launch_tpa<false>(lc.tpa, kick, thermo != 0, one, grid, lc.block, d, b, sc, fa, st);
+             ? launch_tpa<true>(lc.tpa, kick, thermo != 0, one, lc.images != 0, grid, lc.block, d, b, sc, fa, st)
+             : launch_tpa<false>(lc.tpa, kick, thermo != 0, one, false, grid, lc.block, d, b, sc, fa, st);
   }
   if (rc) return rc;
   return cudaPeekAtLastError() == cudaSuccess ? CAVGPU_OK : CAVGPU_E_CUDA;

@@ -708,9 +708,9 @@ int launch_rebuild(const Dev &d, const Box &b, const LaunchCfg &lc, int forced, 
   // us with four warps per window and 138 with one, of 128 (4,900) 137 and 178, but of 256
   // large ones (34,900) 511 and 426.
   if (windows <= num_sms() * SHARED_WINDOWS * (batch && !forced ? 8 : 1)) {
-    if (lc.precision == CAVGPU_MIXED) k_build_shared<1><<<windows * split, 128, 0, st>>>(d, b, forced, split);
+    if (stencil_codes(lc)) k_build_shared<1><<<windows * split, 128, 0, st>>>(d, b, forced, split);
     else k_build_shared<0><<<windows * split, 128, 0, st>>>(d, b, forced, split);
-  } else if (lc.precision == CAVGPU_MIXED) k_build_group<1><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
+  } else if (stencil_codes(lc)) k_build_group<1><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
   else k_build_group<0><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);
   if (lc.exchange) {
     const int rc = launch_exchange_build(d, b, forced, st);
