@@ -223,11 +223,11 @@ __device__ __forceinline__ void mixed_task(const Dev &d, const Box &b, const Ste
     const uint4 *row4 = reinterpret_cast<const uint4 *>(d.nbr + (size_t)task * d.cap * A) + (t * A + a);
     const int4 ri = d.ic[i];
     ti = ri.w;
-    float ax = 0.f, ay = 0.f, az = 0.f, vr = 0.f, pp = 0.f;
+    float ax = 0.f, ay = 0.f, az = 0.f;
     const int4 *ic = d.ic;
     mixed_pairs<TPA, EV, ONE, true>(row4, d.nnbr[i], t, ri, nt, tab, one_type(tab), uh, ul, sc.jump_tolf,
-                                    [ic](uint32_t w) { return ic[w & IDX_MASK]; }, ax, ay, az, vr, pp);
-    fx = ax; fy = ay; fz = az; vir = vr; pe = pp;
+                                    [ic](uint32_t w) { return ic[w & IDX_MASK]; }, ax, ay, az, vir, pe);
+    fx = ax; fy = ay; fz = az;
   }
   fold_lanes<A, EV>(fx, fy, fz, vir, pe);
   if (act && t == 0) {

@@ -6,8 +6,8 @@
 // iteration one coalesced 128-byte read of neighbour words.  Two precisions:
 //   FP64  : image = x_j + s*L, all pair arithmetic in double;
 //   MIXED : FP32 pair arithmetic on exact differences of fixed-point coordinates
-//           (int4 x,y,z,type; to_fixed), FP64 accumulation across lanes, FP64
-//           acceleration/velocity/reductions.
+//           (int4 x,y,z,type; to_fixed) and FP32 sums per lane, FP64 accumulation across
+//           lanes, FP64 acceleration/velocity/reductions.
 #include <algorithm>
 
 #include "cav_mixed.cuh"
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
       if constexpr (MIXED) {
         const int4 ri = d.ic[i];
         ti = ri.w;
-        float ax = 0.f, ay = 0.f, az = 0.f, vr = 0.f, pp = 0.f;
+        float ax = 0.f, ay = 0.f, az = 0.f;
         const int4 *ic = d.ic;
         const uint3 flip = IMG ? wimg[wid].flip : make_uint3(0u, 0u, 0u);
         mixed_pairs<TPA, EV, ONE, false>(row4 + t * A, nn, t, ri, nt, tab, one_type(tab), wimg[wid].hi, wimg[wid].lo, sc.jump_tolf,
@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(256, MIXED ? 4 : 1) k_force(Dev d, Box b, Step
                                     const int4 q = __ldg(&ic[w & IDX_MASK]);
                                     return IMG ? image_of(q, w, flip) : q;
                                   },
-                                  ax, ay, az, vr, pp);
-        fx = ax; fy = ay; fz = az; vir = vr; pe = pp;
+                                  ax, ay, az, vir, pe);
+        fx = ax; fy = ay; fz = az;
       } else {
         const dbl4 xi = d.pos[i];
         ti = type_of(xi.w);
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(256) k_force_seg(Dev d, Box b, StepConsts sc, 
           const uint4 *row4 = reinterpret_cast<const uint4 *>(d.nbr + (size_t)task * cap * A) + (t * A + a);
           const int4 ri = d.ic[i];
           ti = ri.w;
-          float ax = 0.f, ay = 0.f, az = 0.f, vr = 0.f, pp = 0.f;
+          float ax = 0.f, ay = 0.f, az = 0.f;
           if (staged) {
             const int hx = d.cell_of[i] - rowc - x0;  // home cell within the segment
             const int *tr = toff + hx;
@@ -329,13 +329,13 @@ __global__ void __launch_bounds__(256) k_force_seg(Dev d, Box b, StepConsts sc, 
                                    const int k = (int)(w >> CODE_SHIFT), r = (k * 11) >> 5;  // k / 3 for k < 27
                                    return stage[(int)(w & IDX_MASK) + tr[r * U + (k - 3 * r)]];
                                  },
-                                 ax, ay, az, vr, pp);
+                                 ax, ay, az, vir, pe);
           } else {
             const int4 *ic = d.ic;
             mixed_pairs<TPA, EV, ONE, false>(row4, nn, t, ri, nt, tab, one_type(tab), s_uh, s_ul, sc.jump_tolf,
-                                 [ic](uint32_t w) { return __ldg(&ic[w & IDX_MASK]); }, ax, ay, az, vr, pp);
+                                 [ic](uint32_t w) { return __ldg(&ic[w & IDX_MASK]); }, ax, ay, az, vir, pe);
           }
-          fx = ax; fy = ay; fz = az; vir = vr; pe = pp;
+          fx = ax; fy = ay; fz = az;
         }
         fold_lanes<A, EV>(fx, fy, fz, vir, pe);
         if (act && t == 0) {

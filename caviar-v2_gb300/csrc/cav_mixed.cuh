@@ -144,13 +144,18 @@ __device__ __forceinline__ void mixed_pair2(const int4 &ja, const int4 &jb, bool
 // fluid and a launch takes 160 us instead of 186 (one lane per atom); half or a quarter
 // of the gathers through the texture path: 174 and 192 us; 40 or 48 warps per SM (48 and
 // 40 registers): 240 and 320 us, the loop spills.
+// Sums: a lane holds its even and its odd entries in one FP32 sum each.  One lane per atom
+// thus has two sums of ~38 entries where four lanes have eight of ~10, whose pairs meet in
+// FP64: force error 5.51e-7 and 5.45e-7 of the rms at 256,000 atoms (1.31e-6 on four lanes with
+// cell-relative coordinates).  The two are joined in FP32 (in FP64: 5.50e-7, and 1.6% more
+// time per step with one lane, 10% with four), virial and energy in FP64.
 // ONE: single-type system, pair constants in registers; otherwise from the
 // shared-memory table.
 template <int TPA, bool EV, bool ONE, bool COH, class Gather>
 __device__ __forceinline__ void mixed_pairs(const uint4 *row4, int nn, int t, const int4 ri, int nt,
                                             const SmemTabF &tab, const OneType c1, const float4 uh,
                                             const float4 ul, const float jtol, Gather gather, float &ax,
-                                            float &ay, float &az, float &vr, float &pp) {
+                                            float &ay, float &az, double &vr, double &pp) {
   PairSums S;
   S.ax = S.ay = S.az = S.vr = S.pp = f2(0.f, 0.f);
   const int nfull = nn >> 2;
@@ -178,8 +183,8 @@ __device__ __forceinline__ void mixed_pairs(const uint4 *row4, int nn, int t, co
   unf2(S.ay, lo, hi); ay += lo + hi;
   unf2(S.az, lo, hi); az += lo + hi;
   if (EV) {
-    unf2(S.vr, lo, hi); vr -= lo + hi;
-    unf2(S.pp, lo, hi); pp += lo + hi;
+    unf2(S.vr, lo, hi); vr = -((double)lo + (double)hi);
+    unf2(S.pp, lo, hi); pp = (double)lo + (double)hi;
   }
 }
 
