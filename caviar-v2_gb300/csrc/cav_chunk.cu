@@ -43,6 +43,12 @@ constexpr int FP64_ATOMS = 12288;
 // FP64 99.5 and 92.1; of 16 (5,200) mixed 73.9 and 66.6, FP64 120 and 101; of 36 (11,800)
 // mixed 77.0 and 71.2.
 constexpr int MAX_REPLICAS = 6;
+// One block scans the cells of a replica while the others wait, at ~0.7 us per step and 1,000
+// cells: step of a 4,000-atom droplet in boxes of 9,261, 42,875 and 1,225,043 cells mixed 22.7,
+// 46.1 and 828 us here, 25.4, 26.3 and 59.4 with kernels, FP64 40.2, 63.2 and 836 against
+// 47.8, 48.8 and 81.9; of 32,000 atoms mixed 32.8, 58.0 and 913 against 35.1, 36.0 and 71.2.  (The
+// waits of boxes with 10^8 cells would run into the barrier's limit.)
+constexpr int MAX_CELLS = 12288;
 // polls of a barrier before a block gives up (seconds): the launch is cooperative, so a block
 // that never comes means a fault elsewhere; the host then reads F_STALL
 constexpr unsigned BARRIER_POLLS = 1u << 21;
@@ -451,7 +457,7 @@ int pick(const ChunkArgs &A, int kick, bool one, int want, cudaStream_t st) {
 // Sizes for which the kernels' blocks hold one task per warp (the partial sums are then
 // those of the virtual blocks), at the lane counts small systems use.
 bool chunk_fits(const Box &b, const LaunchCfg &lc) {
-  if (b.nrep > MAX_REPLICAS) return false;
+  if (b.nrep > MAX_REPLICAS || b.ncell_all > MAX_CELLS) return false;
   if (lc.images) return false;  // (k_force alone applies image codes to fixed-point coordinates)
   if (lc.use_seg || lc.block != CHUNK_THREADS || (lc.tpa != 2 && lc.tpa != 4)) return false;
   if (lc.precision == CAVGPU_FP64 && (!lc.exchange || lc.tpa != 4 || lc.n > FP64_ATOMS)) return false;
