@@ -539,7 +539,9 @@ int make_repbox(double ce, double skin, double rc, const double lo[3], const dou
     rb->uh[a] = (float)unit;
     rb->ul[a] = (float)(unit - (double)rb->uh[a]);
   }
-  rb->ncell = rb->nc[0] * rb->nc[1] * rb->nc[2];
+  // (beyond 2^30 cells the upload is refused)
+  const double ncell = (double)rb->nc[0] * rb->nc[1] * rb->nc[2];
+  rb->ncell = ncell > 1073741824.0 ? 1 << 30 : (int)ncell;
   return CAVGPU_OK;
 }
 

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) k_scatter(Dev d, Box b, int forced) {
 }
 
 __global__ void __launch_bounds__(256) k_sort_gather(Dev d, Box b, int forced) {
-  const int cell = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int cell = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);  // up to 2^30 cells
   if (cell < b.ncell_all) rebuild_sort_gather(d, b, forced, cell);
 }
 
