@@ -1030,11 +1030,12 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
   const bool eager = c->p.steps_per_graph < 0;
   // small systems: a chunk's steps in one launch (cav_chunk.cu); not while kernel times are
   // taken, nor with constraint::Nve between the steps
-  const bool small = !eager && !c->prof && c->nve.step == 0 && chunk_fits(c->b, c->lc);
+  auto step_kernel = [&] { return !eager && !c->prof && c->nve.step == 0 && chunk_fits(c->b, c->lc); };
+  bool small = step_kernel();
   RK(ensure_status(c));
   int f[F_NWORDS];
   if (c->nan_seen) return CAVGPU_E_NAN;  // a context that met a NaN does not step again
-  const int passes0 = c->passes;
+  int passes0 = c->passes;
   struct InFlight {
     int64_t start;
     int sz, slot;
@@ -1115,6 +1116,8 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
     if (f[F_NAN] || !f[F_OVERFLOW]) return CAVGPU_E_NAN;
     const ChunkPlan plan = *p.plan;  // growing the list frees the graphs that hold it
     RK(complete_overflowed_step(c, plan, k, done, nsteps, every, out5, f[F_OVERFLOW]));
+    if (small && !(small = step_kernel()))  // the list has grown, and left no room for the pair exchange
+      passes0 = c->passes;
     RK(read_flags(c, f));
     if (f[F_HALT]) return f[F_NAN] ? CAVGPU_E_NAN : CAVGPU_E_NLIST_OVERFLOW;
     done += 1;

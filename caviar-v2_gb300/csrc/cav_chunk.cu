@@ -468,6 +468,7 @@ bool chunk_fits(const Box &b, const LaunchCfg &lc) {
 
 int launch_chunk(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int S, int ev, int fuse, int drop,
                  const FoldArgs &fa, cudaStream_t st) {
+  if (lc.precision == CAVGPU_FP64 && (!lc.exchange || !d.recv)) return CAVGPU_E_ARG;
   ChunkArgs A{d, b, sc, fa, S, ev, fuse, drop, force_grid_blocks(lc), b.ncell_all, fuse == FUSE_LANG, lc.n <= BY_ATOM};
   const int want = std::max((lc.n + 32 / lc.tpa - 1) / (32 / lc.tpa), A.by_atom ? lc.n / CHUNK_WARPS : 0);
   const int kick = fuse == FUSE_LANG ? 2 : 1;

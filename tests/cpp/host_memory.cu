@@ -1,0 +1,78 @@
+// host_memory.cu -- the library's host side when device memory runs short, on the CPU
+// (fake_cudart.cpp in place of the runtime).  Argument: the scenario.  Prints what the
+// Python side checks, as key value lines.
+#include <cstdio>
+#include <cstring>
+#include <random>
+#include <vector>
+
+#include "cav_common.cuh"
+#include "fake_cudart.h"
+
+namespace {
+
+struct Md {
+  cavgpu_ctx *c = nullptr;
+  int rc = 0;
+  explicit Md(int n, int capacity = 0, double edge = 12.0) {
+    cavgpu_params p;
+    cavgpu_default_params(&p);
+    for (int a = 0; a < 3; ++a) p.hi[a] = edge;
+    p.nbr_capacity = capacity;
+    std::mt19937 g(1);
+    std::uniform_real_distribution<double> u(0.0, edge);
+    std::vector<double> x(3 * n);
+    for (double &v : x) v = u(g);
+    std::vector<uint64_t> t(n, 0);
+    rc = cavgpu_create(&p, &c);
+    if (!rc) rc = cavgpu_upload(c, n, x.data(), nullptr, t.data(), nullptr);
+    if (!rc) rc = cavgpu_setup(c);
+  }
+  ~Md() { cavgpu_destroy(c); }
+};
+
+void say(const char *key, long long v) { std::printf("%s %lld\n", key, v); }
+
+bool is_chunk(const std::string &name) { return name.find("k_chunk") != std::string::npos; }
+// first member of the step kernel's argument
+cav::Dev &dev_of(void **args) { return *static_cast<cav::Dev *>(args[0]); }
+
+// the list of the first chunk overflows; what happens then is up to the memory limit
+int overflow(size_t room) {
+  Md m(500, 64);
+  say("setup", m.rc);
+  int chunks = 0, nulls = 0;
+  bool fired = false;
+  fake::on_launch = [&](const std::string &name, void **args) {
+    if (!is_chunk(name)) return;
+    cav::Dev &d = dev_of(args);
+    ++chunks;
+    if (!d.recv || !d.hw) ++nulls;
+    if (!fired) {
+      fired = true;
+      d.flags[cav::F_HALT] = 1;
+      d.flags[cav::F_OVERFLOW] = 200;
+      d.flags[cav::F_HALT_STEP] = 3;
+      fake::limit = fake::used + room;
+    }
+  };
+  say("run", cavgpu_run(m.c, 400, 0, nullptr));
+  int64_t st[8];
+  cavgpu_stats(m.c, st);
+  say("steps", st[0]);
+  say("capacity", st[3]);
+  say("chunks", chunks);
+  say("nulls", nulls);
+  say("graphs", st[6]);
+  fake::on_launch = nullptr;
+  return 0;
+}
+
+}  // namespace
+
+int main(int argc, char **argv) {
+  const std::string what = argc > 1 ? argv[1] : "";
+  // 500 atoms, capacity 64 -> 320: list 0.13 -> 0.64 MB; exchange arrays 1.3 -> 3.2 MB
+  if (what == "exchange_lost") return overflow(1 << 20);
+  return 1;
+}

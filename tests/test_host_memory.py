@@ -1,0 +1,45 @@
+"""The library's host side when device memory runs short, without a GPU.
+
+tests/cpp/host_memory.cu drives the C ABI with a stand-in for the CUDA runtime
+(tests/cpp/fake_cudart.cpp) whose memory has a limit and whose kernels do not run.
+"""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import PKG, ROOT
+
+
+@pytest.fixture(scope="module")
+def program():
+    sys.path.insert(0, PKG)
+    import build as B
+
+    if not os.path.exists(B.LIB):
+        B.build()
+    out = os.path.join(ROOT, "tests", "cpp", "_build")
+    os.makedirs(out, exist_ok=True)
+    exe, src = os.path.join(out, "host_memory"), os.path.join(ROOT, "tests", "cpp")
+    objs = [os.path.join(B.OBJ, os.path.splitext(s)[0] + ".o") for s in B.SOURCES]
+    subprocess.run([B.NVCC, *B.ARCH, "-std=c++17", "-O1", "-cudart", "none", "-I" + os.path.join(ROOT, "include"),
+                    "-I" + B.CSRC, "-I" + src, os.path.join(src, "host_memory.cu"), os.path.join(src, "fake_cudart.cpp"),
+                    *objs, "-o", exe], check=True, capture_output=True, text=True)
+
+    def run(scenario):
+        r = subprocess.run([exe, scenario], capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stderr
+        return {k: int(v) for k, v in (line.split() for line in r.stdout.splitlines())}
+
+    return run
+
+
+def test_step_kernel_stops_when_the_exchange_arrays_do_not_fit_any_more(program):
+    """A list that grows in mid-run may leave no room for the pair exchange; the run then goes on
+    with kernels over the full list."""
+    r = program("exchange_lost")
+    assert r["setup"] == 0 and r["run"] == 0
+    assert r["steps"] == 400 and r["capacity"] == 320
+    assert r["nulls"] == 0  # no step kernel without its arrays
+    assert 1 <= r["chunks"] <= 2 and r["graphs"] >= 1
