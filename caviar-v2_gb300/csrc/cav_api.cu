@@ -401,6 +401,16 @@ int clear_status(cavgpu_ctx *c) {
   return CAVGPU_OK;
 }
 
+// gives the arrays of the FP64 pair exchange back
+void drop_exchange(cavgpu_ctx *c) {
+  if (c->p.precision != CAVGPU_FP64) return;  // (d.ic is the mixed form's own)
+  Dev &d = c->d;
+  if (c->x_mem) cudaFree(c->x_mem);
+  c->x_mem = nullptr;
+  d.hw = nullptr; d.hslot = nullptr; d.nh = d.nr = nullptr; d.recv = d.own = nullptr; d.ic = nullptr; d.ev_part = nullptr;
+  c->lc.exchange = 0;
+}
+
 // (Re)allocate the arrays of the FP64 pair exchange for the list's capacity: half of it
 // per atom each way, and no less than 64 of a capacity of 64 (an atom claims half its
 // entries and receives the other half; a row that outgrows this grows the list).  38 bytes
@@ -409,10 +419,7 @@ int clear_status(cavgpu_ctx *c) {
 // instead (k_force), at about twice the time and the same precision.
 int alloc_exchange(cavgpu_ctx *c) {
   Dev &d = c->d;
-  if (c->x_mem) cudaFree(c->x_mem);
-  c->x_mem = nullptr;
-  d.hw = nullptr; d.hslot = nullptr; d.nh = d.nr = nullptr; d.recv = d.own = nullptr; d.ic = nullptr; d.ev_part = nullptr;
-  c->lc.exchange = 0;
+  drop_exchange(c);
   if (d.tpa > 4) return CAVGPU_OK;  // four partial sums: at most four lanes per atom
   const size_t n = ((size_t)c->b.nslot + 31) / 32 * 32, cap_h = (size_t)std::max(std::min(d.cap, 64), d.cap / 2);
   const size_t recv = n * cap_h * sizeof(dbl4), words = n * cap_h * sizeof(uint32_t), slots = n * cap_h * sizeof(uint16_t);
@@ -453,6 +460,7 @@ int alloc_nbr(cavgpu_ctx *c, int cap) {
     cudaFree(c->d.nbr);
     c->d.nbr = nullptr;
   }
+  drop_exchange(c);  // the list comes first: the force does without these arrays
   void *q = nullptr;
   if (cudaMalloc(&q, bytes) != cudaSuccess) { cudaGetLastError(); return CAVGPU_E_NOMEM; }
   c->allocs.push_back(q);

@@ -74,5 +74,7 @@ int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   // 500 atoms, capacity 64 -> 320: list 0.13 -> 0.64 MB; exchange arrays 1.3 -> 3.2 MB
   if (what == "exchange_lost") return overflow(1 << 20);
+  // no room for the new list beside the exchange arrays
+  if (what == "list_grows") return overflow(300 << 10);
   return 1;
 }

@@ -43,3 +43,10 @@ def test_step_kernel_stops_when_the_exchange_arrays_do_not_fit_any_more(program)
     assert r["steps"] == 400 and r["capacity"] == 320
     assert r["nulls"] == 0  # no step kernel without its arrays
     assert 1 <= r["chunks"] <= 2 and r["graphs"] >= 1
+
+
+def test_a_growing_list_takes_the_room_of_the_exchange_arrays(program):
+    """The list's new rows fit once the arrays that the force can do without are given back."""
+    r = program("list_grows")
+    assert r["setup"] == 0 and r["run"] == 0
+    assert r["steps"] == 400 and r["capacity"] == 320 and r["nulls"] == 0
