@@ -70,6 +70,7 @@ _SIGS = {
     "cavgpu_export_ghosts": (C.c_int64, [C.c_void_p, C.c_double, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                          C.c_int64]),
     "cavgpu_stats": (C.c_int, [C.c_void_p, C.c_void_p]),
+    "cavgpu_pair_exchange": (C.c_int, [C.c_void_p]),
     "cavgpu_stream": (C.c_void_p, [C.c_void_p]),
     "cavgpu_set_profiling": (C.c_int, [C.c_void_p, C.c_int32]),
     "cavgpu_read_profile": (C.c_int, [C.c_void_p, C.c_void_p]),
@@ -248,6 +249,10 @@ class System:
         keys = ("steps", "rebuilds", "max_neighbours", "capacity", "threads_per_atom", "block_size",
                 "graph_launches", "kernel_launches")
         return dict(zip(keys, (int(x) for x in o)))
+
+    def pair_exchange(self):
+        """Whether the FP64 form evaluates each pair once (needs more memory) or from both sides."""
+        return bool(self._check(lib().cavgpu_pair_exchange(self._h), "pair_exchange"))
 
     def stream(self):
         return lib().cavgpu_stream(self._h)

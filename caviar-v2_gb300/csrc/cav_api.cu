@@ -71,6 +71,8 @@ std::vector<std::pair<TuneKey, TuneChoice>> g_tune_cache;
 }  // namespace
 
 struct cavgpu_ctx {
+  std::recursive_mutex mu;  // held by every call on the context; see give_back
+  int dev = 0;
   cavgpu_params p{};
   Dev d{};
   Box b{};
@@ -131,19 +133,67 @@ int cuda_rc(cudaError_t e) {
     if (_rc) return _rc;   \
   } while (0)
 
-template <class T>
-int dalloc(cavgpu_ctx *c, T **p, size_t count) {
-  void *q = nullptr;
-  cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-  if (e != cudaSuccess) { cudaGetLastError(); return CAVGPU_E_NOMEM; }
-  c->allocs.push_back(q);
-  *p = static_cast<T *>(q);
-  return CAVGPU_OK;
-}
-
 void free_graphs(cavgpu_ctx *c) {
   for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
   c->graphs.clear();
+}
+
+// gives the arrays of the FP64 pair exchange back
+void drop_exchange(cavgpu_ctx *c) {
+  if (c->p.precision != CAVGPU_FP64) return;  // (d.ic is the mixed form's own)
+  Dev &d = c->d;
+  if (c->x_mem) cudaFree(c->x_mem);
+  c->x_mem = nullptr;
+  d.hw = nullptr; d.hslot = nullptr; d.nh = d.nr = nullptr; d.recv = d.own = nullptr; d.ic = nullptr; d.ev_part = nullptr;
+  c->lc.exchange = 0;
+}
+
+// drop_exchange for a context whose stream may still be at work
+void give_back(cavgpu_ctx *c) {
+  if (!c->x_mem) return;
+  cudaStreamSynchronize(c->st);
+  free_graphs(c);  // they hold the arrays' addresses
+  drop_exchange(c);
+}
+
+// The live contexts.  The exchange arrays are most of an FP64 context's memory and the force
+// does without them, so a context that runs short takes those of the contexts that no call
+// holds at that moment, then its own.  (A context in a call on another thread keeps its
+// arrays.)  Lock order: a call's own context, then the table; other contexts are only tried.
+std::mutex g_ctx_mu;
+std::vector<cavgpu_ctx *> g_ctx;
+
+// device memory that the context cannot do without
+cudaError_t must_malloc(cavgpu_ctx *c, void **q, size_t bytes) {
+  cudaError_t e = cudaMalloc(q, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    {
+      std::lock_guard<std::mutex> table(g_ctx_mu);
+      for (cavgpu_ctx *o : g_ctx) {
+        if (o == c || o->dev != c->dev) continue;
+        std::unique_lock<std::recursive_mutex> l(o->mu, std::try_to_lock);
+        if (l.owns_lock()) give_back(o);
+      }
+    }
+    e = cudaMalloc(q, bytes);
+  }
+  if (e == cudaErrorMemoryAllocation && c->x_mem) {
+    cudaGetLastError();
+    give_back(c);
+    e = cudaMalloc(q, bytes);
+  }
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
+template <class T>
+int dalloc(cavgpu_ctx *c, T **p, size_t count) {
+  void *q = nullptr;
+  if (must_malloc(c, &q, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) return CAVGPU_E_NOMEM;
+  c->allocs.push_back(q);
+  *p = static_cast<T *>(q);
+  return CAVGPU_OK;
 }
 
 bool is_lang(const cavgpu_ctx *c) { return c->p.integrator == CAVGPU_VELOCITY_VERLET_LANGEVIN; }
@@ -401,22 +451,13 @@ int clear_status(cavgpu_ctx *c) {
   return CAVGPU_OK;
 }
 
-// gives the arrays of the FP64 pair exchange back
-void drop_exchange(cavgpu_ctx *c) {
-  if (c->p.precision != CAVGPU_FP64) return;  // (d.ic is the mixed form's own)
-  Dev &d = c->d;
-  if (c->x_mem) cudaFree(c->x_mem);
-  c->x_mem = nullptr;
-  d.hw = nullptr; d.hslot = nullptr; d.nh = d.nr = nullptr; d.recv = d.own = nullptr; d.ic = nullptr; d.ev_part = nullptr;
-  c->lc.exchange = 0;
-}
-
 // (Re)allocate the arrays of the FP64 pair exchange for the list's capacity: half of it
 // per atom each way, and no less than 64 of a capacity of 64 (an atom claims half its
 // entries and receives the other half; a row that outgrows this grows the list).  38 bytes
-// per entry, ~3.7 KB per atom of the benchmark fluid: a system for which that is more than a quarter of the device's
-// memory, or more than is free, evaluates its pairs from both sides over the full list
-// instead (k_force), at about twice the time and the same precision.
+// per entry, ~3.7 KB per atom of the benchmark fluid: a system for which that is more than a
+// quarter of the device's memory, or more than is free, evaluates its pairs from both sides
+// over the full list instead (k_force), at about twice the time and the same precision.  So
+// does a context whose arrays another one took (must_malloc); cavgpu_pair_exchange tells.
 int alloc_exchange(cavgpu_ctx *c) {
   Dev &d = c->d;
   drop_exchange(c);
@@ -462,7 +503,7 @@ int alloc_nbr(cavgpu_ctx *c, int cap) {
   }
   drop_exchange(c);  // the list comes first: the force does without these arrays
   void *q = nullptr;
-  if (cudaMalloc(&q, bytes) != cudaSuccess) { cudaGetLastError(); return CAVGPU_E_NOMEM; }
+  if (must_malloc(c, &q, bytes) != cudaSuccess) return CAVGPU_E_NOMEM;
   c->allocs.push_back(q);
   c->d.nbr = static_cast<uint32_t *>(q);
   c->d.cap = cap;
@@ -568,6 +609,7 @@ int create_common(const cavgpu_params *p, int nrep, const double *lo3, const dou
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) { cudaGetLastError(); return CAVGPU_E_CUDA; }
   cavgpu_ctx *c = new (std::nothrow) cavgpu_ctx();
   if (!c) return CAVGPU_E_NOMEM;
+  cudaGetDevice(&c->dev);
   c->p = *p;
   const double ce = p->nl_cutoff * p->nl_coef;  // Neighborlist::init (src/neighborlist.cpp:317)
   c->cutoff_extra = ce;
@@ -698,6 +740,10 @@ int create_common(const cavgpu_params *p, int nrep, const double *lo3, const dou
   if (!rc) rc = cuda_rc(cudaMemcpyAsync(c->d.step_base, &step0, sizeof(long long), cudaMemcpyHostToDevice, c->st));
   if (!rc) rc = cuda_rc(cudaStreamSynchronize(c->st));
   if (rc) { cavgpu_destroy(c); return rc; }
+  {
+    std::lock_guard<std::mutex> table(g_ctx_mu);
+    g_ctx.push_back(c);
+  }
   *out = c;
   return CAVGPU_OK;
 }
@@ -1191,6 +1237,10 @@ int cavgpu_create_batch(const cavgpu_params *p, int32_t nrep, const double *lo3,
 
 void cavgpu_destroy(cavgpu_ctx *c) {
   if (!c) return;
+  {
+    std::lock_guard<std::mutex> table(g_ctx_mu);  // (waits for a give_back that looks at it)
+    g_ctx.erase(std::remove(g_ctx.begin(), g_ctx.end(), c), g_ctx.end());
+  }
   if (c->st) cudaStreamSynchronize(c->st);
   free_graphs(c);
   for (auto e : c->ev0) cudaEventDestroy(e);
@@ -1207,17 +1257,20 @@ void cavgpu_destroy(cavgpu_ctx *c) {
 int cavgpu_upload(cavgpu_ctx *c, int64_t n, const double *pos3, const double *vel3, const uint64_t *type,
                   const uint64_t *id) {
   if (!c || n < 1 || c->b.nrep != 1) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   return upload_common(c, &n, pos3, vel3, type, id);
 }
 
 int cavgpu_upload_batch(cavgpu_ctx *c, const int64_t *counts, const double *pos3, const double *vel3,
                         const uint64_t *type) {
   if (!c || !counts) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   return upload_common(c, counts, pos3, vel3, type, nullptr);
 }
 
 int cavgpu_set_molecules(cavgpu_ctx *c, const int32_t *mol) {
   if (!c || !mol) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->uploaded || c->set_up || !c->d.mol) return CAVGPU_E_STATE;
   // slots are still in upload order: replica r's atoms from its slot offset, padding -1
   std::vector<int> h(c->b.nslot, -1);
@@ -1231,11 +1284,13 @@ int cavgpu_set_molecules(cavgpu_ctx *c, const int32_t *mol) {
 
 int cavgpu_setup(cavgpu_ctx *c) {
   if (!c) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   return setup_common(c);
 }
 
 int cavgpu_run(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
   if (!c || nsteps < 0 || every < 0 || (every > 0 && !out5)) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (every > 0 && c->b.nrep > 1) return CAVGPU_E_ARG;  // batches: cavgpu_thermo_batch after the call
   if (!c->set_up) return CAVGPU_E_STATE;
   if (nsteps == 0) return CAVGPU_OK;
@@ -1246,6 +1301,7 @@ int cavgpu_step(cavgpu_ctx *c, int64_t nsteps) { return cavgpu_run(c, nsteps, 0,
 
 int cavgpu_autotune(cavgpu_ctx *c, int32_t trial_steps, int32_t flags, int64_t *out6) {
   if (!c || trial_steps < 0) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->set_up) return CAVGPU_E_STATE;
   const int T = trial_steps > 0 ? trial_steps : 40;
   int dev = 0;
@@ -1269,14 +1325,13 @@ int cavgpu_autotune(cavgpu_ctx *c, int32_t trial_steps, int32_t flags, int64_t *
   std::vector<double> snap_rep(c->d.thermo_rep ? 8 * (size_t)c->b.nrep : 0);
   const long long steps0 = c->steps_done, graphs0 = c->graph_launches, kern0 = c->kernel_launches;
   const bool prof0 = c->prof;
-  if (cudaMalloc(&snap, 3 * NS * sizeof(dbl4)) != cudaSuccess) { cudaGetLastError(); return CAVGPU_E_NOMEM; }
-  if (cudaMalloc(&snap_i, 2 * NS * sizeof(int)) != cudaSuccess) { cudaFree(snap); cudaGetLastError(); return CAVGPU_E_NOMEM; }
+  auto need = [&](auto **q, size_t bytes) { return must_malloc(c, reinterpret_cast<void **>(q), bytes) == cudaSuccess; };
+  if (!need(&snap, 3 * NS * sizeof(dbl4))) return CAVGPU_E_NOMEM;
+  if (!need(&snap_i, 2 * NS * sizeof(int))) { cudaFree(snap); return CAVGPU_E_NOMEM; }
   // per-slot crossing counts and molecule indices move with the atoms as well
   int4 *snap_img = nullptr;
   int *snap_mol = nullptr;
-  if ((c->d.img && cudaMalloc(&snap_img, NS * sizeof(int4)) != cudaSuccess) ||
-      (c->d.mol && cudaMalloc(&snap_mol, NS * sizeof(int)) != cudaSuccess)) {
-    cudaGetLastError();
+  if ((c->d.img && !need(&snap_img, NS * sizeof(int4))) || (c->d.mol && !need(&snap_mol, NS * sizeof(int)))) {
     cudaFree(snap); cudaFree(snap_i); cudaFree(snap_img);
     return CAVGPU_E_NOMEM;
   }
@@ -1413,6 +1468,7 @@ int cavgpu_autotune(cavgpu_ctx *c, int32_t trial_steps, int32_t flags, int64_t *
 
 int cavgpu_forces(cavgpu_ctx *c, double *virial, double *pe) {
   if (!c) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->set_up) return CAVGPU_E_STATE;
   const Status *h = nullptr;
   RK(build_and_force(c, &h));
@@ -1433,6 +1489,7 @@ int cavgpu_forces(cavgpu_ctx *c, double *virial, double *pe) {
 
 int cavgpu_thermo(cavgpu_ctx *c, double *out6) {
   if (!c || !out6) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->set_up) return CAVGPU_E_STATE;
   if (c->b.nrep > 1) return CAVGPU_E_ARG;  // cavgpu_thermo_batch
   const Status *h = nullptr;
@@ -1444,6 +1501,7 @@ int cavgpu_thermo(cavgpu_ctx *c, double *out6) {
 
 int cavgpu_thermo_batch(cavgpu_ctx *c, double *out6) {
   if (!c || !out6) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->set_up) return CAVGPU_E_STATE;
   const int R = c->b.nrep;
   if (R == 1) return cavgpu_thermo(c, out6);
@@ -1457,6 +1515,7 @@ int cavgpu_thermo_batch(cavgpu_ctx *c, double *out6) {
 
 int cavgpu_download(cavgpu_ctx *c, double *pos3, double *vel3, double *acc3) {
   if (!c) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->uploaded) return CAVGPU_E_STATE;
   // one kernel, the copies and one wait; the rebuild's scratch holds the host-order arrays
   // (24 of its 32 bytes per slot)
@@ -1474,6 +1533,7 @@ int cavgpu_download(cavgpu_ctx *c, double *pos3, double *vel3, double *acc3) {
 
 int cavgpu_download_images(cavgpu_ctx *c, int32_t *img3) {
   if (!c || !img3) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->uploaded || !c->d.img) return CAVGPU_E_STATE;
   RK(launch_images_to_host(c->d, c->b, c->st));
   CK(cudaMemcpyAsync(img3, c->d.hi3, 3 * sizeof(int32_t) * c->natoms, cudaMemcpyDeviceToHost, c->st));
@@ -1483,6 +1543,7 @@ int cavgpu_download_images(cavgpu_ctx *c, int32_t *img3) {
 
 int64_t cavgpu_export_pairs(cavgpu_ctx *c, int32_t *out5, int64_t cap) {
   if (!c || (cap > 0 && !out5) || c->b.nrep != 1) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->set_up) return CAVGPU_E_STATE;
   std::vector<int> nn(c->b.nslot);
   if (cudaMemcpyAsync(nn.data(), c->d.nnbr, c->b.nslot * sizeof(int), cudaMemcpyDeviceToHost, c->st) != cudaSuccess ||
@@ -1494,8 +1555,8 @@ int64_t cavgpu_export_pairs(cavgpu_ctx *c, int32_t *out5, int64_t cap) {
   if (take <= 0) return total;
   int32_t *rows = nullptr;
   unsigned long long *cnt = nullptr;
-  if (cudaMalloc(&rows, (size_t)take * 5 * sizeof(int32_t)) != cudaSuccess) { cudaGetLastError(); return CAVGPU_E_NOMEM; }
-  if (cudaMalloc(&cnt, sizeof(unsigned long long)) != cudaSuccess) { cudaFree(rows); cudaGetLastError(); return CAVGPU_E_NOMEM; }
+  if (must_malloc(c, (void **)&rows, (size_t)take * 5 * sizeof(int32_t)) != cudaSuccess) return CAVGPU_E_NOMEM;
+  if (must_malloc(c, (void **)&cnt, sizeof(unsigned long long)) != cudaSuccess) { cudaFree(rows); return CAVGPU_E_NOMEM; }
   int rc = cuda_rc(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), c->st));
   if (!rc) rc = launch_export_pairs(c->d, c->b, stencil_codes(c->lc) ? 1 : 0, rows, cnt, take, c->st);
   if (!rc) rc = cuda_rc(cudaMemcpyAsync(out5, rows, (size_t)take * 5 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->st));
@@ -1507,6 +1568,7 @@ int64_t cavgpu_export_pairs(cavgpu_ctx *c, int32_t *out5, int64_t cap) {
 
 int cavgpu_export_bins(cavgpu_ctx *c, int32_t *owned3, int32_t *nbins3) {
   if (!c || c->b.nrep != 1) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->uploaded) return CAVGPU_E_STATE;
   if (nbins3) for (int a = 0; a < 3; ++a) nbins3[a] = c->ref_nb[a];
   if (!owned3) return CAVGPU_OK;
@@ -1520,6 +1582,7 @@ int cavgpu_export_bins(cavgpu_ctx *c, int32_t *owned3, int32_t *nbins3) {
 int64_t cavgpu_export_ghosts(cavgpu_ctx *c, double ghost_cutoff, int32_t *src, int32_t *shift3, double *pos3,
                              int32_t *bins3, int64_t cap) {
   if (!c || ghost_cutoff < 0.0 || c->b.nrep != 1) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   if (!c->uploaded) return CAVGPU_E_STATE;
   const int N = c->natoms;
   int *counts = nullptr, *starts = nullptr;
@@ -1528,7 +1591,7 @@ int64_t cavgpu_export_ghosts(cavgpu_ctx *c, double ghost_cutoff, int32_t *src, i
   const int64_t gcap = std::max<int64_t>(cap, 0);
   int rc = CAVGPU_OK;
   auto M = [&](void **q, size_t bytes) {
-    if (!rc && cudaMalloc(q, std::max<size_t>(bytes, 16)) != cudaSuccess) { cudaGetLastError(); rc = CAVGPU_E_NOMEM; }
+    if (!rc && must_malloc(c, q, std::max<size_t>(bytes, 16)) != cudaSuccess) rc = CAVGPU_E_NOMEM;
   };
   M((void **)&counts, (size_t)N * sizeof(int));
   M((void **)&starts, ((size_t)N + 1) * sizeof(int));
@@ -1555,6 +1618,7 @@ int64_t cavgpu_export_ghosts(cavgpu_ctx *c, double ghost_cutoff, int32_t *src, i
 
 int cavgpu_stats(cavgpu_ctx *c, int64_t *o) {
   if (!c || !o) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   int f[F_NWORDS] = {0};
   if (c->uploaded) RK(read_flags(c, f));
   o[0] = c->steps_done;
@@ -1568,10 +1632,17 @@ int cavgpu_stats(cavgpu_ctx *c, int64_t *o) {
   return CAVGPU_OK;
 }
 
+int cavgpu_pair_exchange(cavgpu_ctx *c) {
+  if (!c) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
+  return c->lc.exchange ? 1 : 0;
+}
+
 void *cavgpu_stream(cavgpu_ctx *c) { return c ? (void *)c->st : nullptr; }
 
 int cavgpu_set_profiling(cavgpu_ctx *c, int32_t on) {
   if (!c) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   c->prof = on != 0;
   c->prof_ms = 0.0;
   c->prof_launches = 0;
@@ -1580,6 +1651,7 @@ int cavgpu_set_profiling(cavgpu_ctx *c, int32_t on) {
 
 int cavgpu_read_profile(cavgpu_ctx *c, double *out2) {
   if (!c || !out2) return CAVGPU_E_ARG;
+  std::lock_guard<std::recursive_mutex> call(c->mu);
   out2[0] = (double)c->prof_launches;
   out2[1] = c->prof_ms;
   return CAVGPU_OK;

@@ -76,7 +76,8 @@ typedef struct cavgpu_params {
   int32_t precision;              /* CAVGPU_FP64 or CAVGPU_MIXED */
   int32_t noise_off;              /* Langevin with eta = 0 (exactness checks) */
   int32_t nbr_capacity;           /* neighbour slots per atom; 0 = sized at set-up */
-  int32_t threads_per_atom;       /* force kernel lanes per atom (1,2,4,8,16); 0 = by system size */
+  int32_t threads_per_atom;       /* force kernel lanes per atom (1,2,4,8,16); 0 = by system size
+                                     (FP64: 1, 2, 4 give the same bits, see cavgpu_pair_exchange) */
   int32_t block_size;             /* force kernel block size (32..256, multiple of 32); 0 = default */
   int32_t steps_per_graph;        /* steps captured per CUDA graph; 0 = default (50); < 0 = no
                                      graphs, every kernel launched from the host (for profilers,
@@ -205,6 +206,17 @@ int64_t cavgpu_export_ghosts(cavgpu_ctx *ctx, double ghost_cutoff, int32_t *src,
 /* Statistics: out8 = {steps done, rebuilds, max neighbours, capacity,
  * threads per atom, block size, graph launches, kernel launches}. */
 int cavgpu_stats(cavgpu_ctx *ctx, int64_t *out8);
+
+/* Whether the FP64 form evaluates each pair once (1) or from both sides over the full list
+ * (0; always of the mixed form).  Once needs 38 bytes per list entry beside the list, ~3.7 KB
+ * per atom of a fluid with 2.8 sigma lists, and takes half the time; the two forms' sums
+ * differ at rounding level.  It is chosen when a list is allocated (setup, autotune, growth),
+ * for 1, 2 or 4 threads per atom, if those arrays take no more than a quarter of the device's
+ * memory and fit.  They are given back, and the full list is used from then on, when
+ * another context of the process runs out of memory while no call is at work on this one.
+ * threads_per_atom = 8 or 16 declines them: for programs that need the memory, or the same
+ * bits whatever else is on the device. */
+int cavgpu_pair_exchange(cavgpu_ctx *ctx);
 
 /* The CUDA stream the context launches on (a cudaStream_t). */
 void *cavgpu_stream(cavgpu_ctx *ctx);

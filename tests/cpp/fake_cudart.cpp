@@ -17,16 +17,19 @@ static std::map<void *, size_t> blocks;
 static std::recursive_mutex mu;
 
 static cudaError_t launch(const void *func, void **args) {
-  std::lock_guard<std::recursive_mutex> g(mu);
-  const std::string name = names.count(func) ? names[func] : "?";
-  ++launches[name];
-  if (on_launch) on_launch(name, args);
+  std::string name = "?";
+  {
+    std::lock_guard<std::recursive_mutex> g(mu);
+    if (names.count(func)) name = names[func];
+    ++launches[name];
+  }
+  if (on_launch && name != "?") on_launch(name, args);
   return cudaSuccess;
 }
 }  // namespace fake
 
 using namespace fake;
-static int capturing = 0;
+static thread_local int capturing = 0;
 
 extern "C" {
 void **__cudaRegisterFatBinary(void *) { static void *h; return &h; }
@@ -36,7 +39,7 @@ void __cudaRegisterFunction(void **, const char *host, char *, const char *name,
   names[host] = name;
 }
 void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, int) {}
-static struct { dim3 g, b; size_t m; void *s; } call;
+static thread_local struct { dim3 g, b; size_t m; void *s; } call;
 unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t m, void *s) { call = {g, b, m, s}; return 0; }
 cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *m, void *s) {
   *g = call.g; *b = call.b; *m = call.m; *(void **)s = call.s;

@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstring>
 #include <random>
+#include <thread>
 #include <vector>
 
 #include "cav_common.cuh"
@@ -68,6 +69,70 @@ int overflow(size_t room) {
   return 0;
 }
 
+int run_all(Md &m, int *nulls) {
+  fake::on_launch = [=](const std::string &name, void **args) {
+    if (is_chunk(name) && !dev_of(args).recv) ++*nulls;
+  };
+  const int rc = cavgpu_run(m.c, 200, 0, nullptr);
+  fake::on_launch = nullptr;
+  return rc;
+}
+
+// a context is created where only the exchange arrays of another one leave room for it
+int second_context() {
+  Md a(500, 64);
+  int nulls = 0;
+  say("setup", a.rc);
+  say("run", run_all(a, &nulls));
+  say("exchange_before", cavgpu_pair_exchange(a.c));
+  fake::limit = fake::used + (200 << 10);
+  {
+    Md b(500, 64);
+    say("second_setup", b.rc);
+    say("second_run", run_all(b, &nulls));
+    say("exchange_after", cavgpu_pair_exchange(a.c));
+    say("run_again", run_all(a, &nulls));
+  }
+  fake::limit = (size_t)-1;
+  say("run_last", run_all(a, &nulls));
+  say("nulls", nulls);
+  return 0;
+}
+
+// the same while a call on another thread holds the first context: it keeps its arrays
+int busy_context() {
+  Md a(500, 64);
+  say("setup", a.rc);
+  fake::limit = fake::used + (200 << 10);
+  int second = 1, nulls = 0, chunks = 0;
+  fake::on_launch = [&](const std::string &name, void **args) {
+    if (!is_chunk(name)) return;
+    if (!dev_of(args).recv) ++nulls;
+    if (++chunks != 1) return;
+    std::thread t([&] { Md b(500, 64); second = b.rc; });
+    t.join();
+  };
+  say("run", cavgpu_run(a.c, 200, 0, nullptr));
+  fake::on_launch = nullptr;
+  say("second_setup", second);
+  say("exchange", cavgpu_pair_exchange(a.c));
+  say("nulls", nulls);
+  return 0;
+}
+
+// the autotuner's snapshot fits once the context's own arrays are given back
+int autotune() {
+  Md a(4000, 128, 20.0);
+  say("setup", a.rc);
+  say("exchange_before", cavgpu_pair_exchange(a.c));
+  fake::limit = fake::used + (100 << 10);
+  say("autotune", cavgpu_autotune(a.c, 4, 0, nullptr));
+  int nulls = 0;
+  say("run", run_all(a, &nulls));
+  say("nulls", nulls);
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -76,5 +141,8 @@ int main(int argc, char **argv) {
   if (what == "exchange_lost") return overflow(1 << 20);
   // no room for the new list beside the exchange arrays
   if (what == "list_grows") return overflow(300 << 10);
+  if (what == "second_context") return second_context();
+  if (what == "busy_context") return busy_context();
+  if (what == "autotune") return autotune();
   return 1;
 }

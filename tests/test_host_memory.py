@@ -50,3 +50,23 @@ def test_a_growing_list_takes_the_room_of_the_exchange_arrays(program):
     r = program("list_grows")
     assert r["setup"] == 0 and r["run"] == 0
     assert r["steps"] == 400 and r["capacity"] == 320 and r["nulls"] == 0
+
+
+def test_a_context_takes_the_exchange_arrays_of_an_idle_one(program):
+    r = program("second_context")
+    assert r["setup"] == 0 and r["run"] == 0 and r["exchange_before"] == 1
+    assert r["second_setup"] == 0 and r["second_run"] == 0 and r["exchange_after"] == 0
+    assert r["run_again"] == 0 and r["run_last"] == 0 and r["nulls"] == 0
+
+
+def test_a_context_in_a_call_keeps_its_exchange_arrays(program):
+    r = program("busy_context")
+    assert r["setup"] == 0 and r["run"] == 0
+    assert r["second_setup"] == -6  # CAVGPU_E_NOMEM
+    assert r["exchange"] == 1 and r["nulls"] == 0
+
+
+def test_autotune_takes_the_room_of_its_own_exchange_arrays(program):
+    r = program("autotune")
+    assert r["setup"] == 0 and r["exchange_before"] == 1
+    assert r["autotune"] == 0 and r["run"] == 0 and r["nulls"] == 0
