@@ -86,6 +86,7 @@ struct cavgpu_ctx {
   int natoms = 0;               // atoms over all replicas
   NveCfg nve{};                 // constraint::Nve (step 0 = off)
   bool uploaded = false, set_up = false;
+  bool stalled = false;  // a grid barrier gave up: the state is half way through a step
   long long steps_done = 0;
   long long graph_launches = 0, kernel_launches = 0;
   int max_nb = 0;
@@ -120,6 +121,11 @@ int cuda_rc(cudaError_t e) {
   if (e == cudaSuccess) return CAVGPU_OK;
   g_last_cuda_error = cudaGetErrorString(e);
   return e == cudaErrorMemoryAllocation ? CAVGPU_E_NOMEM : CAVGPU_E_CUDA;
+}
+
+int stall_rc() {
+  g_last_cuda_error = "the step kernel's blocks did not all reach a barrier";
+  return CAVGPU_E_CUDA;
 }
 
 #define CK(x)                        \
@@ -466,6 +472,9 @@ int alloc_exchange(cavgpu_ctx *c) {
   const size_t recv = n * cap_h * sizeof(dbl4), words = n * cap_h * sizeof(uint32_t), slots = n * cap_h * sizeof(uint16_t);
   const size_t evp = c->b.nrep > 1 ? n * d.tpa * sizeof(double2) : 0;
   const size_t bytes = recv + 4 * n * sizeof(dbl4) + evp + words + slots + n * sizeof(int4) + 2 * n * sizeof(int);
+#ifdef CAV_EXCHANGE_LIMIT  // (tests)
+  if (bytes > (size_t)(CAV_EXCHANGE_LIMIT)) return CAVGPU_OK;
+#endif
   if (bytes > ((size_t)1 << 30)) {  // (the query takes longer than allocating for a small system)
     size_t free_mem = 0, total_mem = 0;
     CK(cudaMemGetInfo(&free_mem, &total_mem));
@@ -1153,7 +1162,11 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
     c->max_nb = std::max(c->max_nb, hf[F_MAXNB]);
     c->nan_seen = hf[F_NAN] != 0;
     c->passes = hf[F_PASSES];
-    if (hf[F_STALL]) return CAVGPU_E_CUDA;  // a grid barrier of the step kernel gave up
+    if (hf[F_STALL]) {  // a grid barrier of the step kernel gave up
+      CK(cudaStreamSynchronize(c->st));
+      c->stalled = true;
+      return stall_rc();
+    }
     if (c->prof) RK(collect_profile(c, p.sz));
     if (!hf[F_HALT]) {
       done = p.start + p.sz;
@@ -1271,6 +1284,7 @@ int cavgpu_upload_batch(cavgpu_ctx *c, const int64_t *counts, const double *pos3
 int cavgpu_set_molecules(cavgpu_ctx *c, const int32_t *mol) {
   if (!c || !mol) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->uploaded || c->set_up || !c->d.mol) return CAVGPU_E_STATE;
   // slots are still in upload order: replica r's atoms from its slot offset, padding -1
   std::vector<int> h(c->b.nslot, -1);
@@ -1285,12 +1299,14 @@ int cavgpu_set_molecules(cavgpu_ctx *c, const int32_t *mol) {
 int cavgpu_setup(cavgpu_ctx *c) {
   if (!c) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   return setup_common(c);
 }
 
 int cavgpu_run(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
   if (!c || nsteps < 0 || every < 0 || (every > 0 && !out5)) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (every > 0 && c->b.nrep > 1) return CAVGPU_E_ARG;  // batches: cavgpu_thermo_batch after the call
   if (!c->set_up) return CAVGPU_E_STATE;
   if (nsteps == 0) return CAVGPU_OK;
@@ -1302,6 +1318,7 @@ int cavgpu_step(cavgpu_ctx *c, int64_t nsteps) { return cavgpu_run(c, nsteps, 0,
 int cavgpu_autotune(cavgpu_ctx *c, int32_t trial_steps, int32_t flags, int64_t *out6) {
   if (!c || trial_steps < 0) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->set_up) return CAVGPU_E_STATE;
   const int T = trial_steps > 0 ? trial_steps : 40;
   int dev = 0;
@@ -1469,6 +1486,7 @@ int cavgpu_autotune(cavgpu_ctx *c, int32_t trial_steps, int32_t flags, int64_t *
 int cavgpu_forces(cavgpu_ctx *c, double *virial, double *pe) {
   if (!c) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->set_up) return CAVGPU_E_STATE;
   const Status *h = nullptr;
   RK(build_and_force(c, &h));
@@ -1490,6 +1508,7 @@ int cavgpu_forces(cavgpu_ctx *c, double *virial, double *pe) {
 int cavgpu_thermo(cavgpu_ctx *c, double *out6) {
   if (!c || !out6) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->set_up) return CAVGPU_E_STATE;
   if (c->b.nrep > 1) return CAVGPU_E_ARG;  // cavgpu_thermo_batch
   const Status *h = nullptr;
@@ -1502,6 +1521,7 @@ int cavgpu_thermo(cavgpu_ctx *c, double *out6) {
 int cavgpu_thermo_batch(cavgpu_ctx *c, double *out6) {
   if (!c || !out6) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->set_up) return CAVGPU_E_STATE;
   const int R = c->b.nrep;
   if (R == 1) return cavgpu_thermo(c, out6);
@@ -1516,6 +1536,7 @@ int cavgpu_thermo_batch(cavgpu_ctx *c, double *out6) {
 int cavgpu_download(cavgpu_ctx *c, double *pos3, double *vel3, double *acc3) {
   if (!c) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->uploaded) return CAVGPU_E_STATE;
   // one kernel, the copies and one wait; the rebuild's scratch holds the host-order arrays
   // (24 of its 32 bytes per slot)
@@ -1534,6 +1555,7 @@ int cavgpu_download(cavgpu_ctx *c, double *pos3, double *vel3, double *acc3) {
 int cavgpu_download_images(cavgpu_ctx *c, int32_t *img3) {
   if (!c || !img3) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->uploaded || !c->d.img) return CAVGPU_E_STATE;
   RK(launch_images_to_host(c->d, c->b, c->st));
   CK(cudaMemcpyAsync(img3, c->d.hi3, 3 * sizeof(int32_t) * c->natoms, cudaMemcpyDeviceToHost, c->st));
@@ -1544,6 +1566,7 @@ int cavgpu_download_images(cavgpu_ctx *c, int32_t *img3) {
 int64_t cavgpu_export_pairs(cavgpu_ctx *c, int32_t *out5, int64_t cap) {
   if (!c || (cap > 0 && !out5) || c->b.nrep != 1) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->set_up) return CAVGPU_E_STATE;
   std::vector<int> nn(c->b.nslot);
   if (cudaMemcpyAsync(nn.data(), c->d.nnbr, c->b.nslot * sizeof(int), cudaMemcpyDeviceToHost, c->st) != cudaSuccess ||
@@ -1569,6 +1592,7 @@ int64_t cavgpu_export_pairs(cavgpu_ctx *c, int32_t *out5, int64_t cap) {
 int cavgpu_export_bins(cavgpu_ctx *c, int32_t *owned3, int32_t *nbins3) {
   if (!c || c->b.nrep != 1) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->uploaded) return CAVGPU_E_STATE;
   if (nbins3) for (int a = 0; a < 3; ++a) nbins3[a] = c->ref_nb[a];
   if (!owned3) return CAVGPU_OK;
@@ -1583,6 +1607,7 @@ int64_t cavgpu_export_ghosts(cavgpu_ctx *c, double ghost_cutoff, int32_t *src, i
                              int32_t *bins3, int64_t cap) {
   if (!c || ghost_cutoff < 0.0 || c->b.nrep != 1) return CAVGPU_E_ARG;
   std::lock_guard<std::recursive_mutex> call(c->mu);
+  if (c->stalled) return stall_rc();
   if (!c->uploaded) return CAVGPU_E_STATE;
   const int N = c->natoms;
   int *counts = nullptr, *starts = nullptr;

@@ -50,8 +50,13 @@ constexpr int MAX_REPLICAS = 6;
 // waits of boxes with 10^8 cells would run into the barrier's limit.)
 constexpr int MAX_CELLS = 12288;
 // polls of a barrier before a block gives up (seconds): the launch is cooperative, so a block
-// that never comes means a fault elsewhere; the host then reads F_STALL
-constexpr unsigned BARRIER_POLLS = 1u << 21;
+// that never comes means a fault elsewhere.  The state is then half way through a step: the
+// host reads F_STALL and the context does nothing more.  (No block goes on past a barrier
+// that another gave up unless all had reached it.)
+#ifndef CAV_BARRIER_POLLS
+#define CAV_BARRIER_POLLS (1u << 21)
+#endif
+constexpr unsigned BARRIER_POLLS = CAV_BARRIER_POLLS;
 
 struct ChunkArgs {
   Dev d;
@@ -287,7 +292,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 4) k_chunk(const __grid_constan
   __shared__ PhaseShared<MIXED> sh;
   __shared__ typename std::conditional<MIXED, SmemTabF, TabX<ONE ? 1 : MAXT * MAXT>>::type tab;
   __shared__ MassTab mtab;
-  if (halted(A.d)) return;  // a chunk after a halt does nothing (the same for every block)
+  if (halted(A.d) || stalled(A.d)) return;  // a chunk after a halt does nothing (the same for every block)
   Dev d = A.d;
   const Box &b = A.b;
   const StepConsts &sc = A.sc;
@@ -470,6 +475,7 @@ int launch_chunk(const Dev &d, const Box &b, const StepConsts &sc, const LaunchC
                  const FoldArgs &fa, cudaStream_t st) {
   if (lc.precision == CAVGPU_FP64 && (!lc.exchange || !d.recv)) return CAVGPU_E_ARG;
   ChunkArgs A{d, b, sc, fa, S, ev, fuse, drop, force_grid_blocks(lc), b.ncell_all, fuse == FUSE_LANG, lc.n <= BY_ATOM};
+  A.d.step_kernel = 1;
   const int want = std::max((lc.n + 32 / lc.tpa - 1) / (32 / lc.tpa), A.by_atom ? lc.n / CHUNK_WARPS : 0);
   const int kick = fuse == FUSE_LANG ? 2 : 1;
   const bool one = lc.ntypes == 1;

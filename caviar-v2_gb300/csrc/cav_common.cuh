@@ -201,6 +201,7 @@ struct Dev {
   int *flags;
   int *req, *nan;             // where a drift asks for a rebuild and reports a NaN (F_REBUILD, F_NAN of flags)
   unsigned int *barrier;      // grid barrier of the step kernel
+  int step_kernel;            // 1 in the step kernel's own copy (halted)
   int partials_alt;           // blocks after which the partial arrays' second halves begin (step kernel)
   double *partials_ke;        // per-block {sum m v^2, sum m v} (4 per block)
   double *partials_ke_end;    // Langevin: the same sums over the velocities at the end of the step
@@ -474,8 +475,13 @@ __device__ inline void nan_check(const Dev &d, int i, const dbl4 &a) {
   }
 }
 
-// the halt word as every thread of a kernel sees it (constant while kernels run)
-__device__ inline bool halted(const Dev &d) { return *(volatile const int *)&d.flags[F_HALT] != 0; }
+// The halt word as every thread of a kernel sees it (constant while kernels run).  After a
+// barrier that gave up kernels do nothing either; the step kernel, in which that word may
+// change, looks at it when it starts.
+__device__ inline bool stalled(const Dev &d) { return *(volatile const int *)&d.flags[F_STALL] != 0; }
+__device__ inline bool halted(const Dev &d) {
+  return *(volatile const int *)&d.flags[F_HALT] != 0 || (d.step_kernel == 0 && stalled(d));
+}
 
 // ---- host-side launch helpers ----------------------------------------------
 struct LaunchCfg {

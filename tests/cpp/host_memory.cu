@@ -133,6 +133,31 @@ int autotune() {
   return 0;
 }
 
+// a barrier of the step kernel gives up
+int stall() {
+  Md m(500, 64);
+  say("setup", m.rc);
+  fake::on_launch = [&](const std::string &name, void **args) {
+    if (is_chunk(name)) dev_of(args).flags[cav::F_STALL] = 1;
+  };
+  say("run", cavgpu_run(m.c, 200, 0, nullptr));
+  fake::on_launch = nullptr;
+  std::vector<double> a(1500);
+  int64_t st[8];
+  say("run_again", cavgpu_run(m.c, 1, 0, nullptr));
+  say("forces", cavgpu_forces(m.c, nullptr, nullptr));
+  say("thermo", cavgpu_thermo(m.c, a.data()));
+  say("download", cavgpu_download(m.c, a.data(), nullptr, nullptr));
+  say("setup_again", cavgpu_setup(m.c));
+  say("autotune", cavgpu_autotune(m.c, 0, 0, nullptr));
+  say("pairs", cavgpu_export_pairs(m.c, nullptr, 0));
+  say("named", std::strstr(cavgpu_last_cuda_error(), "barrier") != nullptr);
+  say("stats", cavgpu_stats(m.c, st));
+  Md n(500, 64);
+  say("other", n.rc ? n.rc : cavgpu_run(n.c, 10, 0, nullptr));
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -144,5 +169,6 @@ int main(int argc, char **argv) {
   if (what == "second_context") return second_context();
   if (what == "busy_context") return busy_context();
   if (what == "autotune") return autotune();
+  if (what == "stall") return stall();
   return 1;
 }

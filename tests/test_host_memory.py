@@ -1,4 +1,4 @@
-"""The library's host side when device memory runs short, without a GPU.
+"""The library's host side when device memory runs short or a kernel gives up, without a GPU.
 
 tests/cpp/host_memory.cu drives the C ABI with a stand-in for the CUDA runtime
 (tests/cpp/fake_cudart.cpp) whose memory has a limit and whose kernels do not run.
@@ -70,3 +70,12 @@ def test_autotune_takes_the_room_of_its_own_exchange_arrays(program):
     r = program("autotune")
     assert r["setup"] == 0 and r["exchange_before"] == 1
     assert r["autotune"] == 0 and r["run"] == 0 and r["nulls"] == 0
+
+
+def test_a_context_whose_barrier_gave_up_refuses_every_use_of_its_state(program):
+    r = program("stall")
+    assert r["setup"] == 0
+    for call in ("run", "run_again", "forces", "thermo", "download", "setup_again", "autotune", "pairs"):
+        assert r[call] == -2, call  # CAVGPU_E_CUDA
+    assert r["named"] == 1 and r["stats"] == 0
+    assert r["other"] == 0  # other contexts go on
