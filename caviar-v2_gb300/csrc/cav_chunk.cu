@@ -433,17 +433,14 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 4) k_chunk(const __grid_constan
 
 template <bool MIXED, int TPA, int KICK, bool ONE>
 int go(const ChunkArgs &A, int want, cudaStream_t st) {
-  static int per_sm = 0, sms = 0;
-  if (!per_sm) {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_chunk<MIXED, TPA, KICK, ONE>, CHUNK_THREADS, 0) != cudaSuccess ||
-        n < 1)
-      return CAVGPU_E_CUDA;
-    per_sm = n;
-  }
-  const int grid = std::max(1, std::min(want, sms * per_sm));
+  static PerDevice blocks_per_sm;  // resident
+  const int per_sm = blocks_per_sm.get([](int) {
+    int n = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_chunk<MIXED, TPA, KICK, ONE>, CHUNK_THREADS, 0);
+    return e == cudaSuccess && n > 0 ? n : -1;
+  });
+  if (per_sm < 1) return CAVGPU_E_CUDA;
+  const int grid = std::max(1, std::min(want, num_sms() * per_sm));
   void *args[] = {const_cast<ChunkArgs *>(&A)};
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_chunk<MIXED, TPA, KICK, ONE>), dim3(grid),
                                      dim3(CHUNK_THREADS), args, 0, st) == cudaSuccess

@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "cavgpu.h"
 
 namespace cav {
@@ -534,6 +536,22 @@ struct FoldArgs {
   int nb_ke, nb_ev, nb_ke_end, ring_slot;
 };
 
+// A number per device, found at first use; safe with several threads and devices.
+struct PerDevice {
+  static constexpr int MAX_DEVICES = 64;
+  std::atomic<int> v[MAX_DEVICES];
+  template <class F>
+  int get(F find) {  // find(device); its result is not 0
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= MAX_DEVICES) return find(dev);
+    int n = v[dev].load(std::memory_order_relaxed);
+    if (n == 0) v[dev].store(n = find(dev), std::memory_order_relaxed);
+    return n;
+  }
+};
+int num_sms();  // of the current device
+
 // Kernel launchers (cav_kernels.cu, cav_force.cu).  `forced` rebuilds every
 // replica regardless of the flags; otherwise the rebuild kernels skip replicas
 // whose half-skin test did not fire.
@@ -570,7 +588,7 @@ struct ForceArgs;
 int launch_exchange_build(const Dev &d, const Box &b, int forced, cudaStream_t st);
 int launch_force_exchange(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int kick, bool ev,
                           const ForceArgs &fa, int grid, int grid_ev, cudaStream_t st);
-int exchange_pair_blocks(int ntask, int sms);
+int exchange_pair_blocks(int ntask);
 int exchange_close_threads();
 int launch_force(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int kick, int thermo,
                  int k_in_chunk, int fuse, int set_cond, cudaGraphConditionalHandle cond, cudaStream_t st,

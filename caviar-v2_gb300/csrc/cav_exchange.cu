@@ -102,17 +102,6 @@ __global__ void __launch_bounds__(256) k_rank(Dev d, Box b, int forced) {
   if (j < b.nslot) rank_slot(d, b, forced, j);
 }
 
-int num_sms() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  return sms;
-}
-
 int exchange_run(int ntask) { return ntask >= num_sms() * MINB * 8 ? 4 : 1; }
 
 inline int chk() { return cudaPeekAtLastError() == cudaSuccess ? CAVGPU_OK : CAVGPU_E_CUDA; }
@@ -152,9 +141,9 @@ void both(int kick, bool ev, bool one, int grid, int grid_ev, const Dev &d, cons
 // instead of 731 FP64 instructions per task) once every warp has eight tasks; below that
 // the longer runs leave too few warps in flight.  131,072 atoms: 283 us with runs of one,
 // 293 with runs of four; 1,048,576 atoms: 1931 and 1867 (both kernels together).
-int exchange_pair_blocks(int ntask, int sms) {
+int exchange_pair_blocks(int ntask) {
   const int run = exchange_run(ntask);
-  return std::max(1, std::min((ntask + run - 1) / run, sms * MINB));
+  return std::max(1, std::min((ntask + run - 1) / run, num_sms() * MINB));
 }
 int exchange_close_threads() { return CLOSE_THREADS; }
 

@@ -447,17 +447,10 @@ int prepare_force_seg(size_t smem_bytes) {
   return CAVGPU_OK;
 }
 
-static int g_num_sms = 0;
-
 int force_grid_blocks(const LaunchCfg &lc) {
-  if (!g_num_sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g_num_sms <= 0) g_num_sms = 148;
-  }
+  const int sms = num_sms();
   if (segments_on(lc))  // one segment per block at a time
-    return lc.nseg < g_num_sms * 4 ? lc.nseg : g_num_sms * 4;
+    return lc.nseg < sms * 4 ? lc.nseg : sms * 4;
   const int A = 32 / lc.tpa, block = lc.exchange ? exchange_close_threads() : lc.block;
   const long long ntask = (lc.n + A - 1) / A;
   const long long warps_per_block = block / 32;
@@ -466,17 +459,16 @@ int force_grid_blocks(const LaunchCfg &lc) {
   // each warp walking its tasks grid-strided (fewer, longer-lived blocks: fewer block
   // reductions and tails; 5% less pair-kernel time and 16% less for the thermo
   // variant on the 1M-atom fluid than four waves); the FP64 kernels: four waves
-  const long long cap = lc.precision == CAVGPU_MIXED ? (long long)g_num_sms * (1024 / block)
-                                                     : (long long)g_num_sms * (2048 / block) * 4;
+  const long long cap = lc.precision == CAVGPU_MIXED ? (long long)sms * (1024 / block)
+                                                     : (long long)sms * (2048 / block) * 4;
   if (need > cap) need = cap;
   return (int)(need < 1 ? 1 : need);
 }
 
 int ev_grid_blocks(const LaunchCfg &lc) {
   if (!lc.exchange) return force_grid_blocks(lc);
-  force_grid_blocks(lc);  // (the SM count)
   const int A = 32 / lc.tpa;
-  return exchange_pair_blocks((lc.n + A - 1) / A, g_num_sms);
+  return exchange_pair_blocks((lc.n + A - 1) / A);
 }
 
 int launch_force(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int kick, int thermo,

@@ -11,15 +11,13 @@ namespace cav {
 
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
-static int num_sms() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  return sms;
+int num_sms() {
+  static PerDevice sms;
+  return sms.get([](int dev) {
+    int n = 0;
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 148;
+  });
 }
 
 // ---------------------------------------------------------------------------

@@ -12,11 +12,14 @@ namespace fake {
 size_t limit = (size_t)-1, used = 0, largest = 0;
 std::function<void(const std::string &, void **)> on_launch;
 std::map<std::string, int> launches;
+thread_local unsigned grid = 0;
+int device = 0, sms[2] = {152, 152};
 static std::map<const void *, std::string> names;
 static std::map<void *, size_t> blocks;
 static std::recursive_mutex mu;
 
-static cudaError_t launch(const void *func, void **args) {
+static cudaError_t launch(const void *func, void **args, dim3 g = dim3(0)) {
+  grid = g.x;
   std::string name = "?";
   {
     std::lock_guard<std::recursive_mutex> g(mu);
@@ -46,8 +49,8 @@ cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *m, void *s) {
   return cudaSuccess;
 }
 cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *f) { *k = (cudaKernel_t)f; return cudaSuccess; }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void **args, size_t, cudaStream_t) { return launch(k, args); }
-cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3, dim3, void **args, size_t, cudaStream_t) { return launch(f, args); }
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3, void **args, size_t, cudaStream_t) { return launch(k, args, g); }
+cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3 g, dim3, void **args, size_t, cudaStream_t) { return launch(f, args, g); }
 
 cudaError_t cudaMalloc(void **p, size_t n) {
   std::lock_guard<std::recursive_mutex> g(mu);
@@ -73,9 +76,9 @@ cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cu
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t) { memset(d, v, n); return cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t *f, size_t *t) { *t = (size_t)284 << 30; *f = limit - used; return cudaSuccess; }
-cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
-cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { *v = 152; return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int *n) { *n = 2; return cudaSuccess; }
+cudaError_t cudaGetDevice(int *d) { *d = device; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int d) { *v = sms[d]; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaPeekAtLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "fake"; }

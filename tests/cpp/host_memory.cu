@@ -1,6 +1,7 @@
 // host_memory.cu -- the library's host side when device memory runs short, on the CPU
 // (fake_cudart.cpp in place of the runtime).  Argument: the scenario.  Prints what the
 // Python side checks, as key value lines.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <random>
@@ -158,6 +159,30 @@ int stall() {
   return 0;
 }
 
+// the largest step-kernel grid of a run
+unsigned chunk_grid(cavgpu_ctx *c) {
+  unsigned g = 0;
+  fake::on_launch = [&](const std::string &name, void **) {
+    if (is_chunk(name)) g = std::max(g, fake::grid);
+  };
+  cavgpu_run(c, 100, 0, nullptr);
+  fake::on_launch = nullptr;
+  return g;
+}
+
+// contexts on two devices of different sizes
+int devices() {
+  fake::sms[1] = 10;
+  Md a(4000, 128, 20.0);
+  say("first", chunk_grid(a.c));
+  fake::device = 1;
+  Md b(4000, 128, 20.0);
+  say("second", chunk_grid(b.c));
+  fake::device = 0;
+  say("first_again", chunk_grid(a.c));
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -170,5 +195,6 @@ int main(int argc, char **argv) {
   if (what == "busy_context") return busy_context();
   if (what == "autotune") return autotune();
   if (what == "stall") return stall();
+  if (what == "devices") return devices();
   return 1;
 }

@@ -79,3 +79,10 @@ def test_a_context_whose_barrier_gave_up_refuses_every_use_of_its_state(program)
         assert r[call] == -2, call  # CAVGPU_E_CUDA
     assert r["named"] == 1 and r["stats"] == 0
     assert r["other"] == 0  # other contexts go on
+
+
+def test_the_step_kernels_grid_fits_the_device_it_runs_on(program):
+    """Blocks of a cooperative launch must all be resident: four per multiprocessor here."""
+    r = program("devices")
+    assert r["second"] <= 10 * 4 < r["first"] <= 152 * 4
+    assert r["first_again"] == r["first"]
