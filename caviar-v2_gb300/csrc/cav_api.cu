@@ -169,6 +169,16 @@ void give_back(cavgpu_ctx *c) {
 std::mutex g_ctx_mu;
 std::vector<cavgpu_ctx *> g_ctx;
 
+// Calls at work on a device's steps (any context, any thread): what the step kernel's grid
+// allows for.  Results do not depend on it.
+struct AtWork {
+  static std::atomic<int> count[PerDevice::MAX_DEVICES];
+  std::atomic<int> &n;
+  explicit AtWork(int dev) : n(count[dev >= 0 && dev < PerDevice::MAX_DEVICES ? dev : 0]) { ++n; }
+  ~AtWork() { --n; }
+};
+std::atomic<int> AtWork::count[PerDevice::MAX_DEVICES];
+
 // device memory that the context cannot do without
 cudaError_t must_malloc(cavgpu_ctx *c, void **q, size_t bytes) {
   cudaError_t e = cudaMalloc(q, bytes);
@@ -1093,6 +1103,7 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
   const bool eager = c->p.steps_per_graph < 0;
   // small systems: a chunk's steps in one launch (cav_chunk.cu); not while kernel times are
   // taken, nor with constraint::Nve between the steps
+  const AtWork at_work(c->dev);
   auto step_kernel = [&] { return !eager && !c->prof && c->nve.step == 0 && chunk_fits(c->b, c->lc); };
   bool small = step_kernel();
   RK(ensure_status(c));
@@ -1128,7 +1139,7 @@ int run_steps(cavgpu_ctx *c, int64_t nsteps, int64_t every, double *out5) {
       if (small && (ev == 0 || c->b.nrep == 1)) {
         plan = plan_of(c, sz, ev);
         const FoldArgs fa = fold_args(c, 0);
-        RK(launch_chunk(c->d, c->b, c->sc, c->lc, sz, ev, fuse_mode(c), plan->dropped, fa, c->st));
+        RK(launch_chunk(c->d, c->b, c->sc, c->lc, sz, ev, fuse_mode(c), plan->dropped, fa, at_work.n, c->st));
         c->kernel_launches += 1;
       } else if (!eager) {
         int rc = CAVGPU_OK;

@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 4) k_chunk(const __grid_constan
 }
 
 template <bool MIXED, int TPA, int KICK, bool ONE>
-int go(const ChunkArgs &A, int want, cudaStream_t st) {
+int go(const ChunkArgs &A, int want, int share, cudaStream_t st) {
   static PerDevice blocks_per_sm;  // resident
   const int per_sm = blocks_per_sm.get([](int) {
     int n = 0;
@@ -440,7 +440,12 @@ int go(const ChunkArgs &A, int want, cudaStream_t st) {
     return e == cudaSuccess && n > 0 ? n : -1;
   });
   if (per_sm < 1) return CAVGPU_E_CUDA;
-  const int grid = std::max(1, std::min(want, num_sms() * per_sm));
+  // Contexts stepped at the same time (threads) divide the blocks that can be resident: a
+  // launch whose blocks do not fit beside the running ones waits for them to end.  Time per
+  // step and context of 4 contexts of 4,000 atoms, each on its own / sharing / as graphs of
+  // kernels, which overlap: mixed 14.8 / 3.9 / 8.0 us, FP64 35.5 / 17.8 / 20.8; of 19,652 atoms mixed
+  // 18.7 / 10.0 / 11.8; of 8 contexts of 48,668 mixed 33.1 / 20.9 / 21.9.
+  const int grid = std::max(1, std::min(want, num_sms() * per_sm / std::min(std::max(share, 1), 4)));
   void *args[] = {const_cast<ChunkArgs *>(&A)};
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_chunk<MIXED, TPA, KICK, ONE>), dim3(grid),
                                      dim3(CHUNK_THREADS), args, 0, st) == cudaSuccess
@@ -449,9 +454,9 @@ int go(const ChunkArgs &A, int want, cudaStream_t st) {
 }
 
 template <bool MIXED, int TPA>
-int pick(const ChunkArgs &A, int kick, bool one, int want, cudaStream_t st) {
-  if (kick == 1) return one ? go<MIXED, TPA, 1, true>(A, want, st) : go<MIXED, TPA, 1, false>(A, want, st);
-  return one ? go<MIXED, TPA, 2, true>(A, want, st) : go<MIXED, TPA, 2, false>(A, want, st);
+int pick(const ChunkArgs &A, int kick, bool one, int want, int share, cudaStream_t st) {
+  if (kick == 1) return one ? go<MIXED, TPA, 1, true>(A, want, share, st) : go<MIXED, TPA, 1, false>(A, want, share, st);
+  return one ? go<MIXED, TPA, 2, true>(A, want, share, st) : go<MIXED, TPA, 2, false>(A, want, share, st);
 }
 
 }  // namespace
@@ -469,16 +474,24 @@ bool chunk_fits(const Box &b, const LaunchCfg &lc) {
 }
 
 int launch_chunk(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int S, int ev, int fuse, int drop,
-                 const FoldArgs &fa, cudaStream_t st) {
+                 const FoldArgs &fa, int share, cudaStream_t st) {
   if (lc.precision == CAVGPU_FP64 && (!lc.exchange || !d.recv)) return CAVGPU_E_ARG;
   ChunkArgs A{d, b, sc, fa, S, ev, fuse, drop, force_grid_blocks(lc), b.ncell_all, fuse == FUSE_LANG, lc.n <= BY_ATOM};
   A.d.step_kernel = 1;
-  const int want = std::max((lc.n + 32 / lc.tpa - 1) / (32 / lc.tpa), A.by_atom ? lc.n / CHUNK_WARPS : 0);
+  // Mixed: four lanes a task per warp and a block per multiprocessor at least (4,000 atoms 12.4
+  // us a step, with a block per task 13.4, with a warp per atom 14.9: more blocks to wait for
+  // at every barrier), two lanes, whose systems are larger, a block per task (32,000 atoms 22.75
+  // against 23.03).  FP64: a block per task, a warp per atom where those evaluate the pairs (the
+  // FP64 pipe is an SM's own: 1,372 atoms 24.5 us, with a task per warp 27.6).
+  const int ntask = (lc.n + 32 / lc.tpa - 1) / (32 / lc.tpa);
+  const int want = lc.precision == CAVGPU_FP64 ? std::max(ntask, A.by_atom ? lc.n / CHUNK_WARPS : 0)
+                   : lc.tpa == 4 ? std::max((ntask + CHUNK_WARPS - 1) / CHUNK_WARPS, std::min(ntask, num_sms()))
+                                 : ntask;
   const int kick = fuse == FUSE_LANG ? 2 : 1;
   const bool one = lc.ntypes == 1;
   if (lc.precision == CAVGPU_MIXED)
-    return lc.tpa == 2 ? pick<true, 2>(A, kick, one, want, st) : pick<true, 4>(A, kick, one, want, st);
-  return pick<false, 4>(A, kick, one, want, st);
+    return lc.tpa == 2 ? pick<true, 2>(A, kick, one, want, share, st) : pick<true, 4>(A, kick, one, want, share, st);
+  return pick<false, 4>(A, kick, one, want, share, st);
 }
 
 }  // namespace cav

@@ -604,10 +604,10 @@ int launch_thermo_replicas(const Dev &d, const Box &b, const ThermoCfg &tc, int 
 int launch_advance_step(const Dev &d, cudaStream_t st);
 // Small systems: S steps in one cooperative launch (cav_chunk.cu).  fuse: Fuse of the steps
 // that drift the next one (rule of ChunkPlan; `drop` = the step kept from it, -1: none),
-// ev: record period; fa: the fold of a recorded step.
+// ev: record period; fa: the fold of a recorded step; share: contexts at work on the device.
 bool chunk_fits(const Box &b, const LaunchCfg &lc);
 int launch_chunk(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int S, int ev, int fuse, int drop,
-                 const FoldArgs &fa, cudaStream_t st);
+                 const FoldArgs &fa, int share, cudaStream_t st);
 // constraint::Nve: kinetic energy, lambda (and the thermo point of the step,
 // ring_slot >= 0 or the current one when thermo != 0), velocity scaling; every
 // kernel returns at once unless (step_base + k) % cfg.step == 0
