@@ -90,6 +90,7 @@ struct cavgpu_ctx {
   long long steps_done = 0;
   long long graph_launches = 0, kernel_launches = 0;
   int max_nb = 0;
+  double row_mean = 0.0;  // list words per atom of the densest replica, were its density even
   std::deque<GraphEntry> graphs;                      // stable references (chunks in flight hold them)
   std::map<std::pair<int, int>, ChunkPlan> eager_plans;  // chunks that are not graphs
   // the status block (thermo and flags, adjacent on the device) in pinned memory: two copies
@@ -509,8 +510,13 @@ int alloc_exchange(cavgpu_ctx *c) {
   return CAVGPU_OK;
 }
 
+// the launches' idea of the row length: the even density's, or three quarters of the longest
+// row (a liquid's longest is 1.3 times its mean) where the system is denser in places
+void note_rows(cavgpu_ctx *c) { c->lc.row = (int)std::max(c->row_mean, 0.75 * c->max_nb); }
+
 // (re)allocate the neighbour list for `cap` slots per atom
 int alloc_nbr(cavgpu_ctx *c, int cap) {
+  note_rows(c);
   cap = (cap + 63) / 64 * 64;  // nbr_index needs cap % (4 * tpa) == 0, tpa <= 16
   const int A = 32 / c->d.tpa;  // whole blocks of A slots (nbr_index)
   const size_t bytes = (size_t)((c->b.nslot + A - 1) / A) * A * (size_t)cap * sizeof(uint32_t);
@@ -892,6 +898,11 @@ int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, cons
   c->natoms = N;
   c->sc.n = NS;
   c->lc.n = NS;
+  double rho = 0.0;  // of the densest replica
+  for (const RepBox &rb : c->reps) rho = std::max(rho, rb.natoms / (rb.L[0] * rb.L[1] * rb.L[2]));
+  const double ce = c->cutoff_extra;
+  c->row_mean = rho * 4.18879020479 * ce * ce * ce;
+  note_rows(c);
   if (!c->p.threads_per_atom) c->lc.tpa = c->d.tpa = default_tpa(NS);
   c->tc.n = N;
   c->tc.n_r_df = c->p.n_r_df;
@@ -996,9 +1007,6 @@ int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, cons
   CK(cudaMemcpyAsync(drep, c->reps.data(), R * sizeof(RepBox), cudaMemcpyHostToDevice, c->st));
   CK(cudaMemsetAsync(dflag, 0, R * sizeof(int), c->st));
   // initial capacity from the densest replica: 1.4 x the mean count in the cutoff sphere, plus headroom
-  double rho = 0.0;
-  for (const RepBox &rb : c->reps) rho = std::max(rho, rb.natoms / (rb.L[0] * rb.L[1] * rb.L[2]));
-  const double ce = c->cutoff_extra;
   const int cap = c->p.nbr_capacity > 0 ? c->p.nbr_capacity : (int)(1.4 * rho * 4.18879020479 * ce * ce * ce) + 48;
   RK(alloc_nbr(c, cap));
   if (on_device) {
@@ -1046,6 +1054,7 @@ int setup_common(cavgpu_ctx *c) {
   if (!c->uploaded) return CAVGPU_E_STATE;
   const Status *h = nullptr;
   RK(build_and_force(c, &h));
+  note_rows(c);
   c->set_up = true;
   return CAVGPU_OK;
 }

@@ -66,6 +66,7 @@ struct ChunkArgs {
   int S, ev, fuse, drop;
   int nblk;        // virtual blocks of the force phase on recorded steps (the kernels' grid)
   int ncell, lang;
+  int shared;      // windows shared by a block's warps (shared_windows)
   int by_atom;     // FP64 form: a warp per atom evaluates the pairs (few atoms)
 };
 
@@ -143,7 +144,8 @@ __device__ __noinline__ bool rebuild(const ChunkArgs &A, int4 *ic, PhaseShared<M
   if (!grid_barrier(d)) return false;
   for (int c = warp; c < A.ncell; c += nwarp) rebuild_sort_gather(d, b, 0, c);
   if (!grid_barrier(d)) return false;
-  rebuild_build<MIXED ? 1 : 0, true>(d, b, 0, sh.build.stage[wid], blockIdx.x, gridDim.x, &sh.build);
+  if (A.shared) rebuild_build<MIXED ? 1 : 0, true>(d, b, 0, sh.build.stage[wid], blockIdx.x, gridDim.x, &sh.build);
+  else rebuild_build<MIXED ? 1 : 0, false>(d, b, 0, sh.build.stage[wid], warp, nwarp, nullptr);
   if (!grid_barrier(d)) return false;
   if (!MIXED) {
     for (int i = warp; i < b.nslot; i += nwarp) claim_slot(d, b, 0, i);
@@ -476,7 +478,7 @@ bool chunk_fits(const Box &b, const LaunchCfg &lc) {
 int launch_chunk(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int S, int ev, int fuse, int drop,
                  const FoldArgs &fa, int share, cudaStream_t st) {
   if (lc.precision == CAVGPU_FP64 && (!lc.exchange || !d.recv)) return CAVGPU_E_ARG;
-  ChunkArgs A{d, b, sc, fa, S, ev, fuse, drop, force_grid_blocks(lc), b.ncell_all, fuse == FUSE_LANG, lc.n <= BY_ATOM};
+  ChunkArgs A{d, b, sc, fa, S, ev, fuse, drop, force_grid_blocks(lc), b.ncell_all, fuse == FUSE_LANG, shared_windows(lc), lc.n <= BY_ATOM};
   A.d.step_kernel = 1;
   // Mixed: four lanes a task per warp and a block per multiprocessor at least (4,000 atoms 12.4
   // us a step, with a block per task 13.4, with a warp per atom 14.9: more blocks to wait for

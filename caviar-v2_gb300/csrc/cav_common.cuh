@@ -495,6 +495,7 @@ struct LaunchCfg {
   int use_seg;     // mixed form: run the segment kernel (shared-memory stage)
   int ntypes;      // 1: the kernels keep the pair constants in registers
   int exchange;    // FP64 form: pairs evaluated once, two kernels per force (cav_exchange.cu)
+  int row;         // list words of an atom in the denser part of the system, about
   int images;      // mixed form: the list holds image codes, applied by the pair kernel (RepBox::flip)
 };
 // the list words of the mixed form hold stencil indices, else image codes

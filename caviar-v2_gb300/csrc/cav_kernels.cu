@@ -705,7 +705,7 @@ int launch_rebuild(const Dev &d, const Box &b, const LaunchCfg &lc, int forced, 
   // so every sixth, so the line lies further up: a step of 56 replicas (1,900 windows) takes 89
   // us with four warps per window and 138 with one, of 128 (4,900) 137 and 178, but of 256
   // large ones (34,900) 511 and 426.
-  if (windows <= num_sms() * SHARED_WINDOWS * (batch && !forced ? 8 : 1)) {
+  if (shared_windows(lc) && windows <= num_sms() * SHARED_WINDOWS * (batch && !forced ? 8 : 1)) {
     if (stencil_codes(lc)) k_build_shared<1><<<windows * split, 128, 0, st>>>(d, b, forced, split);
     else k_build_shared<0><<<windows * split, 128, 0, st>>>(d, b, forced, split);
   } else if (stencil_codes(lc)) k_build_group<1><<<build_grid, BUILD_WARPS * 32, 0, st>>>(d, b, forced);

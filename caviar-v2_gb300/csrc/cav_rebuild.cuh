@@ -397,13 +397,19 @@ struct BuildStage {
 // candidates' rows, about balanced by the candidates that survive the culling; the first
 // writes its hits straight to the list rows, the others keep theirs in shared memory and
 // move them behind those of the parts before.  An atom with more hits in a part than fit
-// there sends the window to one warp.
+// there sends the window to one warp.  Not where rows are so long that every window would
+// end there, after the four warps' work (shared_windows).
 struct BuildShare {
   BuildStage stage[4];
   uint32_t hits[3][SEG_HITS * 32];
   int cnt[4][32];
 };
 __constant__ const int8_t PART_ROWS[5] = {0, 2, 5, 7, 9};  // of ROW_ORDER
+
+// Step mixed, shared and not: rows of 127 words 4,000 atoms 14.5 and 19.8 us, 32,000 atoms 27.3 and
+// 31.2; of 139 words 23.4 and 23.0, 42.1 and 34.3; of 179 words 28.4 and 25.0, 58.2 and 37.9.
+constexpr int SHARED_ROW = 132;
+inline bool shared_windows(const LaunchCfg &lc) { return lc.row <= SHARED_ROW; }
 
 // SHARED false: warp gw of nw takes the windows gw, gw + nw, ...; true: block gw of nw, the
 // warps of a block (four) the parts of its windows.  split > 1: the groups of a window are
