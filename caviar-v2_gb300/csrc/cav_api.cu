@@ -821,7 +821,14 @@ int build_segments(cavgpu_ctx *c) {
 // of 19,652 34.0 and 31.8, of 23,328 34.3 and 32.6, in FP64 of 19,652 85.4 and 83.8.  Two up
 // to 49,152 slots: 42,592 atoms mixed with 2 and 1 lanes 36.6 and 41.9, 55,296 44.7 and 44.9,
 // 62,500 47.8 and 45.0; in FP64 55,296 187 and 164.  8 lanes gain under 2% on the smallest.
-int default_tpa(int nslot) { return nslot >= 49152 ? 1 : nslot > 19456 ? 2 : 4; }
+// Mixed rows of more than 200 words keep two lanes up to 65,536 slots: 55,296 atoms with 281 words
+// per row mixed 82.1 us with one lane and 73.0 with two, with 526 words 147 and 122; 78,732 atoms
+// 98.6 and 104, 166 and 174.  Those of more than 600 words keep four up to 38,912 slots: 970 words,
+// 32,000 atoms 120 us with two lanes and 108 with four, 42,592 atoms 152 and 160.  (FP64, 55,296
+// atoms, 382 words: 465 us with one lane, 524 with two.)
+int default_tpa(int nslot, int mixed_row) {
+  return nslot >= (mixed_row > LONG_ROW ? 65536 : 49152) ? 1 : nslot > (mixed_row > 600 ? 38912 : 19456) ? 2 : 4;
+}
 
 // Lay the replicas out (32-aligned slot ranges, consecutive cell ranges with one
 // padding cell each), allocate every per-slot array and upload the atoms.
@@ -903,7 +910,7 @@ int upload_common(cavgpu_ctx *c, const int64_t *counts, const double *pos3, cons
   const double ce = c->cutoff_extra;
   c->row_mean = rho * 4.18879020479 * ce * ce * ce;
   note_rows(c);
-  if (!c->p.threads_per_atom) c->lc.tpa = c->d.tpa = default_tpa(NS);
+  if (!c->p.threads_per_atom) c->lc.tpa = c->d.tpa = default_tpa(NS, c->p.precision == CAVGPU_MIXED ? c->lc.row : 0);
   c->tc.n = N;
   c->tc.n_r_df = c->p.n_r_df;
   c->tc.k_b = c->p.k_b;

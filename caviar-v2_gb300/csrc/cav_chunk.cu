@@ -471,6 +471,11 @@ bool chunk_fits(const Box &b, const LaunchCfg &lc) {
   if (lc.use_seg || lc.block != CHUNK_THREADS || (lc.tpa != 2 && lc.tpa != 4)) return false;
   if (lc.precision == CAVGPU_FP64 && (!lc.exchange || lc.tpa != 4 || lc.n > FP64_ATOMS)) return false;
   const int ntask = (lc.n + 32 / lc.tpa - 1) / (32 / lc.tpa);
+  // Long rows: no more than a task per resident warp, 16 per SM; the kernels keep twice the warps
+  // in flight.  Mixed, 281 words per row, 32,000 and 42,592 atoms 53.0 and 74.0 us here, 62.8 and
+  // 70.8 with kernels; 526 words 85.7 and 140 against 95.9 and 118; 127 words 28.2 and 39.9
+  // against 37.0 and 44.7.
+  if (lc.precision == CAVGPU_MIXED && lc.row > LONG_ROW && ntask > num_sms() * 16) return false;
   if (force_grid_blocks(lc) * CHUNK_WARPS < ntask) return false;
   return !lc.exchange || ev_grid_blocks(lc) >= ntask;
 }

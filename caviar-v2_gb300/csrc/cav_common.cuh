@@ -498,6 +498,7 @@ struct LaunchCfg {
   int row;         // list words of an atom in the denser part of the system, about
   int images;      // mixed form: the list holds image codes, applied by the pair kernel (RepBox::flip)
 };
+constexpr int LONG_ROW = 200;
 // the list words of the mixed form hold stencil indices, else image codes
 inline bool stencil_codes(const LaunchCfg &lc) { return lc.precision == CAVGPU_MIXED && !lc.images; }
 // the segment kernel runs (its table lookups need stencil indices)

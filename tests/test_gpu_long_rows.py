@@ -1,7 +1,8 @@
 """Systems with long list rows: list cutoffs or densities beyond the usual.
 
 Rows of more than 132 words are built by one warp per window, where shared windows would
-overflow their parts.
+overflow their parts; rows of more than 200 keep two lanes per atom up to 65,536 slots and the
+step kernel to one task per resident warp, rows of more than 600 four lanes up to 38,912.
 """
 import numpy as np
 import pytest
@@ -53,15 +54,27 @@ def test_dense_lists_against_brute_force(rho, voids, precision):
     np.testing.assert_array_equal(got, brute_pairs(pos, L, p["nl_cutoff"] * p["nl_coef"]))
 
 
-@pytest.mark.parametrize("cells,rc", [(10, 3.5), (10, 4.0), (19, 4.0), (22, 3.0)])
-def test_steps_equal_single_kernels(cells, rc):
+# 10 and 19 cells: the step kernel; 22 cells with rows of 281 words: more tasks than resident warps
+@pytest.mark.parametrize("cells,rc,graphs", [(10, 3.5, False), (10, 4.0, False), (19, 4.0, False), (22, 4.0, True),
+                                             (22, 3.0, False)])
+def test_steps_equal_single_kernels(cells, rc, graphs):
     system, out = fluid(cells, rc), []
     for spg in (0, -1):
         s = G.System(*system, precision=G.MIXED, steps_per_graph=spg)
         s.setup()
         rec = s.run(30, 6)
         out.append((rec, *s.state()))
+        if spg == 0:
+            assert (s.stats()["graph_launches"] > 0) == graphs
         assert s.stats()["rebuilds"] > 1
         s.close()
     for x, y in zip(*out):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("cells,rc,lanes", [(16, 4.0, 4), (22, 4.0, 2), (24, 2.5, 1), (24, 4.0, 2), (26, 4.0, 1), (19, 6.0, 4),
+                                            (22, 6.0, 2)])
+def test_default_lanes(cells, rc, lanes):
+    s = G.System(*fluid(cells, rc), precision=G.MIXED)
+    assert s.stats()["threads_per_atom"] == lanes
+    s.close()
