@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <deque>
 #include <map>
@@ -462,9 +463,10 @@ int read_flags(cavgpu_ctx *c, int *f) {
 
 // zeroes every status word but the rebuild counts and the step kernel's phase
 int clear_status(cavgpu_ctx *c) {
-  static_assert(F_REBUILDS == 5 && F_PASSES == 6 && F_HALT == 7 && F_PHASE_REQ == 12, "word order");
+  static_assert(F_REBUILDS == 5 && F_PASSES == 6 && F_PHASE == 18, "word order");
+  static_assert(offsetof(Status, flags) % 8 == 0, "halted() reads a pair of words");
   CK(cudaMemsetAsync(c->d.flags, 0, F_REBUILDS * sizeof(int), c->st));
-  CK(cudaMemsetAsync(c->d.flags + F_HALT, 0, (F_PHASE - F_HALT) * sizeof(int), c->st));
+  CK(cudaMemsetAsync(c->d.flags + F_PASSES + 1, 0, (F_PHASE - F_PASSES - 1) * sizeof(int), c->st));
   return CAVGPU_OK;
 }
 

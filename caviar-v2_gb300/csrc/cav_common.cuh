@@ -85,13 +85,15 @@ enum Flag : int {
   // (the condition kernel, the pair kernel's last block, the end of a rebuild), so
   // that it is constant while any kernel runs; every step kernel that starts with
   // it raised returns at once, and the rest of the chunk does nothing.
-  F_HALT = 7,
+  // (with F_STALL in one aligned pair of words: halted)
+  F_HALT = 10,
+  F_STALL = 11,     // a grid barrier of the step kernel gave up
+  F_UPLOAD_BAD = 7,  // an uploaded atom outside the box, of an unknown type or with a bad id
   F_STEPS_OK = 8,   // steps of the current chunk whose pair kernel ran (the step counter adds them)
   F_HALT_STEP = 9,  // steps of the halted chunk that completed before the halt
-  F_UPLOAD_BAD = 10,  // an uploaded atom outside the box, of an unknown type or with a bad id
   // the step kernel of small systems (cav_chunk.cu): rebuild requests and NaNs by phase,
-  // the phase, a barrier that gave up
-  F_PHASE_REQ = 12, F_PHASE_NAN = 15, F_PHASE = 18, F_STALL = 19,
+  // the phase
+  F_PHASE_REQ = 12, F_PHASE_NAN = 15, F_PHASE = 18,
   F_NWORDS = 20
 };
 
@@ -481,8 +483,10 @@ __device__ inline void nan_check(const Dev &d, int i, const dbl4 &a) {
 // barrier that gave up kernels do nothing either; the step kernel, in which that word may
 // change, looks at it when it starts.
 __device__ inline bool stalled(const Dev &d) { return *(volatile const int *)&d.flags[F_STALL] != 0; }
-__device__ inline bool halted(const Dev &d) {
-  return *(volatile const int *)&d.flags[F_HALT] != 0 || (d.step_kernel == 0 && stalled(d));
+__device__ inline bool halted(const Dev &d) {  // one load: every thread of a rebuild kernel starts with it
+  static_assert(F_HALT % 2 == 0 && F_STALL == F_HALT + 1, "one aligned pair");
+  const unsigned long long both = *(volatile const unsigned long long *)&d.flags[F_HALT];
+  return d.step_kernel ? (unsigned)both != 0u : both != 0ull;
 }
 
 // ---- host-side launch helpers ----------------------------------------------
