@@ -95,8 +95,10 @@ struct cavgpu_ctx {
   std::deque<GraphEntry> graphs;                      // stable references (chunks in flight hold them)
   std::map<std::pair<int, int>, ChunkPlan> eager_plans;  // chunks that are not graphs
   // the status block (thermo and flags, adjacent on the device) in pinned memory: two copies
-  // for the chunks in flight, read back without a full synchronisation, one for other reads
+  // for the chunks in flight, read back without a full synchronisation, one for other reads;
+  // from the first run on (allocating and freeing it takes 300 us), before that `status`
   Status *h_status = nullptr;
+  Status status{};
   bool nan_seen = false;     // F_NAN and F_PASSES of the last status read
   int passes = 0;
   cudaEvent_t ev_status[2] = {nullptr, nullptr};
@@ -444,8 +446,7 @@ int ensure_status(cavgpu_ctx *c) {
 
 // the status block as it is once the stream has done its work (one copy, one wait)
 int read_status(cavgpu_ctx *c, const Status **out) {
-  RK(ensure_status(c));
-  Status *h = c->h_status + 2;
+  Status *h = c->h_status ? c->h_status + 2 : &c->status;
   CK(cudaMemcpyAsync(h, c->d.thermo, sizeof(Status), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
   c->nan_seen = h->flags[F_NAN] != 0;

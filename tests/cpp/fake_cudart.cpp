@@ -13,6 +13,7 @@ size_t limit = (size_t)-1, used = 0, largest = 0;
 std::function<void(const std::string &, void **)> on_launch;
 std::map<std::string, int> launches;
 thread_local unsigned grid = 0;
+int pinned = 0;
 int device = 0, sms[2] = {152, 152};
 static std::map<const void *, std::string> names;
 static std::map<void *, size_t> blocks;
@@ -70,7 +71,7 @@ cudaError_t cudaFree(void *p) {
   free(p);
   return cudaSuccess;
 }
-cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { *p = calloc(1, n); return cudaSuccess; }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { ++pinned; *p = calloc(1, n); return cudaSuccess; }
 cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }

@@ -12,5 +12,6 @@ extern size_t limit, used, largest;  // device memory: most that may be in use, 
 extern std::function<void(const std::string &, void **)> on_launch;
 extern std::map<std::string, int> launches;  // by name; "?" for graphs
 extern thread_local unsigned grid;           // blocks of the launch that the hook sees
+extern int pinned;                           // pinned allocations so far
 extern int device, sms[2];                   // current device, multiprocessors of each
 }  // namespace fake

@@ -183,6 +183,16 @@ int devices() {
   return 0;
 }
 
+// what a context that only evaluates forces pins
+int pinned() {
+  Md m(500, 64);
+  say("forces", cavgpu_forces(m.c, nullptr, nullptr));
+  say("before", fake::pinned);
+  say("run", cavgpu_run(m.c, 10, 0, nullptr));
+  say("after", fake::pinned);
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -196,5 +206,6 @@ int main(int argc, char **argv) {
   if (what == "autotune") return autotune();
   if (what == "stall") return stall();
   if (what == "devices") return devices();
+  if (what == "pinned") return pinned();
   return 1;
 }

@@ -86,3 +86,9 @@ def test_the_step_kernels_grid_fits_the_device_it_runs_on(program):
     r = program("devices")
     assert r["second"] <= 10 * 4 < r["first"] <= 152 * 4
     assert r["first_again"] == r["first"]
+
+
+def test_pinned_memory_is_taken_by_the_first_run(program):
+    r = program("pinned")
+    assert r["forces"] == 0 and r["run"] == 0
+    assert r["before"] == 0 and r["after"] == 1
