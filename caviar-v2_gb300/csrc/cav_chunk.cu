@@ -31,11 +31,8 @@ namespace {
 
 constexpr int CHUNK_THREADS = 128;
 constexpr int CHUNK_WARPS = CHUNK_THREADS / 32;
-// FP64 form: a warp per atom for the pairs up to BY_ATOM atoms (step of 500, 1,372, 4,000 and
-// 8,788 atoms 24, 28, 39 and 59 us, with four lanes per atom 39, 39, 44 and 53), the step kernel
-// up to FP64_ATOMS (19,652 atoms: 102 us against 95 in a graph, whose pair kernel has more
-// warps in flight)
-constexpr int BY_ATOM = 6144;
+// FP64 form: the step kernel up to FP64_ATOMS (19,652 atoms: 102 us against 95 in a graph, whose
+// pair kernel has more warps in flight)
 constexpr int FP64_ATOMS = 12288;
 // With more than a few replicas one rebuilds in nearly every step, and the kernels' rebuild,
 // with more blocks than stay resident, takes less time: step of 4 replicas (4,900 slots) mixed

@@ -5,7 +5,8 @@
 // work taken off it counts and little else does.  A step is two kernels:
 //   k_pairs64  every pair is claimed by one of its two atoms (claims()).  An atom walks the
 //              entries it claimed, evaluates those inside the cutoff, adds the force to its
-//              own sum and stores the opposite force in a slot of the other atom's;
+//              own sum and stores the opposite force in a slot of the other atom's (systems
+//              of few atoms: k_atoms64, a warp per atom);
 //   k_close64  every atom adds the forces it received to its own sum, in a fixed order,
 //              then does the closing update of the step and the next drift.
 // Which pairs are near the cutoff is decided off the FP64 pipe, on FP32 differences of
@@ -56,6 +57,20 @@ __global__ void __launch_bounds__(32, MINB) k_pairs64(Dev d, Box b, StepConsts s
     }
   }
   if (EV) block_sum_store_f<2>(ev_p, &d.partials_ev[(size_t)blockIdx.x * 2]);
+}
+
+// Few atoms: a warp each, unless virial and energy are wanted.  A step as a graph of kernels
+// (constraint::Nve) of 500 / 4,000 atoms: 39.8 / 54.7 us, with k_pairs64 54.9 / 59.0.
+constexpr int ATOM_WARPS = 4;
+template <bool ONE>
+__global__ void __launch_bounds__(32 * ATOM_WARPS) k_atoms64(Dev d, Box b, StepConsts sc) {
+  __shared__ TabX<ONE ? 1 : MAXT * MAXT> tab;
+  __shared__ double share[ATOM_WARPS][32][3];
+  if (halted(d)) return;
+  load_tabx<false, ONE>(d, tab);
+  __syncthreads();
+  const int i = blockIdx.x * ATOM_WARPS + (threadIdx.x >> 5);
+  if (i < sc.n) pair_atom<ONE>(d, b, sc, tab, share[threadIdx.x >> 5], d.tab->nt, i);
 }
 
 // Received forces, closing update, the end of the step.
@@ -129,7 +144,13 @@ void both(int kick, bool ev, bool one, int grid, int grid_ev, const Dev &d, cons
           const ForceArgs &fa, cudaStream_t st) {
   constexpr int A = 32 / TPA;
   const int run = exchange_run((sc.n + A - 1) / A);
-  pairs<TPA>(ev, one, grid_ev, run, d, b, sc, st);
+  if (!ev && sc.n <= BY_ATOM) {
+    const int blocks = (sc.n + ATOM_WARPS - 1) / ATOM_WARPS;
+    if (one) k_atoms64<true><<<blocks, 32 * ATOM_WARPS, 0, st>>>(d, b, sc);
+    else k_atoms64<false><<<blocks, 32 * ATOM_WARPS, 0, st>>>(d, b, sc);
+  } else {
+    pairs<TPA>(ev, one, grid_ev, run, d, b, sc, st);
+  }
   if (kick == 0) close_kick<TPA, 0>(ev, grid, d, b, sc, fa, st);
   else if (kick == 1) close_kick<TPA, 1>(ev, grid, d, b, sc, fa, st);
   else close_kick<TPA, 2>(ev, grid, d, b, sc, fa, st);
