@@ -63,7 +63,6 @@ struct ChunkArgs {
   int S, ev, fuse, drop;
   int nblk;        // virtual blocks of the force phase on recorded steps (the kernels' grid)
   int ncell, lang;
-  int shared;      // windows shared by a block's warps (shared_windows)
   int by_atom;     // FP64 form: a warp per atom evaluates the pairs (few atoms)
 };
 
@@ -124,7 +123,7 @@ __device__ void scan_replica(const Dev &d, const RepBox &rb) {
 // A rebuild pass of the flagged replicas; `ic` = the coordinates current at this step.
 // Not inlined: it runs once in several steps and would take the registers of the others.
 // False when a barrier gave up.
-template <bool MIXED>
+template <bool MIXED, bool SHARED>
 __device__ __noinline__ bool rebuild(const ChunkArgs &A, int4 *ic, PhaseShared<MIXED> &sh) {
   Dev d = A.d;
   d.ic = ic;
@@ -141,7 +140,7 @@ __device__ __noinline__ bool rebuild(const ChunkArgs &A, int4 *ic, PhaseShared<M
   if (!grid_barrier(d)) return false;
   for (int c = warp; c < A.ncell; c += nwarp) rebuild_sort_gather(d, b, 0, c);
   if (!grid_barrier(d)) return false;
-  if (A.shared) rebuild_build<MIXED ? 1 : 0, true>(d, b, 0, sh.build.stage[wid], blockIdx.x, gridDim.x, &sh.build);
+  if constexpr (SHARED) rebuild_build<MIXED ? 1 : 0, true>(d, b, 0, sh.build.stage[wid], blockIdx.x, gridDim.x, &sh.build);
   else rebuild_build<MIXED ? 1 : 0, false>(d, b, 0, sh.build.stage[wid], warp, nwarp, nullptr);
   if (!grid_barrier(d)) return false;
   if (!MIXED) {
@@ -292,7 +291,9 @@ __device__ __forceinline__ void pair_phase(const Dev &d, const Box &b, const Ste
   }
 }
 
-template <bool MIXED, int TPA, int KICK, bool ONE>
+// SHARED: windows of a list build shared by a block's warps (shared_windows; both builds in one
+// kernel cost 0.3 us a step, in the instruction cache)
+template <bool MIXED, int TPA, int KICK, bool ONE, bool SHARED>
 __global__ void __launch_bounds__(CHUNK_THREADS, 4) k_chunk(const __grid_constant__ ChunkArgs A) {
   constexpr int ATOMS = 32 / TPA;
   __shared__ PhaseShared<MIXED> sh;
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 4) k_chunk(const __grid_constan
       break;
     }
     if (need) {
-      if (!rebuild<MIXED>(A, d.ic, sh)) return;
+      if (!rebuild<MIXED, SHARED>(A, d.ic, sh)) return;
       if (flags[F_OVERFLOW]) {
         // the host completes the step and folds its record from the first set of sums: a
         // Langevin step's temperature sums, of its drift above, go there (block 0 has folded
@@ -437,12 +438,12 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 4) k_chunk(const __grid_constan
   }
 }
 
-template <bool MIXED, int TPA, int KICK, bool ONE>
+template <bool MIXED, int TPA, int KICK, bool ONE, bool SHARED>
 int go(const ChunkArgs &A, int want, int share, cudaStream_t st) {
   static PerDevice blocks_per_sm;  // resident
   const int per_sm = blocks_per_sm.get([](int) {
     int n = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_chunk<MIXED, TPA, KICK, ONE>, CHUNK_THREADS, 0);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_chunk<MIXED, TPA, KICK, ONE, SHARED>, CHUNK_THREADS, 0);
     return e == cudaSuccess && n > 0 ? n : -1;
   });
   if (per_sm < 1) return CAVGPU_E_CUDA;
@@ -453,16 +454,24 @@ int go(const ChunkArgs &A, int want, int share, cudaStream_t st) {
   // 18.7 / 10.0 / 11.8; of 8 contexts of 48,668 mixed 33.1 / 20.9 / 21.9.
   const int grid = std::max(1, std::min(want, num_sms() * per_sm / std::min(std::max(share, 1), 4)));
   void *args[] = {const_cast<ChunkArgs *>(&A)};
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_chunk<MIXED, TPA, KICK, ONE>), dim3(grid),
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_chunk<MIXED, TPA, KICK, ONE, SHARED>), dim3(grid),
                                      dim3(CHUNK_THREADS), args, 0, st) == cudaSuccess
              ? CAVGPU_OK
              : CAVGPU_E_CUDA;
 }
 
+template <bool MIXED, int TPA, bool SHARED>
+int pick_kick(const ChunkArgs &A, int kick, bool one, int want, int share, cudaStream_t st) {
+  if (kick == 1)
+    return one ? go<MIXED, TPA, 1, true, SHARED>(A, want, share, st) : go<MIXED, TPA, 1, false, SHARED>(A, want, share, st);
+  return one ? go<MIXED, TPA, 2, true, SHARED>(A, want, share, st) : go<MIXED, TPA, 2, false, SHARED>(A, want, share, st);
+}
+
 template <bool MIXED, int TPA>
-int pick(const ChunkArgs &A, int kick, bool one, int want, int share, cudaStream_t st) {
-  if (kick == 1) return one ? go<MIXED, TPA, 1, true>(A, want, share, st) : go<MIXED, TPA, 1, false>(A, want, share, st);
-  return one ? go<MIXED, TPA, 2, true>(A, want, share, st) : go<MIXED, TPA, 2, false>(A, want, share, st);
+int pick(const ChunkArgs &A, const LaunchCfg &lc, int kick, int want, int share, cudaStream_t st) {
+  const bool one = lc.ntypes == 1;
+  return shared_windows(lc) ? pick_kick<MIXED, TPA, true>(A, kick, one, want, share, st)
+                            : pick_kick<MIXED, TPA, false>(A, kick, one, want, share, st);
 }
 
 }  // namespace
@@ -487,22 +496,23 @@ bool chunk_fits(const Box &b, const LaunchCfg &lc) {
 int launch_chunk(const Dev &d, const Box &b, const StepConsts &sc, const LaunchCfg &lc, int S, int ev, int fuse, int drop,
                  const FoldArgs &fa, int share, cudaStream_t st) {
   if (lc.precision == CAVGPU_FP64 && (!lc.exchange || !d.recv)) return CAVGPU_E_ARG;
-  ChunkArgs A{d, b, sc, fa, S, ev, fuse, drop, force_grid_blocks(lc), b.ncell_all, fuse == FUSE_LANG, shared_windows(lc), lc.n <= BY_ATOM};
+  ChunkArgs A{d, b, sc, fa, S, ev, fuse, drop, force_grid_blocks(lc), b.ncell_all, fuse == FUSE_LANG, lc.n <= BY_ATOM};
   A.d.step_kernel = 1;
-  // Mixed: four lanes a task per warp and a block per multiprocessor at least (4,000 atoms 12.4
-  // us a step, with a block per task 13.4, with a warp per atom 14.9: more blocks to wait for
-  // at every barrier), two lanes, whose systems are larger, a block per task (32,000 atoms 22.75
+  // Mixed: four lanes a task per warp, and a warp per atom (the rebuild's phases) up to a block per
+  // multiprocessor (4,000 atoms 12.4 us a step, with a block per task 13.4, with a warp per atom
+  // 14.9: more blocks to wait for at every barrier; 500 atoms 11.3, with a block per task 11.7,
+  // which does where others are at work), two lanes, whose systems are larger, a block per task (32,000 atoms 22.75
   // against 23.03).  FP64: a block per task, a warp per atom where those evaluate the pairs (the
   // FP64 pipe is an SM's own: 1,372 atoms 24.5 us, with a task per warp 27.6).
   const int ntask = (lc.n + 32 / lc.tpa - 1) / (32 / lc.tpa);
   const int want = lc.precision == CAVGPU_FP64 ? std::max(ntask, A.by_atom ? lc.n / CHUNK_WARPS : 0)
-                   : lc.tpa == 4 ? std::max((ntask + CHUNK_WARPS - 1) / CHUNK_WARPS, std::min(ntask, num_sms()))
+                   : lc.tpa == 4 ? std::max((ntask + CHUNK_WARPS - 1) / CHUNK_WARPS,
+                                                std::min(share > 1 ? ntask : lc.n / CHUNK_WARPS, num_sms()))
                                  : ntask;
   const int kick = fuse == FUSE_LANG ? 2 : 1;
-  const bool one = lc.ntypes == 1;
   if (lc.precision == CAVGPU_MIXED)
-    return lc.tpa == 2 ? pick<true, 2>(A, kick, one, want, share, st) : pick<true, 4>(A, kick, one, want, share, st);
-  return pick<false, 4>(A, kick, one, want, share, st);
+    return lc.tpa == 2 ? pick<true, 2>(A, lc, kick, want, share, st) : pick<true, 4>(A, lc, kick, want, share, st);
+  return pick<false, 4>(A, lc, kick, want, share, st);
 }
 
 }  // namespace cav

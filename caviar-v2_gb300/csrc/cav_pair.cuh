@@ -116,6 +116,13 @@ __device__ __forceinline__ void fold_lanes(double &fx, double &fy, double &fz, d
   }
 }
 
+// NaN for the acceleration of an atom that mixed_track marked (the integers of a position
+// that is not a number give a finite force)
+template <bool MIXED>
+__device__ __forceinline__ void spread_nan(const dbl4 &v, dbl4 &a) {
+  if (MIXED && __double2hiint(v.w) != 0) a.x = a.y = a.z = __longlong_as_double(0x7ff8000000000000ll);
+}
+
 // The closing update of the step of atom i, given its folded force sum.
 // KICK: 0 = store the acceleration only; 1 = velocity-Verlet closing kick
 // v += (a + a_old) * (0.5 dt) (src/md_simulator.cpp:672-679); 2 = Langevin closing
@@ -135,10 +142,6 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
   const double mi = tab.minv[ti];
   dbl4 an = make_dbl4(fx * mi, fy * mi, fz * mi, 0.0);
   dbl4 v;
-  // (mixed form: the integers of a position that is not a number give a finite force)
-  auto poison = [&]() {
-    if (MIXED && __double2hiint(v.w) != 0) an.x = an.y = an.z = __longlong_as_double(0x7ff8000000000000ll);
-  };
   if (KICK == 0) {
     d.acc[i] = an;
     if (EV) {
@@ -149,7 +152,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
   } else if (KICK == 1) {
     v = d.vel[i];
-    poison();
+    spread_nan<MIXED>(v, an);
     const dbl4 ao = d.acc[i];  // a(t), still in place until the store below
     if (MIXED) {
       v.x = fma(an.x + ao.x, sc.hdt, v.x);
@@ -167,7 +170,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
   } else {
     v = d.vel[i];
-    poison();
+    spread_nan<MIXED>(v, an);
     double e0 = 0.0, e1 = 0.0, e2 = 0.0;
     if (!sc.noise_off) {  // replica r draws the noise stream of seed + r with its local ids
       if (MIXED) langevin_eta_f(sc.seed + rep, step, d.id[i], e0, e1, e2);
