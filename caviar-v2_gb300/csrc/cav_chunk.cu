@@ -46,6 +46,10 @@ constexpr int MAX_REPLICAS = 6;
 // 47.8, 48.8 and 81.9; of 32,000 atoms mixed 32.8, 58.0 and 913 against 35.1, 36.0 and 71.2.  (The
 // waits of boxes with 10^8 cells would run into the barrier's limit.)
 constexpr int MAX_CELLS = 12288;
+// And one warp sorts the n atoms of a cell, n^2 / 32 comparisons one after the other: rows of
+// 2,048 words mean up to ~4,000 atoms in a cell and 10 ms, where 19,456 atoms in one cell (a box of
+// two list cutoffs) would take most of the time a barrier waits.
+constexpr int MAX_ROW = 2048;
 // polls of a barrier before a block gives up (seconds): the launch is cooperative, so a block
 // that never comes means a fault elsewhere.  The state is then half way through a step: the
 // host reads F_STALL and the context does nothing more.  (No block goes on past a barrier
@@ -479,7 +483,7 @@ int pick(const ChunkArgs &A, const LaunchCfg &lc, int kick, int want, int share,
 // Sizes for which the kernels' blocks hold one task per warp (the partial sums are then
 // those of the virtual blocks), at the lane counts small systems use.
 bool chunk_fits(const Box &b, const LaunchCfg &lc) {
-  if (b.nrep > MAX_REPLICAS || b.ncell_all > MAX_CELLS) return false;
+  if (b.nrep > MAX_REPLICAS || b.ncell_all > MAX_CELLS || lc.row > MAX_ROW) return false;
   if (lc.images) return false;  // (k_force alone applies image codes to fixed-point coordinates)
   if (lc.use_seg || lc.block != CHUNK_THREADS || (lc.tpa != 2 && lc.tpa != 4)) return false;
   if (lc.precision == CAVGPU_FP64 && (!lc.exchange || lc.tpa != 4 || lc.n > FP64_ATOMS)) return false;

@@ -2,7 +2,8 @@
 
 Rows of more than 132 words are built by one warp per window, where shared windows would
 overflow their parts; rows of more than 200 keep two lanes per atom up to 65,536 slots and the
-step kernel to one task per resident warp, rows of more than 600 four lanes up to 38,912.
+step kernel to one task per resident warp, rows of more than 600 four lanes up to 38,912;
+rows of more than 2,048, whose cells hold thousands of atoms, are not for the step kernel.
 """
 import numpy as np
 import pytest
@@ -78,3 +79,28 @@ def test_default_lanes(cells, rc, lanes):
     s = G.System(*fluid(cells, rc), precision=G.MIXED)
     assert s.stats()["threads_per_atom"] == lanes
     s.close()
+
+
+@pytest.mark.parametrize("cells,graphs,precision", [(9, False, G.FP64), (11, True, G.FP64), (9, False, G.MIXED)])
+def test_cells_of_hundreds_of_atoms(cells, graphs, precision):
+    """Particles a fifth of the usual size in a box of two list cutoffs: 2,916 and 5,324 atoms in
+    eight cells, rows of ~1,500 and ~2,800 words."""
+    rng = np.random.default_rng(3)
+    L = np.full(3, 5.7)
+    pos, box = W.fcc_lattice((cells,) * 3, 0.8442)
+    scale = 5.7 / box[0]
+    pos = np.mod((pos + rng.uniform(-0.05, 0.05, size=pos.shape)) * scale, L)
+    pos[pos >= 5.7] = 0.0
+    p = W.lj_params(L, sigma=np.array([[scale]]), dt=0.0005)
+    out = []
+    for spg in (0, -1):
+        s = G.System(pos, W.thermal_velocities(len(pos), 1.0, np.random.default_rng(1)), np.zeros(len(pos), np.int32), p,
+                     precision=precision, steps_per_graph=spg)
+        s.setup()
+        s.run(6, 3)
+        out.append(s.state())
+        if spg == 0:
+            assert (s.stats()["graph_launches"] > 0) == graphs
+        s.close()
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
