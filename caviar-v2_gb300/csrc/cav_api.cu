@@ -663,8 +663,8 @@ int create_common(const cavgpu_params *p, int nrep, const double *lo3, const dou
   b.ce2_lo = (float)(b.ce2 * (1.0 - 2e-4));
   b.ce2_hi = (float)(b.ce2 * (1.0 + 2e-4));
   b.thr2 = 0.25 * (ce - p->nl_cutoff) * (ce - p->nl_cutoff);
-  // mixed form: shrunk by two fixed-point units of the coarsest axis and by 1e-6; without
-  // a skin every step rebuilds
+  // mixed form: shrunk by two fixed-point units of the coarsest axis and by 1e-6; with less
+  // skin than that the test is done on the positions (track_far)
   double unit = 0.0;
   for (const RepBox &rb : c->reps)
     for (int a = 0; a < 3; ++a) unit = std::max(unit, (double)rb.uh[a]);

@@ -142,7 +142,7 @@ struct Box {
   double ce2;           // cutoff_extra^2, the list predicate r^2 < ce2 (src/neighborlist.cpp:258, :508)
   float ce2_lo, ce2_hi; // FP32 pre-screen band around ce2
   double thr2;          // 0.25 (cutoff_extra - cutoff)^2 (src/neighborlist.cpp:318)
-  float thr2f;          // thr2 in FP32, shrunk: the mixed form's test may only fire early
+  float thr2f;          // thr2 in FP32, shrunk: the mixed form's test may only fire early (-1: no test in FP32)
   RepBox r0;            // replica 0 by value: the single-system path reads no replica table
 };
 
@@ -446,12 +446,13 @@ __device__ inline void half_skin_test(const Dev &d, const Box &b, int rep, int i
 // test on their difference to those of the last build (in FP32 against a threshold
 // shrunk by the units' rounding and 1e-6, so it can only fire early; the window
 // indices tell a displacement that wrapped, as in a system that flies apart).  Where the
-// windows are not known the positions themselves are compared; one that is not a number
-// marks its atom (vel.w), whose next acceleration is then NaN (finish_atom).
+// windows are not known, or the skin is no wider than the units' rounding, the positions
+// themselves are compared; one that is not a number marks its atom (vel.w), whose next
+// acceleration is then NaN (finish_atom).
 __device__ __forceinline__ void track_far(const Dev &d, const Box &b, int rep, int i, const dbl4 &x) {
   const dbl4 r = d.pos_ref[i];
   const double dx = x.x - r.x, dy = x.y - r.y, dz = x.z - r.z, d2 = dx * dx + dy * dy + dz * dz;
-  if (!(d2 <= (double)b.thr2f)) request_rebuild(d, b, rep);
+  if (!(d2 <= b.thr2)) request_rebuild(d, b, rep);
   if (isnan(x.x) || isnan(x.y) || isnan(x.z)) d.vel[i].w = 1.0;
 }
 __device__ inline void mixed_track(const Dev &d, const Box &b, int rep, int i, const dbl4 &x, int4 *out) {
@@ -459,7 +460,7 @@ __device__ inline void mixed_track(const Dev &d, const Box &b, int rep, int i, c
   int3 w;
   const int4 q = fixed_pos(rb, x, type_of(x.w), w), r = d.ic_ref[i];
   out[i] = q;
-  if ((r.w >> 30) != 0 || !window_known(w)) {
+  if ((r.w >> 30) != 0 || !window_known(w) || b.thr2f < 0.0f) {
     track_far(d, b, rep, i, x);
     return;
   }
