@@ -433,9 +433,11 @@ __device__ __forceinline__ bool beyond_window(int q, int qw, int r, int rw) {
 __device__ inline void half_skin_test(const Dev &d, const Box &b, int rep, int i, const dbl4 &x) {
   const dbl4 r = d.pos_ref[i];
   const double dx = x.x - r.x, dy = x.y - r.y, dz = x.z - r.z;
-  // compared as bit patterns (the order of doubles >= +0; a NaN counts as beyond), off the FP64 pipe
-  if ((__double_as_longlong(dx * dx + dy * dy + dz * dz) & 0x7fffffffffffffffll) > __double_as_longlong(b.thr2))
-    request_rebuild(d, b, rep);
+  // compared as bit patterns (the order of doubles >= +0), off the FP64 pipe: beyond the threshold
+  // and up to infinity (a NaN is not beyond it)
+  const unsigned long long thr = (unsigned long long)__double_as_longlong(b.thr2),
+                           d2 = (unsigned long long)__double_as_longlong(dx * dx + dy * dy + dz * dz);
+  if (d2 - thr - 1ull < 0x7ff0000000000000ull - thr) request_rebuild(d, b, rep);
   if (d.ic) {
     int3 w;
     d.ic[i] = fixed_pos(repbox(b, rep), x, type_of(x.w), w);
@@ -452,7 +454,7 @@ __device__ inline void half_skin_test(const Dev &d, const Box &b, int rep, int i
 __device__ __forceinline__ void track_far(const Dev &d, const Box &b, int rep, int i, const dbl4 &x) {
   const dbl4 r = d.pos_ref[i];
   const double dx = x.x - r.x, dy = x.y - r.y, dz = x.z - r.z, d2 = dx * dx + dy * dy + dz * dz;
-  if (!(d2 <= b.thr2)) request_rebuild(d, b, rep);
+  if (d2 > b.thr2) request_rebuild(d, b, rep);  // (not a NaN: the list stays, and the forces show it)
   if (isnan(x.x) || isnan(x.y) || isnan(x.z)) d.vel[i].w = 1.0;
 }
 __device__ inline void mixed_track(const Dev &d, const Box &b, int rep, int i, const dbl4 &x, int4 *out) {

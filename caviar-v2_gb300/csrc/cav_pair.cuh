@@ -116,11 +116,11 @@ __device__ __forceinline__ void fold_lanes(double &fx, double &fy, double &fz, d
   }
 }
 
-// NaN for the acceleration of an atom that mixed_track marked (the integers of a position
-// that is not a number give a finite force)
+// NaN for the acceleration of an atom that mixed_track marked, if it has neighbours (the
+// integers of a position that is not a number give a finite force)
 template <bool MIXED>
-__device__ __forceinline__ void spread_nan(const dbl4 &v, dbl4 &a) {
-  if (MIXED && __double2hiint(v.w) != 0) a.x = a.y = a.z = __longlong_as_double(0x7ff8000000000000ll);
+__device__ __forceinline__ void spread_nan(const Dev &d, int i, const dbl4 &v, dbl4 &a) {
+  if (MIXED && __double2hiint(v.w) != 0 && d.nnbr[i] > 0) a.x = a.y = a.z = __longlong_as_double(0x7ff8000000000000ll);
 }
 
 // The closing update of the step of atom i, given its folded force sum.
@@ -152,7 +152,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
   } else if (KICK == 1) {
     v = d.vel[i];
-    spread_nan<MIXED>(v, an);
+    spread_nan<MIXED>(d, i, v, an);
     const dbl4 ao = d.acc[i];  // a(t), still in place until the store below
     if (MIXED) {
       v.x = fma(an.x + ao.x, sc.hdt, v.x);
@@ -170,7 +170,7 @@ __device__ __forceinline__ void finish_atom(const Dev &d, const Box &b, const St
     }
   } else {
     v = d.vel[i];
-    spread_nan<MIXED>(v, an);
+    spread_nan<MIXED>(d, i, v, an);
     double e0 = 0.0, e1 = 0.0, e2 = 0.0;
     if (!sc.noise_off) {  // replica r draws the noise stream of seed + r with its local ids
       if (MIXED) langevin_eta_f(sc.seed + rep, step, d.id[i], e0, e1, e2);

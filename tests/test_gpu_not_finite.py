@@ -56,3 +56,21 @@ def test_far_displacement_rebuilds(cells, windows):
     assert s.stats()["rebuilds"] == 2  # set-up and the step's own
     assert np.abs(s.state()[2][i]).max() == 0.0  # out of the others' reach
     s.close()
+
+
+@pytest.mark.parametrize("precision", [G.FP64, G.MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("cells,spg", [(3, 0), (3, -1), (12, 0)])
+def test_position_that_is_not_a_number_of_an_atom_on_its_own(cells, spg, precision):
+    """Without neighbours it causes no NaN force, and its displacement is not "more than" half the
+    skin: the others go on, the list stays."""
+    g = np.stack(np.meshgrid(*[np.arange(cells)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos, vel = (g + 0.5) * 4.0, np.zeros((cells ** 3, 3))
+    vel[2, 0] = np.nan
+    s = G.System(pos, vel, np.zeros(len(pos), np.int32), W.lj_params(np.full(3, 4.0 * cells)), precision=precision,
+                 steps_per_graph=spg)
+    s.setup()
+    s.step(10)
+    x, _, a = s.state()
+    assert s.stats()["rebuilds"] == 1 and s.stats()["steps"] == 10
+    assert np.isnan(x[2, 0]) and np.isfinite(np.delete(x, 2, 0)).all() and (a == 0.0).all()
+    s.close()
