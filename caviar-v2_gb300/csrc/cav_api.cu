@@ -27,7 +27,7 @@ constexpr int MAX_GRAPH_STEPS = 1000;  // steps captured per graph, and thermo r
 // fuse[k]: step k's pair kernel also does step k + 1's drift (Fuse), so that a step is
 // one launch; steps that begin a chunk, or follow a step that did not drift them,
 // launch their drift kernel.  The fused steps of a chunk are made even in number,
-// so that the gathered coordinates (FP64 positions or mixed rel), which alternate
+// so that the gathered coordinates (FP64 positions or the mixed form's ic), which alternate
 // between two buffers at every fused step, end the chunk in the buffer they began.
 struct ChunkPlan {
   int S = 0, ev = 0;          // steps; record period (thermo at step k iff ev > 0 and (k + 1) % ev == 0)

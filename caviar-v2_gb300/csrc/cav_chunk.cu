@@ -12,12 +12,11 @@
 // sums per (virtual) block and the same folds, so that the results equal those of the
 // kernels bit for bit.
 //
-// Steps (LJ fluid, us, graph -> here): mixed 4,000 atoms 29.6 -> 17.7, 19,652 36 -> 29, 32,000
-// 41 -> 29, Kob-Andersen Langevin 32,000 37 -> 28; FP64 500 atoms 55 -> 24, 4,000 54 -> 39.
-// Of the 17.7: force, kick and drift 4.7 (one walk through a list row, gather by gather, and
-// ~45 FP64 instructions of 64 cycles per warp), barriers and phase starts 2, a rebuild every
-// seventh step 60 (bin 5, scan 2, scatter 2, sort and gather 4, build 17, barriers and the
-// slowest blocks' waits the rest).
+// Steps (LJ fluid, us, graph of kernels / here): mixed 4,000 atoms 23.3 / 12.4, 19,652 26.9 / 18.9,
+// 32,000 31.0 / 22.6; FP64 500 atoms 29.8 / 19.9, 4,000 42.4 / 35.5.  Of 4,000 mixed atoms: force,
+// kick and drift 4.7 (one walk through a list row, gather by gather, and ~45 FP64 instructions
+// of 64 cycles per warp), barriers and phase starts 2, a rebuild every seventh step ~45 (build 17,
+// bin, scan, scatter, sort and gather 13, barriers and the slowest blocks' waits the rest).
 #include <algorithm>
 
 #include "cav_drift.cuh"
@@ -71,7 +70,8 @@ struct ChunkArgs {
 };
 
 // Barrier of all blocks.  Block 0 adds what makes the word's top bit flip once the others
-// have added one each; nothing has to be reset.  False when the barrier gave up.
+// have added one each (the construction of CUDA's cooperative groups); nothing has to be
+// reset.  False when the barrier gave up.
 __device__ __forceinline__ bool grid_barrier(const Dev &d) {
   __shared__ int s_ok;
   __syncthreads();
@@ -392,10 +392,10 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 4) k_chunk(const __grid_constan
           else close_task<TPA, KICK, true>(v, b, sc, mtab, task, step, fuse_mode, ke);
         }
         if constexpr (MIXED) {
-          block_sum_store_f<2>(ev, &v.partials_ev[(size_t)vb * 2]);
+          block_sum_store<2>(ev, &v.partials_ev[(size_t)vb * 2]);
           __syncthreads();
         }
-        block_sum_store_f<4>(ke, &(KICK == 2 ? v.partials_ke_end : v.partials_ke)[(size_t)vb * 4]);
+        block_sum_store<4>(ke, &(KICK == 2 ? v.partials_ke_end : v.partials_ke)[(size_t)vb * 4]);
         __syncthreads();
       }
     } else {

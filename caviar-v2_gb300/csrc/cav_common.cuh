@@ -492,6 +492,34 @@ __device__ inline bool halted(const Dev &d) {  // one load: every thread of a re
   return d.step_kernel ? (unsigned)both != 0u : both != 0ull;
 }
 
+// a rebuild pass builds the replicas whose half-skin test fired (all when forced);
+// nothing after a halt
+__device__ inline bool rebuild_on(const Dev &d, const Box &b, int rep, int forced) {
+  return !halted(d) && (forced || b.rep_flag[rep] != 0);
+}
+
+#define FULL_MASK 0xffffffffu
+
+// Block reduction of NV doubles in a fixed order (deterministic).
+template <int NV>
+__device__ inline void block_sum_store(double (&v)[NV], double *out /* NV doubles */) {
+  __shared__ double sh[32][NV];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(FULL_MASK, v[k], o);
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh[wid][k] = v[k];
+  __syncthreads();
+  if (threadIdx.x < NV) {  // a thread per value: an FP64 add takes a warp 64 cycles, whoever needs it
+    double s = 0.0;
+    for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
+    out[threadIdx.x] = s;
+  }
+}
+
 // ---- host-side launch helpers ----------------------------------------------
 struct LaunchCfg {
   int precision;   // CAVGPU_FP64 / CAVGPU_MIXED

@@ -21,7 +21,7 @@
 // received force.  LJ fluid, force of a step: 1,048,576 atoms 3.81 -> 1.87 ms, 131,072 atoms
 // 0.52 -> 0.28 ms; of that k_pairs64 three quarters (FP64 pipe 80-85% busy, 691 FP64
 // instructions per 32 atoms and warp against 557 that its lanes need) and k_close64 one (79%,
-// 204 instructions, 1.6 KB read per atom).  A build takes 1.2 ms longer at 1,048,576 atoms
+// 204 instructions, 1.6 KB read per atom, 1.2 of it received forces).  A build takes 1.2 ms longer at 1,048,576 atoms
 // (k_claim 0.7: its atomics and scattered notes; k_rank 0.5: issue), 0.2 ms per step.
 // Tried: all lanes of a warp on one atom after the other in step (1.0-1.05 of the time);
 // each warp in a region of its own (1.5 times the time: the handed-over forces then go to
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(32, MINB) k_pairs64(Dev d, Box b, StepConsts s
                      : pair_tasks<TPA, EV, ONE, false>(d, b, sc, tab, W, nt, rep, task, task_end, ev_p);
     }
   }
-  if (EV) block_sum_store_f<2>(ev_p, &d.partials_ev[(size_t)blockIdx.x * 2]);
+  if (EV) block_sum_store<2>(ev_p, &d.partials_ev[(size_t)blockIdx.x * 2]);
 }
 
 // Few atoms: a warp each, unless virial and energy are wanted.  A step as a graph of kernels
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(CLOSE_THREADS) k_close64(Dev d, Box b, StepCon
     }
   }
   if (EV && !was_halted)
-    block_sum_store_f<4>(ke_p, &(KICK == 2 ? d.partials_ke_end : d.partials_ke)[(size_t)blockIdx.x * 4]);
+    block_sum_store<4>(ke_p, &(KICK == 2 ? d.partials_ke_end : d.partials_ke)[(size_t)blockIdx.x * 4]);
   if (KICK != 0) end_of_step<EV>(d, was_halted, fa);
 }
 

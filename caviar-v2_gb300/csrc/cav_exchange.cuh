@@ -339,16 +339,13 @@ __device__ __forceinline__ void close_ev(const Dev &d, int i) {
 // ---------------------------------------------------------------------------
 // after a list build: the claimed entries of every atom and their receiving slots
 // ---------------------------------------------------------------------------
-__device__ inline bool exchange_on(const Dev &d, const Box &b, int rep, int forced) {
-  return rep >= 0 && !halted(d) && (forced || b.rep_flag[rep] != 0);
-}
-
 // Warp per atom: copies the entries it claims out of its row, takes a receiving slot of the
 // other atom for each and leaves {its slot, the entry} there.  A row that outgrows the
 // space counts as an overflow of the list (which doubles as the room for it).
 __device__ __forceinline__ void claim_slot(const Dev &d, const Box &b, int forced, int i) {
   const int lane = threadIdx.x & 31;
-  if (!exchange_on(d, b, rep_of_slot(b, i), forced)) return;
+  const int rep = rep_of_slot(b, i);
+  if (rep < 0 || !rebuild_on(d, b, rep, forced)) return;
   const int cs = 7 - log2_pow2(d.tpa);  // chunk stride 4A words = 2^(log2 A + 2)
   const uint32_t *const row = d.nbr + nbr_block_base(i, d.cap, d.tpa);
   uint32_t *const out = d.hw + nbr_block_base(i, d.cap_h, d.tpa);
@@ -379,7 +376,8 @@ __device__ __forceinline__ void claim_slot(const Dev &d, const Box &b, int force
 // receiving slot, so that sums do not depend on the order of the atomics.
 __device__ __forceinline__ void rank_slot(const Dev &d, const Box &b, int forced, int j) {
   const int lane = threadIdx.x & 31;
-  if (!exchange_on(d, b, rep_of_slot(b, j), forced)) return;
+  const int rep = rep_of_slot(b, j);
+  if (rep < 0 || !rebuild_on(d, b, rep, forced)) return;
   const int n = min(d.nr[j], d.cap_h);
   const uint2 *const note = reinterpret_cast<const uint2 *>(d.recv) + (size_t)j * d.cap_h;
   for (int p0 = 0; p0 < n; p0 += 64) {  // two notes per lane

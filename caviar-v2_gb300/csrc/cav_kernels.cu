@@ -21,28 +21,6 @@ int num_sms() {
 }
 
 // ---------------------------------------------------------------------------
-// block reduction of NV doubles in a fixed order (deterministic)
-// ---------------------------------------------------------------------------
-template <int NV>
-__device__ inline void block_sum_store(double (&v)[NV], double *out /* NV doubles */) {
-  __shared__ double sh[32][NV];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(FULL_MASK, v[k], o);
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) sh[wid][k] = v[k];
-  __syncthreads();
-  if (threadIdx.x < NV) {  // a thread per value
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
-    out[threadIdx.x] = s;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // integrator stage 1 -- src/md_simulator.cpp:640-656 (velocity Verlet) and
 // :748-837 (Langevin first half); NaN check; half-skin test per replica
 // ---------------------------------------------------------------------------

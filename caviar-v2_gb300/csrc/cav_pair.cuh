@@ -9,27 +9,6 @@
 
 namespace cav {
 
-#define FULL_MASK 0xffffffffu
-
-template <int NV>
-__device__ inline void block_sum_store_f(double (&v)[NV], double *out) {
-  __shared__ double sh[32][NV];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(FULL_MASK, v[k], o);
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) sh[wid][k] = v[k];
-  __syncthreads();
-  if (threadIdx.x < NV) {  // a thread per value: an FP64 add takes a warp 64 cycles, whoever needs it
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
-    out[threadIdx.x] = s;
-  }
-}
-
 struct SmemTabD {
   double rc2[MAXT * MAXT], sig2[MAXT * MAXT], eps4[MAXT * MAXT], gc[MAXT * MAXT], uc[MAXT * MAXT];
   double e6[MAXT * MAXT], e12[MAXT * MAXT];  // 6 eps4 and 12 eps4 (exact: products by 6 and 12)
@@ -277,7 +256,7 @@ static __device__ __noinline__ void fold_thermo(const Dev &d, const FoldArgs &fa
   fold_strided<2>(d.partials_ev, fa.nb_ev, v + 4);
   fold_strided<4>(d.partials_ke_end, fa.nb_ke_end, v + 6);
   __shared__ double out[10];
-  block_sum_store_f<10>(v, out);
+  block_sum_store<10>(v, out);
   __syncthreads();
   if (threadIdx.x != 0) return;
   const ThermoCfg &tc = fa.tc;
@@ -335,9 +314,9 @@ __device__ __forceinline__ void end_of_step(const Dev &d, bool was_halted, const
 template <int KICK, bool EV>
 __device__ inline void store_partials(const Dev &d, double (&ke_p)[4], double (&ev_p)[2]) {
   if (EV) {
-    block_sum_store_f<2>(ev_p, &d.partials_ev[(size_t)blockIdx.x * 2]);
+    block_sum_store<2>(ev_p, &d.partials_ev[(size_t)blockIdx.x * 2]);
     __syncthreads();
-    block_sum_store_f<4>(ke_p, &(KICK == 2 ? d.partials_ke_end : d.partials_ke)[(size_t)blockIdx.x * 4]);
+    block_sum_store<4>(ke_p, &(KICK == 2 ? d.partials_ke_end : d.partials_ke)[(size_t)blockIdx.x * 4]);
   }
 }
 

@@ -7,22 +7,12 @@
 
 namespace cav {
 
-#ifndef FULL_MASK
-#define FULL_MASK 0xffffffffu
-#endif
-
 // ---------------------------------------------------------------------------
 // list rebuild of the flagged replicas: wrap + bin -> per-replica scan ->
 // scatter -> per-cell sort -> gather -> build
 // (Neighborlist::update_cell_list + update_verlet_list_from_cell_list,
 //  src/neighborlist.cpp:422-455, 496-553; Domain::fix_position, src/domain.cpp:443-493)
 // ---------------------------------------------------------------------------
-// a rebuild pass builds the replicas whose half-skin test fired (all when forced);
-// nothing after a halt
-__device__ inline bool rebuild_on(const Dev &d, const Box &b, int rep, int forced) {
-  return !halted(d) && (forced || b.rep_flag[rep] != 0);
-}
-
 // Domain::fix_position's single-image test per axis (src/domain.cpp:443-493):
 // -1 below the lower face (x += L), +1 above the upper face (x -= L), else 0
 __device__ inline int3 wrap_shift(const RepBox &rb, const dbl4 &p) {
