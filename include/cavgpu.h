@@ -11,8 +11,9 @@
  * `const uint64_t*`).
  *
  * One context = one periodic system on one GPU, bound to one CUDA stream;
- * calls on one context are not thread-safe (the reference's Caviar2 object
- * is not re-entrant either).  There is no CPU fallback: without a GPU,
+ * calls on one context exclude one another (the reference's Caviar2 object
+ * is not re-entrant either), contexts may be used from different threads
+ * at the same time.  There is no CPU fallback: without a GPU,
  * cavgpu_create returns CAVGPU_E_CUDA.
  *
  * Error convention: every call returns CAVGPU_OK (0) or a negative status;
@@ -44,7 +45,7 @@ extern "C" {
 
 /* precision of the pair force */
 #define CAVGPU_FP64 0              /* all-FP64 kernels (the parity form) */
-#define CAVGPU_MIXED 1             /* FP32 pair math on cell-relative coordinates, FP64 state */
+#define CAVGPU_MIXED 1             /* FP32 pair math on fixed-point coordinates, FP64 state */
 
 /* integrators (Integrator_t, inc/caviar2/md_simulator.hpp:34-41) */
 #define CAVGPU_VELOCITY_VERLET 0
@@ -76,8 +77,12 @@ typedef struct cavgpu_params {
   int32_t precision;              /* CAVGPU_FP64 or CAVGPU_MIXED */
   int32_t noise_off;              /* Langevin with eta = 0 (exactness checks) */
   int32_t nbr_capacity;           /* neighbour slots per atom; 0 = sized at set-up */
-  int32_t threads_per_atom;       /* force kernel lanes per atom (1,2,4,8,16); 0 = by system size
-                                     (FP64: 1, 2, 4 give the same bits, see cavgpu_pair_exchange) */
+  int32_t threads_per_atom;       /* force kernel lanes per atom (1,2,4,8,16); 0 = by the number of slots
+                                     and the length of the list rows.  FP64: 1, 2 and 4 give the same
+                                     bits, see cavgpu_pair_exchange.  Mixed: a lane adds its share of a
+                                     row in two FP32 sums, lanes meet in FP64, so each number of lanes
+                                     has its own rounding (of 75 words: force error 5.51e-7 of the rms
+                                     with one lane, 5.45e-7 with four) */
   int32_t block_size;             /* force kernel block size (32..256, multiple of 32); 0 = default */
   int32_t steps_per_graph;        /* steps captured per CUDA graph; 0 = default (50); < 0 = no
                                      graphs, every kernel launched from the host (for profilers,
@@ -113,8 +118,7 @@ typedef struct cavgpu_params {
 #define CAVGPU_NVE_KBT 2
 #define CAVGPU_NVE_KB_TEMPERATURE 3
 
-/* pair-kernel variants of the mixed form (the FP64 form has one kernel); both give
- * the same results bit for bit */
+/* pair-kernel variants of the mixed form; both give the same results bit for bit */
 #define CAVGPU_FORCE_AUTO 0       /* grid-strided; the autotuner may switch to segments */
 #define CAVGPU_FORCE_STRIDED 1    /* grid-strided tasks, neighbour gathers from global memory */
 #define CAVGPU_FORCE_SEGMENTS 2   /* row segments staged in shared memory */
@@ -273,7 +277,9 @@ int cavgpu_autotune(cavgpu_ctx *ctx, int32_t trial_steps, int32_t flags, int64_t
  * each with its own periodic box, atom count, cell grid and half-skin rebuild,
  * sharing params, pair table and integrator).  A batch advances with
  * cavgpu_step / cavgpu_run(every = 0) and each replica's trajectory equals that
- * of its own single-system context in FP64 form.  The single-system exports
+ * of its own single-system context in FP64 form (bit for bit, where both or neither
+ * run the pair exchange), in mixed form to FP32 rounding (the default threads_per_atom
+ * follows the slots of the whole batch, and the sums it).  The single-system exports
  * (pairs, bins, ghosts) and cavgpu_thermo refuse batches (CAVGPU_E_ARG). */
 
 /* Create a batch of nrep >= 1 replicas; replica r's box is [lo3[3r..3r+2],
