@@ -454,8 +454,8 @@ int go(const ChunkArgs &A, int want, int share, cudaStream_t st) {
   // Contexts stepped at the same time (threads) divide the blocks that can be resident: a
   // launch whose blocks do not fit beside the running ones waits for them to end.  Time per
   // step and context of 4 contexts of 4,000 atoms, each on its own / sharing / as graphs of
-  // kernels, which overlap: mixed 14.8 / 3.9 / 8.0 us, FP64 35.5 / 17.8 / 20.8; of 19,652 atoms mixed
-  // 18.7 / 10.0 / 11.8; of 8 contexts of 48,668 mixed 33.1 / 20.9 / 21.9.
+  // kernels, which overlap: mixed 14.8 / 3.9 / 8.0 us, FP64 35.5 / 19.6 / 20.8; of 19,652 atoms mixed
+  // 18.7 / 10.3 / 11.7; of 8 contexts of 48,668 mixed 33.1 / 21.7 / 21.6.
   const int grid = std::max(1, std::min(want, num_sms() * per_sm / std::min(std::max(share, 1), 4)));
   void *args[] = {const_cast<ChunkArgs *>(&A)};
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_chunk<MIXED, TPA, KICK, ONE, SHARED>), dim3(grid),
@@ -505,9 +505,10 @@ int launch_chunk(const Dev &d, const Box &b, const StepConsts &sc, const LaunchC
   // Mixed: four lanes a task per warp, and a warp per atom (the rebuild's phases) up to a block per
   // multiprocessor (4,000 atoms 12.4 us a step, with a block per task 13.4, with a warp per atom
   // 14.9: more blocks to wait for at every barrier; 500 atoms 11.3, with a block per task 11.7,
-  // which does where others are at work), two lanes, whose systems are larger, a block per task (32,000 atoms 22.75
-  // against 23.03).  FP64: a block per task, a warp per atom where those evaluate the pairs (the
-  // FP64 pipe is an SM's own: 1,372 atoms 24.5 us, with a task per warp 27.6).
+  // which does where others are at work); two lanes, whose systems are larger, a block per task
+  // (32,000 atoms 22.75 against 23.03).  FP64: a block per task, a warp per atom where those
+  // evaluate the pairs (the FP64 pipe is an SM's own: 1,372 atoms 24.5 us, with a task per warp
+  // 27.6).
   const int ntask = (lc.n + 32 / lc.tpa - 1) / (32 / lc.tpa);
   const int want = lc.precision == CAVGPU_FP64 ? std::max(ntask, A.by_atom ? lc.n / CHUNK_WARPS : 0)
                    : lc.tpa == 4 ? std::max((ntask + CHUNK_WARPS - 1) / CHUNK_WARPS,
