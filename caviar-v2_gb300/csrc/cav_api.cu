@@ -185,7 +185,11 @@ std::atomic<int> AtWork::count[PerDevice::MAX_DEVICES];
 
 // device memory that the context cannot do without
 cudaError_t must_malloc(cavgpu_ctx *c, void **q, size_t bytes) {
+#ifdef CAV_SHORT_OF_MEMORY  // (tests)
+  cudaError_t e = cudaErrorMemoryAllocation;
+#else
   cudaError_t e = cudaMalloc(q, bytes);
+#endif
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     {

@@ -1,5 +1,6 @@
 """Paths that a full-sized GPU does not take by itself, in builds of the library whose limits
-are lower: a grid barrier that gives up, and FP64 forces without the pair exchange.
+are lower: a grid barrier that gives up, FP64 forces without the pair exchange, and contexts
+that take the exchange arrays of others.
 """
 import os
 import subprocess
@@ -93,3 +94,30 @@ def test_forces_without_the_pair_exchange(cells, types, integrator, load):
     for other in (got[normal, 4], got[full, 8]):
         for x, y in zip(ref, other):
             assert np.abs(x - y).max() < 1e-9
+
+
+@pytest.mark.parametrize("cells,integrator", [(4, 0), (9, 2), (17, 1)])
+def test_run_goes_on_after_its_arrays_were_given_back(cells, integrator, load):
+    """In a build whose allocations fail at first, a second context takes the first one's exchange
+    arrays; the first goes on over the full list it has, to rounding as if nothing had happened."""
+    system, out, normal = fluid(cells, 1, integrator), [], G.LIB_PATH
+    short = variant("cavgpu_short", "cav_api.cu", "-DCAV_SHORT_OF_MEMORY")
+    for lib in (normal, short):
+        load(lib)
+        a = G.System(*system)
+        a.setup()
+        a.step(23)
+        assert a.pair_exchange()
+        b = G.System(*system)
+        assert a.pair_exchange() == (lib == normal) and b.pair_exchange()
+        rec = a.run(24, 4)
+        out.append((rec, *a.state(), a.stats()["rebuilds"]))
+        b.setup()
+        b.step(5)
+        b.close()
+        a.step(3)
+        a.close()
+    assert out[0][4] == out[1][4] > 1
+    for x, y in zip(out[0][1:4], out[1][1:4]):
+        assert np.abs(x - y).max() < 1e-8  # sums in another order (2e-11) over 24 steps
+    np.testing.assert_allclose(out[0][0], out[1][0], rtol=1e-10, atol=1e-8 * len(system[0]))
